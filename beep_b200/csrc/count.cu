@@ -1198,44 +1198,112 @@ __device__ __forceinline__ unsigned long long wheel4_thread(const uint64_t *rows
     return cnt;
 }
 
-// One warp, rows of W <= 32 32-bit words (lane k holds word k); the count is
-// returned on lane 0.
-__device__ __forceinline__ unsigned long long wheel4_warp(const uint32_t *rows, uint32_t W, uint32_t a, int lane) {
-    const uint32_t k = (uint32_t)lane;
-    const uint32_t aw = a >> 5;
-    const uint32_t above = ~((2u << (a & 31)) - 1u);
-    auto hi = [&](uint32_t w) { return k > aw ? w : (k == aw ? (w & above) : 0u); };
-    const uint32_t ra = k < W ? hi(rows[(size_t)a * W + k]) : 0u;
-    uint32_t U = 0, w = ra;
-    unsigned bal = __ballot_sync(kFull, w != 0);
-    while (bal) {
-        const int L = __ffs(bal) - 1;
-        const uint32_t ww = __shfl_sync(kFull, w, L);
-        const uint32_t b = ((uint32_t)L << 5) + (uint32_t)(__ffs(ww) - 1);
-        if (lane == L)
-            w &= w - 1;
-        if (k < W)
-            U |= rows[(size_t)b * W + k];
-        bal = __ballot_sync(kFull, w != 0);
-    }
-    uint32_t u = k < W ? hi(U) : 0u;
-    unsigned long long cnt = 0;
-    bal = __ballot_sync(kFull, u != 0);
-    while (bal) {
-        const int L = __ffs(bal) - 1;
-        const uint32_t uu = __shfl_sync(kFull, u, L);
-        const uint32_t c = ((uint32_t)L << 5) + (uint32_t)(__ffs(uu) - 1);
-        if (lane == L)
-            u &= u - 1;
-        uint32_t n = k < W ? (uint32_t)__popc(ra & rows[(size_t)c * W + k]) : 0u;
+// Wider rows: bit-sliced counters. A lane owns one word column (32 domain
+// vertices c) and counts, for one vertex a, the b of row(a) below a whose row
+// holds c -- |row(a) & row(c) below a| for all 32 c at once: slice k of the
+// counters holds bit k of each. Eight row words at a time go through carry-
+// save adders (two three-input logic instructions each, about 2.5 a word), so
+// the 32 x nb counter increments of a column cost a load and ~2.5 logic
+// instructions per b. The 4-cycles whose largest vertex is a and whose
+// opposite vertex is c number C(count, 2), and every 4-cycle of the
+// neighbourhood graph is counted once, at its largest vertex. Taking the
+// largest vertex keeps the b below a: in the ascending order these are the
+// sparser rows (R-MAT s16 ef28: half the b-c pairs that the smallest gives).
+constexpr int kC4MaxSlices = 15; // counts up to 2^15 - 1
+
+__device__ __forceinline__ void c4_csa(uint32_t &carry, uint32_t &sum, uint32_t x, uint32_t y) {
+    const uint32_t z = sum;
+    sum = x ^ y ^ z;
+    carry = (x & y) | (x & z) | (y & z);
+}
+
+// Adds eight words to the counters of NS slices.
+template <int NS> __device__ __forceinline__ void c4_add8(uint32_t (&s)[NS], const uint32_t (&d)[8]) {
+    static_assert(NS >= 4, "eight words carry into slice 3");
+    uint32_t t0, t1, f0, f1, e;
+    c4_csa(t0, s[0], d[0], d[1]);
+    c4_csa(t1, s[0], d[2], d[3]);
+    c4_csa(f0, s[1], t0, t1);
+    c4_csa(t0, s[0], d[4], d[5]);
+    c4_csa(t1, s[0], d[6], d[7]);
+    c4_csa(f1, s[1], t0, t1);
+    c4_csa(e, s[2], f0, f1);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            n += __shfl_xor_sync(kFull, n, o);
-        if (lane == 0)
-            cnt = sat_add(cnt, (unsigned long long)n * (n - (n ? 1u : 0u)) / 2);
-        bal = __ballot_sync(kFull, u != 0);
+    for (int k = 3; k < NS; ++k) {
+        if (!e)
+            break;
+        const uint32_t t = s[k] & e;
+        s[k] ^= e;
+        e = t;
     }
-    return cnt;
+}
+
+// Sum of C(n, 2) over the 32 counters n of slices [0, L) restricted to mask:
+// n = sum 2^k s_k, so C(n, 2) = sum_k (4^k - 2^k) / 2 s_k + sum_{j<k} 2^(j+k) s_j s_k.
+template <int NS>
+__device__ __forceinline__ unsigned long long c4_pairs(uint32_t (&s)[NS], int L, uint32_t mask) {
+    unsigned long long tot = 0;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        if (k < L) {
+            s[k] &= mask;
+            tot += (unsigned long long)__popc(s[k]) * (((1ull << (2 * k)) - (1ull << k)) / 2);
+#pragma unroll
+            for (int j = 0; j < k; ++j)
+                tot += (unsigned long long)__popc(s[j] & s[k]) << (j + k);
+        }
+    }
+    return tot;
+}
+
+// Appends the set bits of this lane's word w (word index k) to ib in order,
+// group-wide (G lanes, mask gmask); returns the group's total.
+template <int G>
+__device__ __forceinline__ uint32_t c4_indices(uint32_t w, uint32_t k, uint16_t *ib, int glane, unsigned gmask) {
+    const uint32_t n = (uint32_t)__popc(w);
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(gmask, inc, o, G);
+        if (glane >= o)
+            inc += y;
+    }
+    uint32_t at = inc - n;
+    while (w) {
+        ib[at++] = (uint16_t)((k << 5) + (uint32_t)(__ffs(w) - 1));
+        w &= w - 1;
+    }
+    const uint32_t total = __shfl_sync(gmask, inc, G - 1, G);
+    __syncwarp(gmask);
+    return total;
+}
+
+// Rows in shared memory, W <= G words each (stride RS): a group of G lanes
+// counts the 4-cycles whose largest vertex is a; this lane's part is returned.
+// ib: D 16-bit entries of the group's own.
+template <int G, int NS>
+__device__ __forceinline__ unsigned long long wheel4_group(const uint32_t *rows, uint32_t RS, uint32_t a,
+                                                           uint16_t *ib, int glane, unsigned gmask) {
+    const uint32_t k = (uint32_t)glane, aw = a >> 5;
+    const uint32_t below = (1u << (a & 31)) - 1u; // bits of word aw below a
+    const uint32_t cm = k < aw ? 0xffffffffu : (k == aw ? below : 0u);
+    const uint32_t ra = k <= aw ? rows[(size_t)a * RS + k] & cm : 0u;
+    const uint32_t nb = c4_indices<G>(ra, k, ib, glane, gmask);
+    if (nb < 2)
+        return 0;
+    uint32_t s[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i)
+        s[i] = 0;
+    for (uint32_t i = 0; i < nb; i += 8) {
+        uint32_t d[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            d[q] = (k <= aw && i + q < nb) ? rows[(size_t)ib[i + q] * RS + k] : 0u;
+        c4_add8<NS>(s, d);
+    }
+    __syncwarp(gmask); // ib is rewritten by the group's next call
+    return c4_pairs<NS>(s, 32 - __clz((int)nb), cm);
 }
 
 template <int DEND, bool ENUM, int G, int MAXD>
@@ -1647,11 +1715,21 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         } else if constexpr (G == 0) {
             const uint64_t *r64 = reinterpret_cast<const uint64_t *>(rows);
             if (wheel) { // block-uniform; rows of the whole domain
+                // 8 lanes per vertex, rows of 8 words; index lists in the
+                // space of the row builder's arrays (free again):
+                // (3 pad + 1.75 nslots) words >= 17 maxD against 32 groups x D / 2
+                static_assert(2 * kThreadNW == 8, "8 words a row");
+                const int gl = lane & 7;
+                const unsigned gm = 0xffu << (lane & 24);
+                uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 3) * (size_t)((D + 1) & ~1u);
                 for (;;) {
-                    const uint32_t j = atomicAdd(&s_j, 1u);
+                    uint32_t j = 0;
+                    if (gl == 0)
+                        j = atomicAdd(&s_j, 1u);
+                    j = __shfl_sync(gm, j, 0, 8);
                     if (j >= D)
                         break;
-                    cnt = sat_add(cnt, wheel4_thread<kThreadNW>(r64, j));
+                    cnt = sat_add(cnt, wheel4_group<8, 9>(rows, 8, D - 1 - j, ib, gl, gm));
                 }
             } else if (DEND == 3 || pr.lp.free_from <= 2) { // block-uniform
                 // level 2 is the last or is counted in closed form: O(1) per level-1 vertex
@@ -1717,7 +1795,9 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     break;
                 if constexpr (G == 32) {
                     if (wheel) { // block-uniform; rows of the whole domain
-                        cnt = sat_add(cnt, wheel4_warp(rows, W, j, glane));
+                        uint16_t *ib =
+                            reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 5) * (size_t)((D + 1) & ~1u);
+                        cnt = sat_add(cnt, wheel4_group<32, 11>(rows, W, D - 1 - j, ib, glane, gmask));
                         continue;
                     }
                 }
@@ -1793,6 +1873,9 @@ __host__ __device__ __forceinline__ uint64_t nb_edges_offset(uint32_t D, uint32_
 __host__ __device__ __forceinline__ uint64_t large_root_words(uint32_t D, uint32_t rlo, bool nb = false) {
     return ((nb ? nb_edges_offset(D, rlo) + 2 : nb_deg_offset(D, rlo)) + 31) & ~(uint64_t)31;
 }
+
+// Tasks of a large root's walk: its level-1 vertices, or (4-wheel) the (a, strip) pairs.
+__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, int wheel4);
 
 __device__ __forceinline__ uint32_t find_batch(const uint32_t *__restrict__ start, uint32_t nb, uint32_t t) {
     // last b with start[b] <= t
@@ -2067,6 +2150,59 @@ __device__ __forceinline__ void wheel4_task(const uint32_t *__restrict__ bm, con
     __syncwarp(); // U back to zero before the warp's next task
 }
 
+// Roots whose rows have at most kC4StripMaxW words: the bit-sliced counters of
+// the medium tier (c4_add8) over the arena's rows. A task is (root, a, strip
+// of 32 words): lane k counts column word 32 s + k over every b of row(a)
+// below a. Strips keep the tasks of a hub's neighbourhood short: its largest a
+// have thousands of b and a dozen strips.
+// Task t of a root: strip s holds the a in [1024 s, D), largest first.
+constexpr uint32_t kC4StripMaxW = 512;
+__host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D) {
+    const uint32_t S = (D + 1023) / 1024;
+    return S * D - 512 * S * (S - 1);
+}
+static_assert((kC4StripMaxW * 32) >> kC4MaxSlices == 0, "a count fits the slices");
+
+__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, int wheel4) {
+    return wheel4 && (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D - j0;
+}
+
+__device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, uint32_t W, uint32_t D, uint32_t t,
+                                              uint16_t *ib, int lane, unsigned long long &cnt) {
+    uint32_t st = 0;
+    while (t >= D - 1024 * st) {
+        t -= D - 1024 * st;
+        ++st;
+    }
+    const uint32_t a = D - 1 - t, aw = a >> 5, k = 32 * st + (uint32_t)lane;
+    const uint32_t below = (1u << (a & 31)) - 1u;
+    const uint32_t *ra = bm + (size_t)a * W, *col = bm + k;
+    uint32_t s[kC4MaxSlices];
+#pragma unroll
+    for (int i = 0; i < kC4MaxSlices; ++i)
+        s[i] = 0;
+    uint32_t total = 0;
+    for (uint32_t w0 = 0; w0 <= aw; w0 += 32) {
+        const uint32_t wi = w0 + (uint32_t)lane;
+        uint32_t w = wi <= aw ? ra[wi] : 0u;
+        if (wi == aw)
+            w &= below;
+        const uint32_t nb = c4_indices<32>(w, wi, ib, lane, kFull);
+        total += nb;
+        for (uint32_t i = 0; i < nb; i += 8) {
+            uint32_t d[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                d[q] = (k <= aw && i + q < nb) ? col[(size_t)ib[i + q] * W] : 0u;
+            c4_add8<kC4MaxSlices>(s, d);
+        }
+        __syncwarp();
+    }
+    if (total >= 2)
+        cnt = sat_add(cnt, c4_pairs<kC4MaxSlices>(s, 32 - __clz((int)total),
+                                                  k < aw ? 0xffffffffu : (k == aw ? below : 0u)));
+}
+
 // A donated task of level P resumes the walk at that level over its
 // iteration range (the task's x[2 .. P-1] restored first).
 template <int P, int DEND, bool ENUM>
@@ -2257,6 +2393,7 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
     // and on exit)
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
+    __shared__ uint16_t s_ib[8][1024];
     PairRegs pr;
     uint32_t cur = 0xffffffffu;
     unsigned long long cnt = 0;
@@ -2283,6 +2420,10 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
         pair_domain(pr, r, beg, D, j0);
         const uint32_t W = (D + 31) >> 5;
         const uint32_t *rows = arena + bt.off[b]; // rows of the whole domain: rlo == 0
+        if (W <= kC4StripMaxW) {
+            c4_strip_task(rows, W, D, t - bt.tstart[b], s_ib[threadIdx.x >> 5], lane, cnt);
+            continue;
+        }
         RowLists rl;
         rl.cap = list_cap(W);
         rl.nzc = rows + (size_t)D * W;
@@ -2803,7 +2944,7 @@ __global__ void k_large_meta(const PairDev *__restrict__ pairs, const uint64_t *
         const uint32_t rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
         words[i] = large_root_words(D, rlo, pl.nbhd != kNbNone);
         chunks[i] = (D + kRowsPerChunk - 1) / kRowsPerChunk;
-        tasks[i] = D - j0;
+        tasks[i] = large_tasks(D, j0, pl.wheel4);
     }
 }
 
@@ -3407,7 +3548,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
         struct R {
             uint64_t item;
-            uint32_t D, j0, dend; // dend: the depth slot
+            uint32_t D, tasks, dend; // dend: the depth slot
             uint64_t words; // bitmap rows [rlo, D) of D bits and their word lists
         };
         std::vector<R> rs(nl);
@@ -3416,7 +3557,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             const uint32_t D = lD[i], rlo = pl.rows_needed == 2 ? 0u : (pl.rows_needed == 1 ? lj[i] : D);
             const uint64_t words = large_root_words(D, rlo, pl.nbhd != kNbNone);
             const PairDev &pdv = hp[(uint32_t)(litems[i] >> 32)];
-            rs[i] = R{litems[i], D, lj[i], depth_slot(pl, 4, pdv.en.out != nullptr), words};
+            rs[i] = R{litems[i], D, large_tasks(D, lj[i], pl.wheel4), depth_slot(pl, 4, pdv.en.out != nullptr), words};
         }
         std::sort(rs.begin(), rs.end(), [](const R &a, const R &b) { return a.D > b.D; });
         // batch boundaries and the arena size (largest batch)
@@ -3474,7 +3615,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 ts_all.push_back(0);
                 for (uint32_t e = 0; e < gp.second; ++e) {
                     const R &x = rs[i0 + gp.first + e];
-                    acc += x.D - x.j0;
+                    acc += x.tasks;
                     ts_all.push_back(acc);
                 }
             }

@@ -1,0 +1,39 @@
+"""4-wheel counts by bit-sliced counters (medium tier: rows in shared memory,
+large tier: strips of 32 words) against the oracle, at the edges of their
+words, strips and tiers and with counters that reach the highest slices."""
+import numpy as np
+import pytest
+
+import beep_b200 as B
+from beep_b200 import patterns as P
+from oracle import pyoracle as O
+from oracle import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_over(n, p, twins, seed):
+    """Hub 0 over n vertices with G(n, p) among them; with twins, the last two
+    of the n are joined to all the others, so that they have n - 2 common
+    neighbours in the hub's neighbourhood."""
+    rng = np.random.default_rng(seed)
+    m = int(p * n * (n - 1) / 2)
+    us = [np.zeros(n, np.int64), rng.integers(1, n + 1, m)]
+    vs = [np.arange(1, n + 1), rng.integers(1, n + 1, m)]
+    for t in (n - 1, n) if twins else ():
+        us.append(np.full(n - 2, t, np.int64))
+        vs.append(np.arange(1, n - 1))
+    return synth.to_csr(n + 1, np.concatenate(us), np.concatenate(vs))
+
+
+@pytest.mark.parametrize("n,p,twins", [
+    (64, 0.3, True), (65, 0.3, True), (96, 0.5, False), (255, 0.1, True), (256, 0.1, True), (257, 0.1, True),
+    (300, 0.5, False), (1023, 0.01, True), (1024, 0.01, True), (1025, 0.01, True), (2048, 0.004, True),
+    (2049, 0.004, True), (16384, 0.0003, True), (16385, 0.0003, True)])
+def test_hub_neighbourhoods(ctx, n, p, twins):
+    rp, col = hub_over(n, p, twins, n)
+    exp = O.count(rp, col, P.W5, apply_root_cap=False)["count"]
+    assert exp > 0
+    g = B.Graph.from_csr(ctx, rp, col)
+    assert B.count(g, P.W5) == exp
+    g.close()
