@@ -1145,6 +1145,15 @@ __device__ __forceinline__ uint32_t pair_rlo(const PairRegs &pr, uint32_t D, uin
 constexpr int kSmallWarps = 8;
 constexpr int kTinyMaxD = 16;
 
+// A walk of depth 6 or more multiplies a root's work by its density at every
+// level: one dense root of 256 vertices walked by one block took 172 ms of a
+// 187 ms launch (7-cliques, R-MAT s14 ef12). Launches of such depths therefore
+// list every root of more than kSplitMinD vertices `parts` times; each part
+// builds the rows again (a small share of its walk) and takes every parts-th
+// chunk of the walk. (6- and 7-cliques there together: 193 -> 31 ms.)
+constexpr uint32_t kSplitMinD = 24;
+inline uint32_t walk_parts(int dend, bool enumerate) { return enumerate || dend < 6 ? 1u : (dend == 6 ? 8u : 32u); }
+
 template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigned long long v, unsigned gmask) {
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1)
@@ -1309,7 +1318,7 @@ __device__ __forceinline__ unsigned long long wheel4_group(const uint32_t *rows,
 template <int DEND, bool ENUM, int G, int MAXD>
 __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(const PairDev *__restrict__ pairs,
                                                            const uint64_t *__restrict__ items, uint32_t nitems,
-                                                           unsigned long long *exit_t) {
+                                                           uint32_t parts, unsigned long long *exit_t) {
     constexpr int NG = kSmallWarps * 32 / G; // groups per block
     __shared__ uint64_t s_rows[NG][MAXD];
     __shared__ uint32_t s_A[NG][MAXD];
@@ -1326,8 +1335,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
     EnumCtx ec;
     unsigned long long cnt = 0;
     bool wheel = false; // the 4-wheel's closed form (counts)
-    for (uint32_t ri = blockIdx.x * NG + gid; ri < nitems; ri += gridDim.x * NG) {
-        const uint64_t it = items[ri];
+    // largest domains first (the list rises): the last roots taken are short
+    for (uint64_t vi = blockIdx.x * NG + gid; vi < (uint64_t)nitems * parts; vi += gridDim.x * NG) {
+        const uint32_t ri = (uint32_t)(vi / parts), part = (uint32_t)(vi - (uint64_t)ri * parts);
+        const uint64_t it = items[nitems - 1 - ri];
         const uint32_t p = item_pair(it), r = item_root(it);
         if (p != cur) { // group-uniform
             cnt = group_sum<G>(cnt, gmask);
@@ -1349,6 +1360,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
         uint32_t beg, D, j0;
         pair_domain(pr, r, beg, D, j0);
         const uint32_t rlo = pair_rlo(pr, D, j0);
+        const bool split = parts > 1 && D > kSplitMinD && pr.lp.free_from > 2;
+        if (part > 0 && !split) // the root's first part takes it whole
+            continue;
+        const uint32_t nparts = split ? parts : 1u;
         for (uint32_t i = glane; i < D; i += G) {
             A[i] = pr.v.col[beg + i];
             rows[i] = 0;
@@ -1390,7 +1405,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
             group_excl_scan<G>(s_cnt, n1, glane, gmask);
             __syncwarp(gmask);
             const uint32_t T = s_cnt[n1];
-            for (uint32_t t = glane; t < T; t += G) {
+            for (uint32_t t = part * G + glane; t < T; t += nparts * G) {
                 uint32_t a = 0, b = n1;
                 while (b - a > 1) {
                     const uint32_t mid = (a + b) >> 1;
@@ -1594,6 +1609,125 @@ __device__ __forceinline__ void nbhd_medium_warp(int form, const uint32_t *rows,
 }
 
 // ---------------------------------------------------------------------------
+// cliques in the medium tier (counts only). Row i holds only the neighbours
+// above i, RS (odd) words apart, so the candidates that follow x1 < .. < xp are
+// the AND of their rows with no bound to apply, and half the row bits are set.
+// One thread per (x1, x2) edge of the neighbourhood graph. The last two levels
+// are taken together: the edges inside a candidate set S are counted word pair
+// by word pair, S's word k giving the vertices y and its word w >= k, held in
+// a register, the part of row(y) to count -- one shared load, an AND and a
+// popcount per (y, word) instead of a fresh AND of every row. In the
+// ascending order the dense part of a neighbourhood sits at its end, so a leaf
+// touches about two words of the up to 32 (R-MAT s17 ef28: 1.9 for D <= 256,
+// 2.5 for D <= 1024); lanes that own whole walks use them all, where a warp
+// per walk used two or three of its 32 lanes. The odd stride spreads the
+// lanes' rows over the banks. Bound by issue and by shared loads with bank
+// conflicts. (5-cliques on R-MAT s17 ef28: 470 -> 18.3 ms.)
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ uint32_t clique_stride(uint32_t W) { return W | 1u; }
+
+// Word k of the candidates that follow x[1..NP].
+template <int NP>
+__device__ __forceinline__ uint32_t clique_word(const uint32_t *rows, uint32_t RS, const uint32_t (&x)[kMaxQ],
+                                                uint32_t k) {
+    uint32_t w = rows[x[1] * RS + k];
+#pragma unroll
+    for (int q = 2; q <= NP; ++q)
+        w &= rows[x[q] * RS + k];
+    return w;
+}
+
+// Ways to complete x[1..P] to x[1..DEND-1].
+template <int P, int DEND>
+__device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t (&x)[kMaxQ],
+                                            unsigned long long &cnt) {
+    uint32_t n = 0;
+    if constexpr (P == DEND - 2) {
+        for (uint32_t k = x[P] >> 5; k < W; ++k)
+            n += (uint32_t)__popc(clique_word<P>(rows, RS, x, k));
+        cnt += n;
+    } else if constexpr (P == DEND - 3) {
+        for (uint32_t k = x[P] >> 5; k < W; ++k) {
+            const uint32_t sk = clique_word<P>(rows, RS, x, k);
+            if (!sk)
+                continue;
+            const uint32_t *rk = rows + (k << 5) * RS;
+            for (uint32_t b = sk; b;) { // y < z in word k: b without y is S above y
+                const uint32_t *ry = rk + (uint32_t)(__ffs(b) - 1) * RS;
+                b &= b - 1;
+                n += (uint32_t)__popc(ry[k] & b);
+            }
+            for (uint32_t w = k + 1; w < W; ++w) {
+                const uint32_t sw = clique_word<P>(rows, RS, x, w);
+                if (!sw)
+                    continue;
+                for (uint32_t b = sk; b; b &= b - 1)
+                    n += (uint32_t)__popc(rk[(uint32_t)(__ffs(b) - 1) * RS + w] & sw);
+            }
+        }
+        cnt += n;
+    } else {
+        for (uint32_t k = x[P] >> 5; k < W; ++k)
+            for (uint32_t b = clique_word<P>(rows, RS, x, k); b; b &= b - 1) {
+                x[P + 1] = (k << 5) + (uint32_t)(__ffs(b) - 1);
+                clique_walk<P + 1, DEND>(rows, RS, W, x, cnt);
+            }
+    }
+}
+
+// Every clique of a root's domain graph (block-wide): warps take 32 (x1, x2)
+// edges at a time from s_j, chunks part, part + parts, ..; s_cnt: D + 1 words.
+template <int DEND>
+__device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
+                                            uint32_t *s_cnt, uint32_t *s_j, uint32_t part, uint32_t parts,
+                                            unsigned long long &cnt) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = threadIdx.x; i < D; i += blockDim.x) {
+        uint32_t c = 0;
+        for (uint32_t k = i >> 5; k < W; ++k)
+            c += (uint32_t)__popc(rows[i * RS + k]);
+        s_cnt[i] = c;
+    }
+    if (threadIdx.x == 0)
+        *s_j = part;
+    __syncthreads();
+    if (threadIdx.x < 32)
+        warp_excl_scan(s_cnt, D, (int)threadIdx.x);
+    __syncthreads();
+    const uint32_t T = s_cnt[D];
+    for (;;) {
+        uint32_t c = 0;
+        if (lane == 0)
+            c = atomicAdd(s_j, parts);
+        const uint32_t t = (__shfl_sync(kFull, c, 0) << 5) + (uint32_t)lane;
+        if (t - (uint32_t)lane >= T)
+            break;
+        if (t < T) {
+            uint32_t a = 0, b = D; // last i with s_cnt[i] <= t
+            while (b - a > 1) {
+                const uint32_t mid = (a + b) >> 1;
+                if (s_cnt[mid] <= t)
+                    a = mid;
+                else
+                    b = mid;
+            }
+            uint32_t x[kMaxQ];
+            x[1] = a;
+            uint32_t j = t - s_cnt[a], k = a >> 5, w = rows[a * RS + k];
+            for (uint32_t pc = (uint32_t)__popc(w); j >= pc; pc = (uint32_t)__popc(w)) {
+                j -= pc;
+                w = rows[a * RS + ++k];
+            }
+            for (; j; --j)
+                w &= w - 1;
+            x[2] = (k << 5) + (uint32_t)(__ffs(w) - 1);
+            clique_walk<2, DEND>(rows, RS, W, x, cnt);
+        }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
 // medium tier: block per root, bitmap in shared memory
 // ---------------------------------------------------------------------------
 // G lanes per level-1 vertex (32: domains of up to 1024 vertices, rows of up
@@ -1606,7 +1740,8 @@ __device__ __forceinline__ void nbhd_medium_warp(int form, const uint32_t *rows,
 template <int DEND, bool ENUM, int G>
 __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 : 2) : 1) k_medium(const PairDev *__restrict__ pairs,
                                                 const uint64_t *__restrict__ items, uint32_t nitems,
-                                                unsigned *cursor, uint32_t maxD, unsigned long long *exit_t) {
+                                                uint32_t parts, unsigned *cursor, uint32_t maxD,
+                                                unsigned long long *exit_t) {
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t s_ri, s_j, s_full;
     const int lane = threadIdx.x & 31;
@@ -1624,13 +1759,14 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
     EnumCtx ec;
     unsigned long long cnt = 0;
     bool wheel = false; // the 4-wheel's closed form (counts)
+    bool clique = false; // upper rows, clique_root (counts)
     int nbform = kNbNone; // a neighbourhood-statistics form (counts)
     unsigned long long nb_plus = 0, nb_minus = 0;
     for (;;) {
         if (threadIdx.x == 0)
             s_ri = atomicAdd(cursor, 1u);
         __syncthreads();
-        const uint32_t ri = s_ri;
+        const uint32_t ri = s_ri / parts, part = s_ri - ri * parts;
         if (ri >= nitems)
             break;
         const uint64_t it = items[ri];
@@ -1651,6 +1787,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 make_ec(ec, pairs[p].en, pairs[p].pl, pr.v);
             wheel = DEND == 5 && !ENUM && pairs[p].pl.wheel4;
             nbform = (DEND == 5 && !ENUM) ? (int)pairs[p].pl.nbhd : (int)kNbNone;
+            clique = DEND >= 4 && !ENUM && pairs[p].pl.clique;
         }
         if constexpr (ENUM) { // k tuples reserved: skip the root before its rows are built
             if (threadIdx.x == 0)
@@ -1664,19 +1801,31 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         uint32_t beg, D, j0;
         pair_domain(pr, r, beg, D, j0);
         const uint32_t rlo = pair_rlo(pr, D, j0);
+        const bool split = parts > 1 && D > kSplitMinD;
+        if (part > 0 && !split) { // block-uniform: the root's first part takes it whole
+            __syncthreads();
+            continue;
+        }
+        const uint32_t nparts = split ? parts : 1u;
         const uint32_t W = (D + 31) >> 5;
-        const uint32_t row_words = G == 0 ? 2 * kThreadNW : W; // 32-bit words per row
+        // 32-bit words per row
+        const uint32_t row_words = clique ? clique_stride(W) : (G == 0 ? 2 * kThreadNW : W);
         for (uint32_t i = threadIdx.x; i < D; i += blockDim.x)
             A[i] = pr.v.col[beg + i];
         for (uint32_t i = threadIdx.x; i < (D - rlo) * row_words; i += blockDim.x)
             rows[i] = 0;
         if (threadIdx.x == 0)
-            s_j = j0;
+            s_j = G == 0 ? j0 : j0 + part;
         __syncthreads();
         if (rlo < D) { // block-uniform
             hash_build(A, D, hkeys, hidx, nslots, hshift);
             __syncthreads();
-            if constexpr (G == 0) {
+            if (clique) {
+                build_rows_hashed(pr.v, 1, A, D, 0, s_hb, s_pre, s_len, hkeys, hidx, nslots, hshift,
+                                  [&](uint32_t i, uint32_t k) { // i < k
+                                      atomicOr(&rows[i * row_words + (k >> 5)], 1u << (k & 31));
+                                  });
+            } else if constexpr (G == 0) {
                 unsigned long long *r64 = reinterpret_cast<unsigned long long *>(rows);
                 build_rows_hashed(pr.v, pr.asc, A, D, rlo, s_hb, s_pre, s_len, hkeys, hidx, nslots, hshift,
                                   [&](uint32_t i, uint32_t k) {
@@ -1711,7 +1860,14 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 stats_done = true;
             }
         }
-        if (stats_done) {
+        bool clique_done = false;
+        if constexpr (DEND >= 4 && !ENUM) {
+            if (clique) {
+                clique_root<DEND>(rows, row_words, W, D, s_pre, &s_j, part, nparts, cnt);
+                clique_done = true;
+            }
+        }
+        if (stats_done || clique_done) {
         } else if constexpr (G == 0) {
             const uint64_t *r64 = reinterpret_cast<const uint64_t *>(rows);
             if (wheel) { // block-uniform; rows of the whole domain
@@ -1733,7 +1889,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 }
             } else if (DEND == 3 || pr.lp.free_from <= 2) { // block-uniform
                 // level 2 is the last or is counted in closed form: O(1) per level-1 vertex
-                for (;;) {
+                while (part == 0) {
                     const uint32_t j = atomicAdd(&s_j, 1u);
                     if (j >= D)
                         break;
@@ -1760,7 +1916,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     warp_excl_scan(s_cnt, n1, (int)threadIdx.x);
                 __syncthreads();
                 const uint32_t T = s_cnt[n1];
-                for (uint32_t t = threadIdx.x; t < T; t += blockDim.x) {
+                for (uint32_t t = part * blockDim.x + threadIdx.x; t < T; t += nparts * blockDim.x) {
                     uint32_t a = 0, b = n1; // last i with s_cnt[i] <= t
                     while (b - a > 1) {
                         const uint32_t mid = (a + b) >> 1;
@@ -1789,7 +1945,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
             for (;;) {
                 uint32_t j = 0;
                 if (glane == 0)
-                    j = atomicAdd(&s_j, 1u);
+                    j = atomicAdd(&s_j, nparts);
                 j = __shfl_sync(gmask, j, 0, G);
                 if (j >= D)
                     break;
@@ -3021,13 +3177,13 @@ __global__ void k_alg_bytes(const PairDev *__restrict__ pairs, const uint64_t *_
 
 template <bool ENUM>
 beep_status launch_small(int dend, int group, int grid, cudaStream_t s, const PairDev *pairs, const uint64_t *items,
-                         uint32_t n, unsigned long long *exit_t) {
+                         uint32_t n, uint32_t parts, unsigned long long *exit_t) {
 #define BEEP_CASE(D)                                                                                               \
     case D:                                                                                                        \
         if (group == 8)                                                                                            \
-            k_small<D, ENUM, 8, kTinyMaxD><<<grid, kSmallWarps * 32, 0, s>>>(pairs, items, n, exit_t);              \
+            k_small<D, ENUM, 8, kTinyMaxD><<<grid, kSmallWarps * 32, 0, s>>>(pairs, items, n, parts, exit_t);              \
         else                                                                                                       \
-            k_small<D, ENUM, 32, kSmallMaxD><<<grid, kSmallWarps * 32, 0, s>>>(pairs, items, n, exit_t);            \
+            k_small<D, ENUM, 32, kSmallMaxD><<<grid, kSmallWarps * 32, 0, s>>>(pairs, items, n, parts, exit_t);            \
         break;
     BEEP_DEPTH_SWITCH(dend, BEEP_CASE)
 #undef BEEP_CASE
@@ -3122,6 +3278,7 @@ struct LaunchRec {
     size_t smem = 0;
     const uint64_t *items = nullptr;
     uint32_t n = 0, maxD = 0;
+    uint32_t parts = 1; // small and medium tiers: times every root is listed (walk_parts)
     unsigned *cursor = nullptr;
     Batch bt{};
     void *mptr = nullptr;
@@ -3682,8 +3839,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         uint64_t *list = nullptr;
         BEEP_TRY(make_list(k, list));
         const uint32_t maxD = tier_max[k];
-        // 32-bit words per row: 8 (4 x 64 bits) in the thread-mode sub-tier
-        const uint32_t W = sub == 0 ? 2 * kThreadNW : (maxD + 31) / 32;
+        // 32-bit words per row: 8 (4 x 64 bits) in the thread-mode sub-tier;
+        // clique rows take an odd number
+        const uint32_t W = clique_stride(sub == 0 ? 2 * kThreadNW : (maxD + 31) / 32);
         const size_t pad = (maxD + 4) & ~3u;
         // the domain hash: nslots ids, nslots 16-bit indices and the filter
         const size_t nslots = hash_slots(maxD);
@@ -3700,6 +3858,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             r.dend = sl % kDepths;
             r.enumerate = sl >= kDepths;
             r.group = sub == 0 ? 0 : 32;
+            r.parts = walk_parts(r.dend, r.enumerate);
             r.grid = ctx->num_sms * per_sm;
             r.block = block;
             r.smem = smem;
@@ -3732,7 +3891,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 r.dend = sl % kDepths;
                 r.enumerate = sl >= kDepths;
                 r.group = group;
-                r.grid = (int)std::min<int64_t>(((int64_t)cnt + per_block - 1) / per_block,
+                r.parts = part == 0 ? 1u : walk_parts(r.dend, r.enumerate);
+                r.grid = (int)std::min<int64_t>(((int64_t)cnt * r.parts + per_block - 1) / per_block,
                                                 (int64_t)ctx->num_sms * 8);
                 r.block = kSmallWarps * 32;
                 r.items = list + first;
@@ -3895,15 +4055,15 @@ beep_status issue(Ctx *ctx, LaunchPlan *lp, bool timing, bool serial, bool stall
 #define BEEP_CASE(D)                                                                                               \
     case D:                                                                                                        \
         if (r.enumerate && r.group == 0)                                                                           \
-            k_medium<D, true, 0><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.cursor, r.maxD, ex); \
+            k_medium<D, true, 0><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.parts, r.cursor, r.maxD, ex); \
         else if (r.enumerate)                                                                                      \
-            k_medium<D, true, 32><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.cursor, r.maxD,    \
+            k_medium<D, true, 32><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.parts, r.cursor, r.maxD,    \
                                                                    ex);                                           \
         else if (r.group == 0)                                                                                     \
-            k_medium<D, false, 0><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.cursor, r.maxD,    \
+            k_medium<D, false, 0><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.parts, r.cursor, r.maxD,    \
                                                                    ex);                                           \
         else                                                                                                       \
-            k_medium<D, false, 32><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.cursor, r.maxD,   \
+            k_medium<D, false, 32><<<r.grid, r.block, r.smem, rs>>>(lp->d_pairs, r.items, r.n, r.parts, r.cursor, r.maxD,   \
                                                                     ex);                                          \
         break;
             BEEP_DEPTH_SWITCH(r.dend, BEEP_CASE)
@@ -3920,9 +4080,9 @@ beep_status issue(Ctx *ctx, LaunchPlan *lp, bool timing, bool serial, bool stall
             break;
         case LaunchRec::kSmall:
             if (r.enumerate)
-                BEEP_TRY(launch_small<true>(r.dend, r.group, r.grid, rs, lp->d_pairs, r.items, r.n, ex));
+                BEEP_TRY(launch_small<true>(r.dend, r.group, r.grid, rs, lp->d_pairs, r.items, r.n, r.parts, ex));
             else
-                BEEP_TRY(launch_small<false>(r.dend, r.group, r.grid, rs, lp->d_pairs, r.items, r.n, ex));
+                BEEP_TRY(launch_small<false>(r.dend, r.group, r.grid, rs, lp->d_pairs, r.items, r.n, r.parts, ex));
             st.small_launches++;
             break;
         }

@@ -75,6 +75,7 @@ struct DevPlan {
     uint32_t sym0;           // bit p: position p must follow position 0
     int32_t wheel4;          // the 4-wheel's plan: counted per (x1, x3) pair in closed form
     int32_t nbhd;            // NbhdForm: in the large tier, counted from neighbourhood statistics
+    int32_t clique;          // a complete query, every position ordered after the ones before it
 };
 
 // Five-vertex central queries whose count at a root v follows from statistics

@@ -354,6 +354,11 @@ beep_status compile_plan(int32_t qn, const std::vector<int32_t> &rp, const std::
         else if (edges == 5 && seq(2, 2, 3, 3) && hubs == 2 && universal_after)
             D.nbhd = kNbDiamond;
     }
+    // A clique: every position adjacent to and ordered after all before it,
+    // so a walk reads only the part of a row above its vertex.
+    D.clique = D.restricted && D.asc && D.dend == qn && qn >= 4;
+    for (int p = 2; p < qn; ++p)
+        D.clique = D.clique && D.back[p] == ((1u << p) - 2u) && after[p] == ((1u << p) - 2u);
     if (D.nbhd)
         D.rows_needed = 2; // the statistics read every row of the neighbourhood
     P.nbhd = D.nbhd;
