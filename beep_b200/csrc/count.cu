@@ -1087,6 +1087,7 @@ struct PairDev {
     EnumDev en;                // enumeration output (out == nullptr: none)
     uint32_t min_deg;          // roots: degree >= max_qdeg ...
     uint32_t cap_deg;          // ... and < cap_deg (reference root cap, else 2^32-1)
+    uint32_t sup;              // counted from degrees and triangle counts (SupForm): no items
     uint32_t shard_mod;        // > 1: only roots whose input id % shard_mod == shard_rem
     uint32_t shard_rem;
 };
@@ -2966,6 +2967,323 @@ __global__ void k_gen_tasks(const uint32_t *__restrict__ D, const uint32_t *__re
 }
 
 // ---------------------------------------------------------------------------
+// degree and triangle-count forms (SupForm)
+//
+// Every triangle of a view is found once, at its lowest vertex: for an
+// oriented edge (u, v), u < v, the shorter of u's neighbours above v and v's
+// neighbours above v is looked up in the other list. The oriented lists are
+// short whatever the hubs (184 entries at most on R-MAT s20 ef3, whose largest
+// degree is 18,500), so no root needs a bitmap, and one launch over the edges
+// replaces the classification, the item sort and a row-building kernel per
+// tier. A warp takes 32 consecutive CSR entries; their lookups are flattened
+// over the lanes, two in flight per lane. The lists and the searched prefixes
+// sit in L1/L2; the pass is bound by the dependent loads of the binary
+// searches (7 a lookup). (4-clique and diamond step on R-MAT s20 ef3: 3.85 ->
+// 2.33 ms, with one view for both; tailed triangle on a power-law graph of 2^18
+// vertices from raw edges: 14.0 -> 6.4 ms.)
+// ---------------------------------------------------------------------------
+struct SupView {
+    ViewDev v;
+    uint32_t n;
+    uint64_t eoff;           // first entry of the view in the flattened entries (a multiple of 32)
+    uint64_t voff;           // the same for its vertices
+    uint32_t *cnt;           // triangles of every entry (u, v), u < v; null: not needed
+    unsigned long long *tv;  // twice the triangles of every vertex; null: not needed
+    unsigned long long *out[kSupForms]; // counters of the forms (null: not asked for)
+};
+
+__device__ __forceinline__ uint32_t sup_find_view(const SupView *__restrict__ views, uint32_t nv, uint64_t e) {
+    uint32_t lo = 0, hi = nv;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (views[mid].eoff <= e)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// The vertex whose row holds entry e: last u in [lo, hi) with rp[u] <= e.
+__device__ __forceinline__ uint32_t sup_row_of(const uint32_t *__restrict__ rp, uint32_t lo, uint32_t hi, uint32_t e) {
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (rp[mid] <= e)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Row of entry e0 + lane for the lanes with e0 + lane < m (no row is empty,
+// so it is within 31 rows of e0's).
+__device__ __forceinline__ uint32_t sup_warp_row(const uint32_t *__restrict__ rp, uint32_t n, uint32_t e0,
+                                                 uint32_t e) {
+    const uint32_t u0 = sup_row_of(rp, 0, n, e0);
+    return sup_row_of(rp, u0, min(n, u0 + 32), e);
+}
+
+constexpr int kSupWarps = 8;
+
+__global__ void __launch_bounds__(kSupWarps * 32) k_sup_triangles(const SupView *__restrict__ views, uint32_t nv,
+                                                                  uint64_t nchunks, unsigned long long *exit_t) {
+    __shared__ uint32_t s_pre[kSupWarps][33], s_it[kSupWarps][32], s_lo[kSupWarps][32], s_hi[kSupWarps][32];
+    __shared__ uint32_t s_c[kSupWarps][32];
+    __shared__ unsigned long long s_f1[kSupWarps][32], s_f2[kSupWarps][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint32_t cur = 0xffffffffu;
+    SupView sv{};
+    unsigned long long tri = 0, e1 = 0, e2 = 0;
+    auto flush = [&]() {
+        if (sv.out[kSupTriangle]) {
+            tri = warp_sum(tri);
+            if (lane == 0)
+                flush_count(sv.out[kSupTriangle], tri);
+        }
+        if (sv.out[kSupEdgeIso]) {
+            e1 = warp_sum(e1);
+            if (lane == 0)
+                flush_count(sv.out[kSupEdgeIso], e1);
+        }
+        if (sv.out[kSupEdgeIso2]) {
+            e2 = warp_sum(e2);
+            if (lane == 0)
+                flush_count(sv.out[kSupEdgeIso2], e2);
+        }
+        tri = e1 = e2 = 0;
+    };
+    // chunks are dealt out in turn: the dense part of a graph (consecutive
+    // entries) spreads over every warp
+    const uint64_t nwarps = (uint64_t)gridDim.x * kSupWarps;
+    for (uint64_t c = (uint64_t)blockIdx.x * kSupWarps + wp; c < nchunks; c += nwarps) {
+        const uint32_t vi = nv == 1 ? 0u : sup_find_view(views, nv, c * 32);
+        if (vi != cur) {
+            if (cur != 0xffffffffu)
+                flush();
+            cur = vi;
+            sv = views[vi];
+        }
+        const uint32_t *rp = sv.v.rp, *col = sv.v.col;
+        const uint32_t m = rp[sv.n], eb = (uint32_t)(c * 32 - sv.eoff), e = eb + (uint32_t)lane;
+        const bool weights = sv.out[kSupEdgeIso] || sv.out[kSupEdgeIso2];
+        if (eb >= m)
+            continue;
+        uint32_t work = 0, it = 0, lo = 0, hi = 0;
+        unsigned long long f1 = 0, f2 = 0;
+        if (e < m) {
+            const uint32_t u = sup_warp_row(rp, sv.n, eb, e);
+            const uint32_t ub = rp[u], ue = rp[u + 1];
+            if (e >= ub + sv.v.split[u]) {
+                const uint32_t v = col[e], vb = rp[v], ve = rp[v + 1], vs = vb + sv.v.split[v];
+                const uint32_t na = ue - e - 1, nb = ve - vs;
+                if (na && nb) {
+                    const bool by_u = na <= nb; // the shorter list is walked, the other searched
+                    work = by_u ? na : nb;
+                    it = by_u ? e + 1 : vs;
+                    lo = by_u ? vs : e + 1;
+                    hi = by_u ? ve : ue;
+                    if (weights) {
+                        f1 = (unsigned long long)(ue - ub - 2) + (ve - vb - 2);
+                        f2 = sat_add(binom2(ue - ub - 2), binom2(ve - vb - 2));
+                    }
+                }
+            }
+        }
+        uint32_t inc = work;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o)
+                inc += y;
+        }
+        const uint32_t T = __shfl_sync(kFull, inc, 31);
+        if (T == 0)
+            continue;
+        __syncwarp();
+        s_pre[wp][lane] = inc - work;
+        s_it[wp][lane] = it - (inc - work); // entry of lookup t: s_it + t
+        s_lo[wp][lane] = lo;
+        s_hi[wp][lane] = hi;
+        if (sv.cnt)
+            s_c[wp][lane] = 0;
+        if (weights) {
+            s_f1[wp][lane] = f1;
+            s_f2[wp][lane] = f2;
+        }
+        __syncwarp();
+        constexpr int kU = 2; // lookups in flight per lane
+        for (uint32_t t = (uint32_t)lane; t < T; t += 32 * kU) {
+            uint32_t own[kU], pi[kU], w[kU], l[kU], h[kU];
+#pragma unroll
+            for (int j = 0; j < kU; ++j) {
+                const uint32_t tj = t + 32u * j;
+                own[j] = 0;
+                l[j] = h[j] = pi[j] = w[j] = 0;
+                if (tj < T) {
+                    uint32_t a = 0, b = 32; // last lane with s_pre <= tj: the one whose lookups hold tj
+                    while (b - a > 1) {
+                        const uint32_t mid = (a + b) >> 1;
+                        if (s_pre[wp][mid] <= tj)
+                            a = mid;
+                        else
+                            b = mid;
+                    }
+                    own[j] = a;
+                    pi[j] = s_it[wp][a] + tj;
+                    w[j] = col[pi[j]];
+                    l[j] = s_lo[wp][a];
+                    h[j] = s_hi[wp][a];
+                }
+            }
+            uint32_t end[kU];
+#pragma unroll
+            for (int j = 0; j < kU; ++j)
+                end[j] = h[j];
+            // lower bounds of both, step by step
+            bool more = true;
+            while (more) {
+                more = false;
+#pragma unroll
+                for (int j = 0; j < kU; ++j)
+                    if (l[j] < h[j]) {
+                        const uint32_t mid = (l[j] + h[j]) >> 1;
+                        if (col[mid] < w[j])
+                            l[j] = mid + 1;
+                        else
+                            h[j] = mid;
+                        more = more || l[j] < h[j];
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < kU; ++j) {
+                if (!(l[j] < end[j] && col[l[j]] == w[j]))
+                    continue;
+                ++tri;
+                if (weights) {
+                    const unsigned long long d = (unsigned long long)(rp[w[j] + 1] - rp[w[j]]) - 2;
+                    e1 = sat_add(e1, s_f1[wp][own[j]] + d);
+                    e2 = sat_add(e2, sat_add(s_f2[wp][own[j]], binom2(d)));
+                }
+                if (sv.cnt) {
+                    atomicAdd(&s_c[wp][own[j]], 1u);
+                    atomicAdd(&sv.cnt[pi[j]], 1u);
+                    atomicAdd(&sv.cnt[l[j]], 1u);
+                }
+            }
+        }
+        __syncwarp();
+        if (sv.cnt && s_c[wp][lane])
+            atomicAdd(&sv.cnt[e], s_c[wp][lane]);
+    }
+    if (cur != 0xffffffffu)
+        flush();
+    if (lane == 0)
+        record_exit(exit_t);
+}
+
+// The forms that are sums over the edges of their triangle counts, and every
+// vertex's triangles (twice their number) where a form needs them. Bound by
+// reading the counts (4 bytes an entry); rows are found only for warps that
+// hold an edge with a triangle.
+__global__ void __launch_bounds__(256) k_sup_edges(const SupView *__restrict__ views, uint32_t nv, uint64_t nchunks) {
+    const int lane = threadIdx.x & 31;
+    uint32_t cur = 0xffffffffu;
+    SupView sv{};
+    unsigned long long sum2 = 0, sum3 = 0, wi = 0;
+    auto flush = [&]() {
+        if (sv.out[kSupDiamond] || sv.out[kSupTwoEdges]) {
+            sum2 = warp_sum(sum2);
+            if (lane == 0 && sv.out[kSupDiamond])
+                flush_count(sv.out[kSupDiamond], sum2);
+            if (lane == 0 && sv.out[kSupTwoEdges])
+                flush_count(sv.out[kSupTwoEdges] + 4, sat_add(sum2, sum2));
+        }
+        if (sv.out[kSupBook3]) {
+            sum3 = warp_sum(sum3);
+            if (lane == 0)
+                flush_count(sv.out[kSupBook3], sum3);
+        }
+        if (sv.out[kSupWedgeIso]) {
+            wi = warp_sum(wi);
+            if (lane == 0)
+                flush_count(sv.out[kSupWedgeIso], wi);
+        }
+        sum2 = sum3 = wi = 0;
+    };
+    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nwarps) {
+        const uint32_t vi = nv == 1 ? 0u : sup_find_view(views, nv, c * 32);
+        if (vi != cur) {
+            if (cur != 0xffffffffu)
+                flush();
+            cur = vi;
+            sv = views[vi];
+        }
+        if (!sv.cnt)
+            continue;
+        const uint32_t *rp = sv.v.rp;
+        const uint32_t m = rp[sv.n], eb = (uint32_t)(c * 32 - sv.eoff), e = eb + (uint32_t)lane;
+        const uint32_t x = e < m ? sv.cnt[e] : 0u;
+        if (!__ballot_sync(kFull, x != 0))
+            continue;
+        if (x >= 2)
+            sum2 = sat_add(sum2, binom2(x));
+        if (x >= 3 && sv.out[kSupBook3])
+            sum3 = add_binom(sum3, x, 3);
+        if (x && (sv.out[kSupWedgeIso] || sv.tv)) {
+            const uint32_t u = sup_warp_row(rp, sv.n, eb, e), v = sv.v.col[e];
+            if (x >= 2) {
+                const unsigned long long d = (unsigned long long)(rp[u + 1] - rp[u]) + (rp[v + 1] - rp[v]) - 6;
+                wi = sat_add(wi, sat_mul(binom2(x), d));
+            }
+            if (sv.tv) {
+                atomicAdd(&sv.tv[u], (unsigned long long)x);
+                atomicAdd(&sv.tv[v], (unsigned long long)x);
+            }
+        }
+    }
+    if (cur != 0xffffffffu)
+        flush();
+}
+
+// The forms that are sums over the vertices: stars and the pairs of triangles
+// at a vertex.
+__global__ void __launch_bounds__(256) k_sup_vertices(const SupView *__restrict__ views, uint32_t nv) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = 0; i < nv; ++i) {
+        const SupView &sv = views[i];
+        if (!sv.tv && !sv.out[kSupStar2] && !sv.out[kSupStar3] && !sv.out[kSupStar4])
+            continue;
+        unsigned long long st[3] = {0, 0, 0}, tt = 0;
+        for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < sv.n;
+             v += (uint64_t)gridDim.x * blockDim.x) {
+            const uint32_t d = sv.v.rp[v + 1] - sv.v.rp[v];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (sv.out[kSupStar2 + k])
+                    st[k] = add_binom(st[k], d, k + 2);
+            if (sv.tv) {
+                const unsigned long long t = sv.tv[v] / 2;
+                tt = sat_add(tt, sat_mul(t & 1 ? t : t / 2, t & 1 ? (t - 1) / 2 : (t ? t - 1 : 0)));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (sv.out[kSupStar2 + k]) {
+                const unsigned long long x = warp_sum(st[k]);
+                if (lane == 0)
+                    flush_count(sv.out[kSupStar2 + k], x);
+            }
+        if (sv.tv) {
+            tt = warp_sum(tt);
+            if (lane == 0)
+                flush_count(sv.out[kSupTwoEdges] + 2, tt);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // root classification over the vertices of every pair (flattened index)
 // ---------------------------------------------------------------------------
 constexpr int kTiers = 5;   // 1 small (D <= 64), 2 medium (<= 256), 3 medium (<= 1024), 4 large,
@@ -2989,9 +3307,13 @@ __device__ __forceinline__ uint32_t find_pair(const uint64_t *__restrict__ offs,
 // largest domain and per (tier, depth) the number of roots.
 __global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__restrict__ offs, uint32_t npairs,
                            uint64_t N, TierCfg cfg, uint8_t *tier, uint32_t *dom, unsigned *tier_max,
-                           unsigned *tier_depth, unsigned *tiny_depth, unsigned long long *large_words) {
+                           unsigned *tier_depth, unsigned *tiny_depth, unsigned long long *large_words,
+                           unsigned *sup_tiers) {
     __shared__ unsigned s_hist[kTiers * kSlots];
     __shared__ unsigned s_tiny[kSlots];
+    __shared__ unsigned s_sup[kTiers]; // roots of pairs that take no items, by domain size
+    if (threadIdx.x < kTiers)
+        s_sup[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < kTiers * kSlots; i += blockDim.x)
         s_hist[i] = 0;
     for (int i = threadIdx.x; i < kSlots; i += blockDim.x)
@@ -3028,6 +3350,11 @@ __global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__
         }
         tier[t] = tc;
         dom[t] = D;
+        if (pd.sup) {
+            if (tc)
+                atomicAdd(&s_sup[tc - 1], 1u);
+            continue;
+        }
         if (tc == 4) {
             const uint32_t rn = pd.pl.rows_needed, rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
             atomicAdd(large_words, (unsigned long long)large_root_words(D, rlo, pd.pl.nbhd != kNbNone));
@@ -3053,6 +3380,8 @@ __global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__
     for (int i = threadIdx.x; i < kSlots; i += blockDim.x)
         if (s_tiny[i])
             atomicAdd(&tiny_depth[i], s_tiny[i]);
+    if (threadIdx.x < kTiers && s_sup[threadIdx.x])
+        atomicAdd(&sup_tiers[threadIdx.x], s_sup[threadIdx.x]);
 }
 
 // Sort keys of every flattened vertex for all item lists at once:
@@ -3064,10 +3393,14 @@ __global__ void k_list_keys(const uint8_t *__restrict__ tier, const uint32_t *__
                             uint64_t N, uint32_t *keys, uint32_t *vals) {
     constexpr uint32_t kDomMask = (1u << 24) - 1u;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t tc = tier[t];
-        uint32_t key = 0xffffffffu;
+        uint32_t tc = tier[t];
+        uint32_t key = 0xffffffffu, p = 0;
         if (tc) {
-            const uint32_t p = find_pair(offs, npairs, t);
+            p = find_pair(offs, npairs, t);
+            if (pairs[p].sup)
+                tc = 0; // takes no items
+        }
+        if (tc) {
             const uint32_t slot = depth_slot(pairs[p].pl, tc, pairs[p].en.out != nullptr);
             const uint32_t d = min(dom[t], kDomMask);
             const uint32_t dk = tc == 1 ? d : (tc == 5 ? 0u : kDomMask - d);
@@ -3151,7 +3484,8 @@ __global__ void k_alg_bytes(const PairDev *__restrict__ pairs, const uint64_t *_
             const uint32_t w = gcol[k];
             b += 4ull * (grp[w + 1] - grp[w]);
         }
-        const int slot = tc == 1 ? 0 : (tc == 4 ? 2 : 1);
+        // (pairs without items count with the small tier, as their time does)
+        const int slot = tc == 1 || pairs[p].sup ? 0 : (tc == 4 ? 2 : 1);
         acc[slot] += a;
         alg[slot] += b;
     }
@@ -3271,7 +3605,10 @@ template <bool ENUM> beep_status large_dfs_blocks_per_sm(int dend, int *out) {
 // ---------------------------------------------------------------------------
 struct LaunchRec {
     enum Kind { kSmall, kMedium, kLargeRows, kLargeLists, kLargeDfs, kLargeWheel, kGeneral, kMemset, kLargeNbDeg,
-                kLargeNbhd } kind;
+                kLargeNbhd, kSupTri, kSupEdge, kSupVertex } kind;
+    const SupView *sup = nullptr; // degree and triangle-count forms: views and 32-entry chunks
+    uint32_t nsup = 0;
+    uint64_t nchunks = 0;
     const uint32_t *tstart = nullptr; // list walker: task prefix of the items
     int dend = 0, grid = 0, block = 0;
     int group = 32; // small tier: lanes per root
@@ -3318,6 +3655,8 @@ struct LaunchPlan {
     std::vector<std::shared_ptr<View>> views; // kept alive while the plan exists
     std::vector<void *> allocs;
     std::vector<uint32_t> live; // spec index of each device pair
+    std::vector<uint32_t> from; // the pair whose counter holds each pair's count (itself, or an equal one)
+    unsigned *d_sup_tiers = nullptr; // roots by tier of the pairs that take no items (null: none)
     uint32_t np = 0;
     PairDev *d_pairs = nullptr;
     uint64_t *d_offs = nullptr;
@@ -3346,8 +3685,9 @@ struct LaunchPlan {
     unsigned long long *d_exit = nullptr;
     uint32_t nexit = 0;
     // host words after the pair counts and byte counters: donation control
-    // blocks (as u32), then exit times
-    size_t tel_words() const { return (size_t)ndon * kDonWords / 2 + 2 * (size_t)nexit; }
+    // blocks (as u32), then exit times, then the item-less pairs' roots by tier
+    static constexpr size_t kSupWords = 4;
+    size_t tel_words() const { return (size_t)ndon * kDonWords / 2 + 2 * (size_t)nexit + kSupWords; }
     size_t host_words() const { return kPairWords * (size_t)np + kAux + tel_words(); }
     beep_stats st{};
     cudaGraphExec_t exec = nullptr;
@@ -3379,7 +3719,7 @@ void LaunchPlanDeleter::operator()(LaunchPlan *p) const { delete p; }
 // neighbourhood statistics' sums; BEEP_COUNT_OVERFLOW when a flag is set or
 // the total reaches the limit.
 static uint64_t pair_result(const LaunchPlan *lp, uint32_t i) {
-    const unsigned long long *c = lp->h_counts + kPairWords * (size_t)i;
+    const unsigned long long *c = lp->h_counts + kPairWords * (size_t)lp->from[i];
     if (c[1] || c[3] || c[5] || c[2] < c[4])
         return BEEP_COUNT_OVERFLOW;
     const uint64_t st = c[2] - c[4], v = c[0] + st;
@@ -3402,6 +3742,26 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     std::vector<PairDev> hp;
     std::vector<uint64_t> offs{0};
     std::vector<Graph *> dropped;
+    // Pairs counted from degrees and triangle counts: whole counts only (the
+    // sums are not per root). Their view is an ascending one whose peel
+    // removes no more than theirs would: peeled vertices are in no match, and
+    // the unpeeled view keeps the degrees that the forms of threshold 1 read.
+    auto sup_form = [&](const PairSpec &ps) -> int32_t {
+        const bool whole = ps.nshards <= 1 && !ps.en && !(options & (BEEP_OPT_REFERENCE_ROOT_CAP | BEEP_OPT_NO_NBHD));
+        return whole ? ps.plan.dev.support : (int32_t)kSupNone;
+    };
+    std::map<Graph *, int32_t> sup_qdeg; // per graph, the least peel threshold of those pairs
+    for (auto &ps : specs)
+        if (ps.g->n != 0 && ps.plan.dev.dend >= 3 && sup_form(ps)) {
+            auto r = sup_qdeg.emplace(ps.g, ps.plan.info.min_qdeg);
+            r.first->second = std::min(r.first->second, ps.plan.info.min_qdeg);
+        }
+    struct SupKey {
+        View *v;
+        std::vector<int32_t> pair; // first pair of every form, or -1
+    };
+    std::vector<SupKey> sups;
+    std::vector<uint64_t> sup_m; // entries of each of their views, at most
     for (size_t i = 0; i < specs.size(); ++i) {
         const PairSpec &ps = specs[i];
         if (ps.g->n == 0 || ps.plan.dev.dend < 3)
@@ -3412,7 +3772,21 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         }
         std::shared_ptr<View> v;
         bool built = false;
-        BEEP_TRY(get_view(ctx, ps.g, ps.plan.info.min_qdeg, ps.plan.dev.asc, false, &v, &built));
+        const int32_t form = sup_form(ps);
+        int32_t qdeg = ps.plan.info.min_qdeg, asc = ps.plan.dev.asc;
+        if (form) {
+            qdeg = sup_qdeg[ps.g];
+            asc = 1;
+        } else if (asc && !ps.g->views.count({(int)qdeg, 1})) {
+            // the call's other view of the graph will do when this pair's own
+            // would have to be built for it: the vertices that the stronger
+            // peel drops are in no match, and whole matches (not prefixes)
+            // are counted once in any order
+            auto it = sup_qdeg.find(ps.g);
+            if (it != sup_qdeg.end() && it->second <= qdeg && ps.plan.dev.dend == ps.plan.dev.K)
+                qdeg = it->second;
+        }
+        BEEP_TRY(get_view(ctx, ps.g, qdeg, asc, false, &v, &built));
         lp->views.push_back(v);
         st.peel_rounds = v->peel_rounds; // view-build launches are counted where they happen
         if (v->n == 0)
@@ -3435,6 +3809,22 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             pd.en.out = ps.en->d_out;
             pd.en.k = ps.en->k;
         }
+        uint32_t from = (uint32_t)hp.size();
+        if (form) {
+            pd.sup = (uint32_t)form;
+            pd.pl.asc = 1;
+            size_t k = 0;
+            while (k < sups.size() && sups[k].v != v.get())
+                ++k;
+            if (k == sups.size())
+                sups.push_back(SupKey{v.get(), std::vector<int32_t>(kSupForms, -1)});
+            if (sups[k].pair[form] < 0)
+                sups[k].pair[form] = (int32_t)hp.size();
+            from = (uint32_t)sups[k].pair[form];
+            sup_m.resize(sups.size());
+            sup_m[k] = (uint64_t)ps.g->m;
+        }
+        lp->from.push_back(from);
         hp.push_back(pd);
         lp->live.push_back((uint32_t)i);
         offs.push_back(offs.back() + (uint64_t)v->n);
@@ -3465,12 +3855,17 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     BEEP_TRY(lp->alloc(lp->d_pairs, np));
     BEEP_TRY(lp->alloc(lp->d_offs, np + 1));
     BEEP_TRY(lp->alloc(lp->d_tier, N));
-    uint32_t *d_dom, *d_sel, *d_keys, *d_keys2;
+    bool items = false; // some pair's roots go through the tiers
+    for (auto &pd : hp)
+        items = items || !pd.sup;
+    uint32_t *d_dom, *d_sel = nullptr, *d_keys = nullptr, *d_keys2 = nullptr;
     unsigned *d_misc;
     BEEP_TRY(lp->alloc(d_dom, N));
-    BEEP_TRY(lp->alloc(d_sel, N));
-    BEEP_TRY(lp->alloc(d_keys, N));
-    BEEP_TRY(lp->alloc(d_keys2, N));
+    if (items) {
+        BEEP_TRY(lp->alloc(d_sel, N));
+        BEEP_TRY(lp->alloc(d_keys, N));
+        BEEP_TRY(lp->alloc(d_keys2, N));
+    }
     BEEP_TRY(lp->alloc(d_misc, 256));
     BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_pairs, hp.data(), np * sizeof(PairDev), cudaMemcpyHostToDevice, s));
     BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_offs, offs.data(), (np + 1) * 8, cudaMemcpyHostToDevice, s));
@@ -3479,7 +3874,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     // d_misc: [0, 8) largest domain per tier, [8, 8 + kTiers * kSlots) roots
     // per (tier, depth slot), [120, 120 + kSlots) tiny small-tier roots per
     // slot, [144, 146) arena words of the large tier (u64)
-    constexpr int kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144;
+    // and [148, 148 + kTiers) roots per tier of the pairs that take no items
+    constexpr int kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144, kMiscSup = 148;
     static_assert(kMiscSlots + kTiers * kSlots <= kMiscTiny && kMiscTiny + kSlots <= kMiscLarge, "d_misc layout");
     TierCfg cfg = tiers;
     cfg.tiny_max = std::min<uint32_t>(cfg.tiny_max, kTinyMaxD);
@@ -3488,12 +3884,16 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     cfg.med_max = std::min<uint32_t>(cfg.med_max, kMediumMaxD);
     k_classify<<<gv, 256, 0, s>>>(lp->d_pairs, lp->d_offs, np, N, cfg, lp->d_tier, d_dom, d_misc,
                                   d_misc + kMiscSlots, d_misc + kMiscTiny,
-                                  reinterpret_cast<unsigned long long *>(d_misc + kMiscLarge));
+                                  reinterpret_cast<unsigned long long *>(d_misc + kMiscLarge), d_misc + kMiscSup);
     BEEP_CUDA_TRY(cudaGetLastError());
     st.kernel_launches += 1;
-    unsigned h_misc[kMiscLarge + 2];
-    BEEP_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
-    BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+    unsigned h_misc[kMiscLarge + 2] = {0};
+    if (items) { // the tiers' sizes decide the launches
+        BEEP_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
+        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    if (!sups.empty())
+        lp->d_sup_tiers = d_misc + kMiscSup; // read back with the counts
     const unsigned *tier_max = h_misc;
     const unsigned *tier_depth = h_misc + kMiscSlots; // [tier * kSlots + slot]
     const unsigned *tiny_depth = h_misc + kMiscTiny;  // [slot]
@@ -3943,6 +4343,75 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             first += cnt;
         }
     }
+    // degree and triangle-count forms: one pass over the oriented edges of
+    // every view they use, then (where asked for) over its edges' and
+    // vertices' triangle counts
+    if (!sups.empty()) {
+        std::vector<SupView> hs(sups.size());
+        uint64_t eoff = 0, voff = 0;
+        bool tri = false, edge = false, vertex = false;
+        for (size_t k = 0; k < sups.size(); ++k) {
+            SupView &sv = hs[k];
+            std::memset(&sv, 0, sizeof(sv));
+            const View *v = sups[k].v;
+            sv.v = ViewDev{v->row_ptr.as<uint32_t>(), v->col.as<uint32_t>(), v->split.as<uint32_t>(),
+                           v->orig.as<uint32_t>()};
+            sv.n = (uint32_t)v->n;
+            sv.eoff = eoff;
+            sv.voff = voff;
+            eoff += (sup_m[k] + 31) & ~31ull;
+            voff += (uint64_t)v->n;
+            for (int f = 1; f < kSupForms; ++f)
+                if (sups[k].pair[f] >= 0)
+                    sv.out[f] = hp[sups[k].pair[f]].count;
+            const bool c = sv.out[kSupDiamond] || sv.out[kSupBook3] || sv.out[kSupWedgeIso] || sv.out[kSupTwoEdges];
+            tri = tri || c || sv.out[kSupTriangle] || sv.out[kSupEdgeIso] || sv.out[kSupEdgeIso2];
+            edge = edge || c;
+            vertex = vertex || sv.out[kSupTwoEdges] || sv.out[kSupStar2] || sv.out[kSupStar3] || sv.out[kSupStar4];
+            auto zeroed = [&](void *ptr, size_t bytes) {
+                LaunchRec ms;
+                ms.kind = LaunchRec::kMemset;
+                ms.mptr = ptr;
+                ms.mbytes = bytes;
+                lp->recs.push_back(ms);
+            };
+            if (c) {
+                BEEP_TRY(lp->alloc(sv.cnt, sup_m[k]));
+                zeroed(sv.cnt, std::max<uint64_t>(sup_m[k], 1) * 4);
+            }
+            if (sv.out[kSupTwoEdges]) {
+                BEEP_TRY(lp->alloc(sv.tv, (size_t)v->n));
+                zeroed(sv.tv, (size_t)v->n * 8);
+            }
+        }
+        SupView *d_sups = nullptr;
+        BEEP_TRY(lp->alloc(d_sups, hs.size()));
+        BEEP_CUDA_TRY(cudaMemcpyAsync(d_sups, hs.data(), hs.size() * sizeof(SupView), cudaMemcpyHostToDevice, s));
+        LaunchRec r;
+        r.sup = d_sups;
+        r.nsup = (uint32_t)hs.size();
+        r.nchunks = eoff / 32;
+        r.block = kSupWarps * 32;
+        r.sink = &st.small_ms;
+        const int64_t chunk_blocks = std::max<int64_t>(1, (int64_t)((r.nchunks + kSupWarps - 1) / kSupWarps));
+        if (tri) {
+            r.kind = LaunchRec::kSupTri;
+            r.grid = (int)std::min<int64_t>(chunk_blocks, (int64_t)ctx->num_sms * 8);
+            r.tail_slot = 0;
+            lp->recs.push_back(r);
+            r.tail_slot = -1;
+        }
+        if (edge) {
+            r.kind = LaunchRec::kSupEdge;
+            r.grid = (int)std::min<int64_t>(chunk_blocks, (int64_t)ctx->num_sms * 8);
+            lp->recs.push_back(r);
+        }
+        if (vertex) {
+            r.kind = LaunchRec::kSupVertex;
+            r.grid = (int)std::min<uint64_t>((voff + 255) / 256, (uint64_t)ctx->num_sms * 4);
+            lp->recs.push_back(r);
+        }
+    }
     // shared-memory opt-ins are host calls: done here, never inside a capture
     for (auto &r : lp->recs)
         if (r.kind == LaunchRec::kMedium) {
@@ -4051,6 +4520,21 @@ beep_status issue(Ctx *ctx, LaunchPlan *lp, bool timing, bool serial, bool stall
             BEEP_CUDA_TRY(cudaGetLastError());
             st.large_dfs_launches++;
             break;
+        case LaunchRec::kSupTri:
+            k_sup_triangles<<<r.grid, r.block, 0, rs>>>(r.sup, r.nsup, r.nchunks, ex);
+            BEEP_CUDA_TRY(cudaGetLastError());
+            st.small_launches++;
+            break;
+        case LaunchRec::kSupEdge:
+            k_sup_edges<<<r.grid, r.block, 0, rs>>>(r.sup, r.nsup, r.nchunks);
+            BEEP_CUDA_TRY(cudaGetLastError());
+            st.small_launches++;
+            break;
+        case LaunchRec::kSupVertex:
+            k_sup_vertices<<<r.grid, r.block, 0, rs>>>(r.sup, r.nsup);
+            BEEP_CUDA_TRY(cudaGetLastError());
+            st.small_launches++;
+            break;
         case LaunchRec::kMedium:
 #define BEEP_CASE(D)                                                                                               \
     case D:                                                                                                        \
@@ -4115,6 +4599,9 @@ static cudaError_t readback(LaunchPlan *lp, cudaStream_t s, bool timing) {
     if (e == cudaSuccess && timing && lp->nexit)
         e = cudaMemcpyAsync(tel + (size_t)lp->ndon * kDonWords / 2, lp->d_exit, 2 * (size_t)lp->nexit * 8,
                             cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && lp->d_sup_tiers)
+        e = cudaMemcpyAsync(tel + (size_t)lp->ndon * kDonWords / 2 + 2 * (size_t)lp->nexit, lp->d_sup_tiers,
+                            kTiers * 4, cudaMemcpyDeviceToHost, s);
     return e;
 }
 
@@ -4231,6 +4718,15 @@ beep_status execute_plan(Ctx *ctx, LaunchPlan *lp, uint32_t options, const std::
         st.general_ms = lp->st.general_ms;
         lp->st.small_ms = lp->st.medium_ms = lp->st.large_encode_ms = lp->st.large_dfs_ms = 0;
         lp->st.general_ms = 0;
+    }
+    if (lp->d_sup_tiers) {
+        const unsigned *n = reinterpret_cast<const unsigned *>(lp->h_counts + kPairWords * (size_t)lp->np + kAux +
+                                                               (size_t)lp->ndon * kDonWords / 2 +
+                                                               2 * (size_t)lp->nexit);
+        st.roots_small += n[0];
+        st.roots_medium += (int64_t)n[1] + n[2];
+        st.roots_large += n[3];
+        st.roots += (int64_t)n[0] + n[1] + n[2] + n[3];
     }
     for (size_t i = 0; i < ncounts; ++i)
         counts[i] = 0;

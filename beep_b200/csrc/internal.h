@@ -75,6 +75,7 @@ struct DevPlan {
     uint32_t sym0;           // bit p: position p must follow position 0
     int32_t wheel4;          // the 4-wheel's plan: counted per (x1, x3) pair in closed form
     int32_t nbhd;            // NbhdForm: in the large tier, counted from neighbourhood statistics
+    int32_t support;         // SupForm: counted from degrees and triangle counts
     int32_t clique;          // a complete query, every position ordered after the ones before it
 };
 
@@ -91,6 +92,25 @@ enum NbhdForm : int32_t {
     kNbPath4 = 4,    // H = path on 4 vertices:     sum over edges (d_u - 1)(d_w - 1) - 3T
     kNbPaw = 5,      // H = paw (universal vertex u after v): sum_u t_u (d_u - 2), t_u triangles at u
     kNbDiamond = 6   // H = diamond (both universal vertices after v): sum over edges C(c(u, w), 2)
+};
+
+// Queries whose count is a sum over the graph's vertices and edges of terms in
+// their degrees d and triangle counts (c_e at an edge, t_v at a vertex). They
+// are counted over the oriented edges of one view, without neighbourhood
+// bitmaps or root tiers (counts of all roots only: no shard, no root cap).
+enum SupForm : int32_t {
+    kSupNone = 0,
+    kSupTriangle = 1, // the triangle: one per triangle
+    kSupEdgeIso = 2,  // cone over an edge + 1 isolated vertex: sum_v t_v (d_v - 2)
+    kSupEdgeIso2 = 3, // cone over an edge + 2 isolated:        sum_v t_v C(d_v - 2, 2)
+    kSupDiamond = 4,  // two triangles on an edge:              sum_e C(c_e, 2)
+    kSupBook3 = 5,    // three triangles on an edge:            sum_e C(c_e, 3)
+    kSupWedgeIso = 6, // cone over a wedge + 1 isolated:        sum_e C(c_e, 2) (d_u + d_v - 6)
+    kSupTwoEdges = 7, // cone over two disjoint edges:          sum_v C(t_v, 2) - 2 sum_e C(c_e, 2)
+    kSupStar2 = 8,    // stars: sum_v C(d_v, leaves)
+    kSupStar3 = 9,
+    kSupStar4 = 10,
+    kSupForms = 11
 };
 
 struct QueryPlan {

@@ -354,6 +354,29 @@ beep_status compile_plan(int32_t qn, const std::vector<int32_t> &rp, const std::
         else if (edges == 5 && seq(2, 2, 3, 3) && hubs == 2 && universal_after)
             D.nbhd = kNbDiamond;
     }
+    // Degree and triangle-count forms: central queries at full depth whose
+    // positions 1.. carry at most one edge, a wedge, two disjoint edges, a
+    // three-leaf star or (four vertices in all) a path.
+    D.support = kSupNone;
+    if (P.central && D.dend == qn && qn >= 3 && qn <= 5) {
+        int deg[5] = {0, 0, 0, 0, 0}, edges = 0;
+        for (int p = 2; p < qn; ++p)
+            for (int q = 1; q < p; ++q)
+                if (D.back[p] >> q & 1u) {
+                    ++edges;
+                    ++deg[p];
+                    ++deg[q];
+                }
+        const int maxd = *std::max_element(deg, deg + 5);
+        if (edges == 0)
+            D.support = qn == 3 ? kSupStar2 : (qn == 4 ? kSupStar3 : kSupStar4);
+        else if (edges == 1)
+            D.support = qn == 3 ? kSupTriangle : (qn == 4 ? kSupEdgeIso : kSupEdgeIso2);
+        else if (edges == 2)
+            D.support = qn == 4 ? kSupDiamond : (maxd == 2 ? kSupWedgeIso : kSupTwoEdges);
+        else if (edges == 3 && qn == 5 && maxd == 3)
+            D.support = kSupBook3;
+    }
     // A clique: every position adjacent to and ordered after all before it,
     // so a walk reads only the part of a row above its vertex.
     D.clique = D.restricted && D.asc && D.dend == qn && qn >= 4;
