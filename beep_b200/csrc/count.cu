@@ -1288,19 +1288,62 @@ __device__ __forceinline__ uint32_t c4_indices(uint32_t w, uint32_t k, uint16_t 
     return total;
 }
 
+// What the counters of one vertex a are summed into. b runs over row(a), c over
+// the columns; n_c counts the b whose row holds c.
+enum C4Mode : int {
+    kC4Cycles = 0,    // b < a, every c < a: C(n_c, 2), the 4-cycles with largest vertex a
+    kC4Triangles = 1, // b < a, c of row(a) above a: n_c, the triangles whose middle vertex is a
+    kC4Paw = 2,       // b < c, both of row(a): n_c, the triangles at a
+    kC4Diamond = 3    // every b of row(a), c of row(a) above a: C(n_c, 2) over the edges (a, c)
+};
+
+// Masks of one word of row(a) (index k, contents w): the b's in it, the c's.
+template <int MODE>
+__device__ __forceinline__ uint32_t c4_b_bits(uint32_t w, uint32_t k, uint32_t a) {
+    if (MODE == kC4Paw || MODE == kC4Diamond)
+        return w;
+    return k < (a >> 5) ? w : (k == (a >> 5) ? w & ((1u << (a & 31)) - 1u) : 0u);
+}
+template <int MODE>
+__device__ __forceinline__ uint32_t c4_c_bits(uint32_t w, uint32_t k, uint32_t a) {
+    if (MODE == kC4Paw)
+        return w;
+    const uint32_t aw = a >> 5;
+    if (MODE == kC4Cycles)
+        return k < aw ? 0xffffffffu : (k == aw ? (1u << (a & 31)) - 1u : 0u);
+    return k > aw ? w : (k == aw ? w & ~((2u << (a & 31)) - 1u) : 0u);
+}
+// Word k of row b as a counter input: the paw counts only c > b.
+template <int MODE> __device__ __forceinline__ uint32_t c4_input(uint32_t w, uint32_t k, uint32_t b) {
+    if (MODE != kC4Paw)
+        return w;
+    const uint32_t bw = b >> 5;
+    return k > bw ? w : (k == bw ? w & ~((2u << (b & 31)) - 1u) : 0u);
+}
+// The mode's sum over the counters of slices [0, L) in the columns of mask.
+template <int MODE, int NS>
+__device__ __forceinline__ unsigned long long c4_sum(uint32_t (&s)[NS], int L, uint32_t mask) {
+    if constexpr (MODE == kC4Cycles || MODE == kC4Diamond) {
+        return c4_pairs<NS>(s, L, mask);
+    } else {
+        unsigned long long tot = 0;
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            tot += (unsigned long long)__popc(s[k] & mask) << k;
+        return tot;
+    }
+}
+
 // Rows in shared memory, W <= G words each (stride RS): a group of G lanes
-// counts the 4-cycles whose largest vertex is a; this lane's part is returned.
-// ib: D 16-bit entries of the group's own.
-template <int G, int NS>
-__device__ __forceinline__ unsigned long long wheel4_group(const uint32_t *rows, uint32_t RS, uint32_t a,
-                                                           uint16_t *ib, int glane, unsigned gmask) {
-    const uint32_t k = (uint32_t)glane, aw = a >> 5;
-    const uint32_t below = (1u << (a & 31)) - 1u; // bits of word aw below a
-    const uint32_t cm = k < aw ? 0xffffffffu : (k == aw ? below : 0u);
-    const uint32_t ra = k <= aw ? rows[(size_t)a * RS + k] & cm : 0u;
-    const uint32_t nb = c4_indices<G>(ra, k, ib, glane, gmask);
-    if (nb < 2)
-        return 0;
+// takes vertex a; this lane's part of the sum is returned. ib: D 16-bit
+// entries of the group's own.
+template <int MODE, int G, int NS>
+__device__ __forceinline__ unsigned long long c4_group(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t a,
+                                                       uint16_t *ib, int glane, unsigned gmask) {
+    const uint32_t k = (uint32_t)glane;
+    const uint32_t ra = k < W ? rows[(size_t)a * RS + k] : 0u;
+    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra, k, a) : 0u;
+    const uint32_t nb = c4_indices<G>(c4_b_bits<MODE>(ra, k, a), k, ib, glane, gmask);
     uint32_t s[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i)
@@ -1308,12 +1351,17 @@ __device__ __forceinline__ unsigned long long wheel4_group(const uint32_t *rows,
     for (uint32_t i = 0; i < nb; i += 8) {
         uint32_t d[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-            d[q] = (k <= aw && i + q < nb) ? rows[(size_t)ib[i + q] * RS + k] : 0u;
+        for (int q = 0; q < 8; ++q) {
+            d[q] = 0;
+            if (cm && i + q < nb) {
+                const uint32_t b = ib[i + q];
+                d[q] = c4_input<MODE>(rows[(size_t)b * RS + k], k, b);
+            }
+        }
         c4_add8<NS>(s, d);
     }
     __syncwarp(gmask); // ib is rewritten by the group's next call
-    return c4_pairs<NS>(s, 32 - __clz((int)nb), cm);
+    return nb ? c4_sum<MODE, NS>(s, 32 - __clz((int)nb), cm) : 0ull;
 }
 
 template <int DEND, bool ENUM, int G, int MAXD>
@@ -1440,28 +1488,6 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
 // plus / minus. The walk would instead enumerate every (x1, x2, x3) prefix.
 // Block-wide (block-uniform call); s_deg: D words, s_misc: 2 words.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void nbhd_term(int form, unsigned long long du, unsigned long long dw, uint32_t c_all,
-                                          uint32_t c_above, unsigned long long rest, unsigned long long &plus,
-                                          unsigned long long &minus, unsigned long long &tri) {
-    switch (form) {
-    case kNbTriIso: // triangles (u < w < x) once, times the isolated vertex's choices
-        plus = sat_add(plus, sat_mul(c_above, rest));
-        break;
-    case kNbPath4: // paths x - u - w - y, minus the closed ones (x = y): 3T
-        plus = sat_add(plus, (du - 1) * (dw - 1));
-        minus = sat_add(minus, c_all);
-        break;
-    case kNbPaw: // triangles (u, w, x) with x after w: each once
-        tri += c_above;
-        break;
-    case kNbDiamond: // C(common neighbours, 2) of the edge (u, w)
-        plus = sat_add(plus, binom2(c_all));
-        break;
-    default:
-        break;
-    }
-}
-
 // Degrees of rows[0, D) into s_deg and their sum into s_misc[0]; a warp per
 // row (rw words of 32 bits, at most 32), or a thread per row (rw > 32 words
 // never occur here: the thread sub-tier's rows are 8 words).
@@ -1483,129 +1509,65 @@ __device__ __forceinline__ void nbhd_degrees(const uint32_t *rows, uint32_t rw, 
         atomicAdd(&s_misc[0], part);
 }
 
-// Thread sub-tier: rows of NW 64-bit words, a thread per task u.
-template <int NW>
-__device__ __forceinline__ void nbhd_medium_thread(int form, const uint64_t *r64, uint32_t D, uint32_t j0,
-                                                   uint32_t *s_deg, uint32_t *s_misc, unsigned long long &plus,
-                                                   unsigned long long &minus) {
+// Groups of G lanes (rows of W <= G words, RS apart) take the vertices u; the
+// edges' common neighbours come from the bit-sliced counters of the 4-wheel
+// (c4_group), 32 edges a lane at once. ib: the group's D 16-bit entries.
+// (12 power-law graphs x 15 patterns, replayed: 21.5 -> 15.7 ms with the large
+// tier's strips; a warp per u walking word lists had tails of 15 ms.)
+template <int G, int NS>
+__device__ __forceinline__ void nbhd_medium(int form, const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
+                                            uint32_t j0, uint32_t *s_deg, uint32_t *s_misc, uint16_t *ib_all,
+                                            unsigned long long &plus, unsigned long long &minus) {
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    uint16_t *ib = ib_all + (threadIdx.x / G) * (size_t)((D + 1) & ~1u);
     if (threadIdx.x == 0) {
         s_misc[0] = 0;
         s_misc[1] = j0;
     }
     __syncthreads();
-    nbhd_degrees(reinterpret_cast<const uint32_t *>(r64), 2 * NW, D, s_deg, s_misc);
-    __syncthreads();
-    const unsigned long long E = s_misc[0] / 2, rest = D >= 3 ? D - 3 : 0;
-    if (form == kNbTwoEdges && threadIdx.x == 0)
-        plus = sat_add(plus, binom2(E)); // C(E, 2): E < 2^15 here
-    for (;;) {
-        const uint32_t u = atomicAdd(&s_misc[1], 1u);
-        if (u >= D)
-            break;
-        const unsigned long long du = s_deg[u];
-        if (form == kNbWedgeIso) {
-            plus = sat_add(plus, binom2(du) * rest);
-            continue;
-        }
-        if (form == kNbTwoEdges) {
-            minus = sat_add(minus, binom2(du));
-            continue;
-        }
-        uint64_t ru[NW];
-#pragma unroll
-        for (int i = 0; i < NW; ++i)
-            ru[i] = r64[(size_t)u * NW + i];
-        const bool all_w = form == kNbPaw; // else the edges (u, w) with w after u
-        const uint32_t ui = u >> 6;
-        unsigned long long tri = 0;
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-            uint64_t bits = ru[i];
-            if (!all_w)
-                bits = (uint32_t)i < ui ? 0ull : ((uint32_t)i == ui ? (bits & ~((2ull << (u & 63)) - 1ull)) : bits);
-            while (bits) {
-                const uint32_t w = (uint32_t)i * 64 + (uint32_t)(__ffsll((long long)bits) - 1);
-                bits &= bits - 1;
-                const uint64_t *rw = r64 + (size_t)w * NW;
-                const uint32_t wi = w >> 6;
-                const uint64_t wm = ~((2ull << (w & 63)) - 1ull); // bits of word wi above w
-                uint32_t c_all = 0, c_above = 0;
-#pragma unroll
-                for (int k = 0; k < NW; ++k) {
-                    const uint64_t x = ru[k] & rw[k];
-                    c_all += (uint32_t)__popcll(x);
-                    c_above += (uint32_t)__popcll((uint32_t)k < wi ? 0ull : ((uint32_t)k == wi ? (x & wm) : x));
-                }
-                nbhd_term(form, du, s_deg[w], c_all, c_above, rest, plus, minus, tri);
-            }
-        }
-        if (form == kNbPaw && du >= 2)
-            plus = sat_add(plus, sat_mul(tri, du - 2));
-    }
-}
-
-// Warp sub-tier: rows of W <= 32 words, a warp per task u (lane k holds word
-// k of row u; each edge's common neighbours are one warp sum).
-__device__ __forceinline__ void nbhd_medium_warp(int form, const uint32_t *rows, uint32_t W, uint32_t D,
-                                                 uint32_t j0, uint32_t *s_deg, uint32_t *s_misc,
-                                                 unsigned long long &plus, unsigned long long &minus) {
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        s_misc[0] = 0;
-        s_misc[1] = j0;
-    }
-    __syncthreads();
-    nbhd_degrees(rows, W, D, s_deg, s_misc);
+    nbhd_degrees(rows, RS, D, s_deg, s_misc);
     __syncthreads();
     const unsigned long long E = s_misc[0] / 2, rest = D >= 3 ? D - 3 : 0;
     if (form == kNbTwoEdges && threadIdx.x == 0)
         plus = sat_add(plus, binom2(E)); // C(E, 2): E < 2^19 here
     for (;;) {
         uint32_t u = 0;
-        if (lane == 0)
+        if (gl == 0)
             u = atomicAdd(&s_misc[1], 1u);
-        u = __shfl_sync(kFull, u, 0);
+        u = __shfl_sync(gm, u, 0, G);
         if (u >= D)
             break;
         const unsigned long long du = s_deg[u];
-        if (form == kNbWedgeIso || form == kNbTwoEdges) {
-            if (lane == 0) {
-                if (form == kNbWedgeIso)
-                    plus = sat_add(plus, binom2(du) * rest);
-                else
-                    minus = sat_add(minus, binom2(du));
-            }
-            continue;
+        switch (form) {
+        case kNbWedgeIso:
+            if (gl == 0)
+                plus = sat_add(plus, binom2(du) * rest);
+            break;
+        case kNbTwoEdges:
+            if (gl == 0)
+                minus = sat_add(minus, binom2(du));
+            break;
+        case kNbTriIso: // triangles once, times the isolated vertex's choices
+            plus = sat_add(plus, sat_mul(c4_group<kC4Triangles, G, NS>(rows, RS, W, u, ib, gl, gm), rest));
+            break;
+        case kNbPath4: { // paths x - u - w - y over the edges (u, w > u), minus the closed ones (x = y): 3T
+            const uint32_t k = (uint32_t)gl;
+            for (uint32_t b = k < W ? c4_c_bits<kC4Triangles>(rows[(size_t)u * RS + k], k, u) : 0u; b; b &= b - 1)
+                plus = sat_add(plus, (du - 1) * (unsigned long long)(s_deg[(k << 5) + (uint32_t)(__ffs(b) - 1)] - 1));
+            minus = sat_add(minus, 3 * c4_group<kC4Triangles, G, NS>(rows, RS, W, u, ib, gl, gm));
+            break;
         }
-        const uint32_t ru = (uint32_t)lane < W ? rows[(size_t)u * W + lane] : 0u;
-        const uint32_t uw = u >> 5;
-        uint32_t bits = ru;
-        if (form != kNbPaw)
-            bits = (uint32_t)lane < uw ? 0u : ((uint32_t)lane == uw ? (bits & ~((2u << (u & 31)) - 1u)) : bits);
-        unsigned long long tri = 0;
-        unsigned bal = __ballot_sync(kFull, bits != 0);
-        while (bal) {
-            const int L = __ffs(bal) - 1;
-            const uint32_t wb = __shfl_sync(kFull, bits, L);
-            const uint32_t w = (uint32_t)L * 32 + (uint32_t)(__ffs(wb) - 1);
-            if (lane == L)
-                bits &= bits - 1;
-            bal = __ballot_sync(kFull, bits != 0);
-            const uint32_t x = (uint32_t)lane < W ? (ru & rows[(size_t)w * W + lane]) : 0u;
-            const uint32_t wi = w >> 5;
-            uint32_t c_all = (uint32_t)__popc(x);
-            uint32_t c_above = (uint32_t)__popc((uint32_t)lane < wi ? 0u
-                                                                     : ((uint32_t)lane == wi ? (x & ~((2u << (w & 31)) - 1u)) : x));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                c_all += __shfl_xor_sync(kFull, c_all, o);
-                c_above += __shfl_xor_sync(kFull, c_above, o);
-            }
-            if (lane == 0)
-                nbhd_term(form, du, s_deg[w], c_all, c_above, rest, plus, minus, tri);
+        case kNbPaw:
+            if (du >= 2)
+                plus = sat_add(plus, sat_mul(c4_group<kC4Paw, G, NS>(rows, RS, W, u, ib, gl, gm), du - 2));
+            break;
+        case kNbDiamond: // C(common neighbours, 2) of the edges (u, w > u)
+            plus = sat_add(plus, c4_group<kC4Diamond, G, NS>(rows, RS, W, u, ib, gl, gm));
+            break;
+        default:
+            break;
         }
-        if (form == kNbPaw && lane == 0 && du >= 2)
-            plus = sat_add(plus, sat_mul(tri, du - 2));
     }
 }
 
@@ -1744,7 +1706,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                                                 uint32_t parts, unsigned *cursor, uint32_t maxD,
                                                 unsigned long long *exit_t) {
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t s_ri, s_j, s_full;
+    __shared__ uint32_t s_ri, s_j, s_full, s_nb[2];
     const int lane = threadIdx.x & 31;
     const uint32_t pad = (maxD + 4) & ~3u;
     const uint32_t nslots = hash_slots(maxD), hshift = 32u - (uint32_t)__ffs((int)nslots) + 1u;
@@ -1853,11 +1815,13 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         bool stats_done = false; // counted by the neighbourhood statistics
         if constexpr (DEND == 5 && !ENUM) {
             if (nbform) { // block-uniform; rows of the whole domain
+                // the domain list's place takes the degrees, the row
+                // builder's arrays the index lists (as for the 4-wheel)
+                uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb);
                 if constexpr (G == 0)
-                    nbhd_medium_thread<kThreadNW>(nbform, reinterpret_cast<const uint64_t *>(rows), D, j0, s_hb,
-                                                  s_len, nb_plus, nb_minus);
+                    nbhd_medium<8, 9>(nbform, rows, 8, 8, D, j0, A, s_nb, ib, nb_plus, nb_minus);
                 else
-                    nbhd_medium_warp(nbform, rows, W, D, j0, s_hb, s_len, nb_plus, nb_minus);
+                    nbhd_medium<32, 11>(nbform, rows, W, W, D, j0, A, s_nb, ib, nb_plus, nb_minus);
                 stats_done = true;
             }
         }
@@ -1886,7 +1850,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     j = __shfl_sync(gm, j, 0, 8);
                     if (j >= D)
                         break;
-                    cnt = sat_add(cnt, wheel4_group<8, 9>(rows, 8, D - 1 - j, ib, gl, gm));
+                    cnt = sat_add(cnt, c4_group<kC4Cycles, 8, 9>(rows, 8, 8, D - 1 - j, ib, gl, gm));
                 }
             } else if (DEND == 3 || pr.lp.free_from <= 2) { // block-uniform
                 // level 2 is the last or is counted in closed form: O(1) per level-1 vertex
@@ -1954,7 +1918,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     if (wheel) { // block-uniform; rows of the whole domain
                         uint16_t *ib =
                             reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 5) * (size_t)((D + 1) & ~1u);
-                        cnt = sat_add(cnt, wheel4_group<32, 11>(rows, W, D - 1 - j, ib, glane, gmask));
+                        cnt = sat_add(cnt, c4_group<kC4Cycles, 32, 11>(rows, W, W, D - 1 - j, ib, glane, gmask));
                         continue;
                     }
                 }
@@ -2031,8 +1995,8 @@ __host__ __device__ __forceinline__ uint64_t large_root_words(uint32_t D, uint32
     return ((nb ? nb_edges_offset(D, rlo) + 2 : nb_deg_offset(D, rlo)) + 31) & ~(uint64_t)31;
 }
 
-// Tasks of a large root's walk: its level-1 vertices, or (4-wheel) the (a, strip) pairs.
-__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, int wheel4);
+// Tasks of a large root's walk: its level-1 vertices, or (vertex, strip) pairs.
+__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, const DevPlan &pl);
 
 __device__ __forceinline__ uint32_t find_batch(const uint32_t *__restrict__ start, uint32_t nb, uint32_t t) {
     // last b with start[b] <= t
@@ -2320,10 +2284,53 @@ __host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D) {
 }
 static_assert((kC4StripMaxW * 32) >> kC4MaxSlices == 0, "a count fits the slices");
 
-__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, int wheel4) {
-    return wheel4 && (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D - j0;
+__host__ __device__ __forceinline__ bool nbhd_strips(int nbhd, uint32_t D) {
+    return nbhd >= kNbTriIso && (D + 31) / 32 <= kC4StripMaxW;
+}
+__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, const DevPlan &pl) {
+    if (nbhd_strips(pl.nbhd, D))
+        return (D - j0) * ((D + 1023) / 1024); // (u, strip) pairs
+    return pl.wheel4 && (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D - j0;
 }
 
+// One strip of vertex a: this lane's part of the mode's sum.
+template <int MODE>
+__device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restrict__ bm, uint32_t W, uint32_t a,
+                                                       uint32_t st, uint16_t *ib, int lane) {
+    const uint32_t k = 32 * st + (uint32_t)lane;
+    const uint32_t *ra = bm + (size_t)a * W, *col = bm + k;
+    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra[k], k, a) : 0u;
+    if (!__ballot_sync(kFull, cm != 0))
+        return 0;
+    uint32_t s[kC4MaxSlices];
+#pragma unroll
+    for (int i = 0; i < kC4MaxSlices; ++i)
+        s[i] = 0;
+    uint32_t total = 0;
+    // the b's: all of row(a), below a, or (paw, c > b) up to the strip's last word
+    const uint32_t wend = MODE == kC4Diamond ? W : (MODE == kC4Paw ? min(W, 32 * st + 32) : (a >> 5) + 1);
+    for (uint32_t w0 = 0; w0 < wend; w0 += 32) {
+        const uint32_t wi = w0 + (uint32_t)lane;
+        const uint32_t nb = c4_indices<32>(wi < wend ? c4_b_bits<MODE>(ra[wi], wi, a) : 0u, wi, ib, lane, kFull);
+        total += nb;
+        for (uint32_t i = 0; i < nb; i += 8) {
+            uint32_t d[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                d[q] = 0;
+                if (cm && i + q < nb) {
+                    const uint32_t b = ib[i + q];
+                    d[q] = c4_input<MODE>(col[(size_t)b * W], k, b);
+                }
+            }
+            c4_add8<kC4MaxSlices>(s, d);
+        }
+        __syncwarp();
+    }
+    return total ? c4_sum<MODE, kC4MaxSlices>(s, 32 - __clz((int)total), cm) : 0ull;
+}
+
+// 4-wheel task t of a root.
 __device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, uint32_t W, uint32_t D, uint32_t t,
                                               uint16_t *ib, int lane, unsigned long long &cnt) {
     uint32_t st = 0;
@@ -2331,33 +2338,7 @@ __device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, u
         t -= D - 1024 * st;
         ++st;
     }
-    const uint32_t a = D - 1 - t, aw = a >> 5, k = 32 * st + (uint32_t)lane;
-    const uint32_t below = (1u << (a & 31)) - 1u;
-    const uint32_t *ra = bm + (size_t)a * W, *col = bm + k;
-    uint32_t s[kC4MaxSlices];
-#pragma unroll
-    for (int i = 0; i < kC4MaxSlices; ++i)
-        s[i] = 0;
-    uint32_t total = 0;
-    for (uint32_t w0 = 0; w0 <= aw; w0 += 32) {
-        const uint32_t wi = w0 + (uint32_t)lane;
-        uint32_t w = wi <= aw ? ra[wi] : 0u;
-        if (wi == aw)
-            w &= below;
-        const uint32_t nb = c4_indices<32>(w, wi, ib, lane, kFull);
-        total += nb;
-        for (uint32_t i = 0; i < nb; i += 8) {
-            uint32_t d[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                d[q] = (k <= aw && i + q < nb) ? col[(size_t)ib[i + q] * W] : 0u;
-            c4_add8<kC4MaxSlices>(s, d);
-        }
-        __syncwarp();
-    }
-    if (total >= 2)
-        cnt = sat_add(cnt, c4_pairs<kC4MaxSlices>(s, 32 - __clz((int)total),
-                                                  k < aw ? 0xffffffffu : (k == aw ? below : 0u)));
+    cnt = sat_add(cnt, c4_strip<kC4Cycles>(bm, W, D - 1 - t, st, ib, lane));
 }
 
 // A donated task of level P resumes the walk at that level over its
@@ -2769,6 +2750,7 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
     // [2 Wm, 3 Wm)
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
+    __shared__ uint16_t s_ib[8][1024];
     PairRegs pr;
     uint32_t cur = 0xffffffffu;
     int form = kNbNone;
@@ -2806,6 +2788,33 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
         rl.nzl = rl.nzc + D;
         const uint32_t *deg = rows + nb_deg_offset(D, 0);
         const unsigned long long E = *reinterpret_cast<const unsigned long long *>(rows + nb_edges_offset(D, 0)) / 2;
+        if (nbhd_strips(form, D)) {
+            // the forms' per-edge terms by bit-sliced counters; forms without
+            // them (wedge, two edges) and wider rows take nbhd_task
+            const uint32_t S = (D + 1023) / 1024, ti = t - bt.tstart[b], st = ti % S, u = j0 + ti / S;
+            uint16_t *ib = s_ib[threadIdx.x >> 5];
+            const unsigned long long du = deg[u], rest = D - 3;
+            switch (form) {
+            case kNbTriIso:
+                plus = sat_add(plus, sat_mul(c4_strip<kC4Triangles>(rows, W, u, st, ib, lane), rest));
+                break;
+            case kNbPath4: {
+                const uint32_t k = 32 * st + (uint32_t)lane;
+                for (uint32_t x = k < W ? c4_c_bits<kC4Triangles>(rows[(size_t)u * W + k], k, u) : 0u; x; x &= x - 1)
+                    plus = sat_add(plus, (du - 1) * (unsigned long long)(deg[(k << 5) + (uint32_t)(__ffs(x) - 1)] - 1));
+                minus = sat_add(minus, 3 * c4_strip<kC4Triangles>(rows, W, u, st, ib, lane));
+                break;
+            }
+            case kNbPaw:
+                if (du >= 2)
+                    plus = sat_add(plus, sat_mul(c4_strip<kC4Paw>(rows, W, u, st, ib, lane), du - 2));
+                break;
+            default: // kNbDiamond
+                plus = sat_add(plus, c4_strip<kC4Diamond>(rows, W, u, st, ib, lane));
+                break;
+            }
+            continue;
+        }
         const uint32_t u = j0 + (t - bt.tstart[b]);
         nbhd_task(form, rows, rl, deg, E, W, D, u, t == bt.tstart[b], ws + 2 * (size_t)Wm, lane, plus, minus);
     }
@@ -3433,7 +3442,7 @@ __global__ void k_large_meta(const PairDev *__restrict__ pairs, const uint64_t *
         const uint32_t rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
         words[i] = large_root_words(D, rlo, pl.nbhd != kNbNone);
         chunks[i] = (D + kRowsPerChunk - 1) / kRowsPerChunk;
-        tasks[i] = large_tasks(D, j0, pl.wheel4);
+        tasks[i] = large_tasks(D, j0, pl);
     }
 }
 
@@ -4114,7 +4123,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             const uint32_t D = lD[i], rlo = pl.rows_needed == 2 ? 0u : (pl.rows_needed == 1 ? lj[i] : D);
             const uint64_t words = large_root_words(D, rlo, pl.nbhd != kNbNone);
             const PairDev &pdv = hp[(uint32_t)(litems[i] >> 32)];
-            rs[i] = R{litems[i], D, large_tasks(D, lj[i], pl.wheel4), depth_slot(pl, 4, pdv.en.out != nullptr), words};
+            rs[i] = R{litems[i], D, large_tasks(D, lj[i], pl), depth_slot(pl, 4, pdv.en.out != nullptr), words};
         }
         std::sort(rs.begin(), rs.end(), [](const R &a, const R &b) { return a.D > b.D; });
         // batch boundaries and the arena size (largest batch)
