@@ -3312,21 +3312,54 @@ __device__ __forceinline__ uint32_t find_pair(const uint64_t *__restrict__ offs,
     return lo;
 }
 
-// tier[t] for flattened vertex t; dom[t] = its domain size; per tier the
-// largest domain and per (tier, depth) the number of roots.
-__global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__restrict__ offs, uint32_t npairs,
-                           uint64_t N, TierCfg cfg, uint8_t *tier, uint32_t *dom, unsigned *tier_max,
-                           unsigned *tier_depth, unsigned *tiny_depth, unsigned long long *large_words,
-                           unsigned *sup_tiers) {
-    __shared__ unsigned s_hist[kTiers * kSlots];
-    __shared__ unsigned s_tiny[kSlots];
+// The item lists are filled by buckets: (tier, depth slot, domain class), the
+// classes of a (tier, slot) in the order its kernel wants -- small roots by
+// rising domain (tiny ones first; the kernel starts at the end), medium and
+// large ones by falling domain (heaviest first), list-walker roots as they
+// come. k_classify counts the buckets, k_list_offsets turns the counts into
+// offsets and the per-tier totals that size the launches, k_list_fill writes
+// the items. Within a bucket the order is that of arrival: no count depends on
+// it. (A radix sort of 32-bit keys over all vertices did this in eight
+// launches; these are three, with no key arrays. 4-cliques of a resident
+// power-law graph of 100,003 vertices: 0.52 -> 0.45 ms a call.)
+constexpr uint32_t kDomClasses = 64;
+constexpr uint32_t kBuckets = kTiers * kSlots * kDomClasses;
+
+__host__ __device__ __forceinline__ uint32_t dom_class(uint32_t tier, uint32_t D) {
+    if (tier == 1)
+        return D < 63 ? D : 63; // at most kSmallMaxD = 64
+    if (tier == 2 || tier == 3)
+        return 63 - (D / 16 < 63 ? D / 16 : 63); // at most kMediumMaxD = 1024
+    if (tier == 4) { // half-octaves
+#ifdef __CUDA_ARCH__
+        const uint32_t lg = 31u - (uint32_t)__clz((int)D);
+#else
+        const uint32_t lg = 31u - (uint32_t)__builtin_clz(D);
+#endif
+        return 63 - (2 * lg + ((D >> (lg - 1)) & 1u));
+    }
+    return 0;
+}
+static_assert(kTinyMaxD < 63 && kSmallMaxD <= 64 && kMediumMaxD <= 1024, "domain classes");
+
+// Words of the planning block: largest domain per tier [0, 8), roots per
+// (tier, slot) [8, 118), tiny small-tier roots per slot [120, 142), arena
+// words of the large tier (u64) [144, 146), roots per tier of the pairs that
+// take no items [148, 153), bucket counts (then offsets) from kMiscBuckets on.
+constexpr uint32_t kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144, kMiscSup = 148, kMiscBuckets = 160;
+static_assert(kMiscSlots + kTiers * kSlots <= kMiscTiny && kMiscTiny + kSlots <= kMiscLarge, "planning block");
+constexpr uint32_t kMiscWords = kMiscBuckets + kBuckets;
+
+// tier[t] for flattened vertex t; dom[t] = its domain size.
+__global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pairs,
+                                                  const uint64_t *__restrict__ offs, uint32_t npairs, uint64_t N,
+                                                  TierCfg cfg, uint8_t *tier, uint32_t *dom, unsigned *misc) {
+    __shared__ unsigned s_hist[kBuckets];
     __shared__ unsigned s_sup[kTiers]; // roots of pairs that take no items, by domain size
+    for (uint32_t i = threadIdx.x; i < kBuckets; i += blockDim.x)
+        s_hist[i] = 0;
     if (threadIdx.x < kTiers)
         s_sup[threadIdx.x] = 0;
-    for (int i = threadIdx.x; i < kTiers * kSlots; i += blockDim.x)
-        s_hist[i] = 0;
-    for (int i = threadIdx.x; i < kSlots; i += blockDim.x)
-        s_tiny[i] = 0;
     __syncthreads();
     uint32_t mx[kTiers] = {0, 0, 0, 0, 0};
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x) {
@@ -3343,7 +3376,7 @@ __global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__
             D = deg;
             j0 = pd.pl.pos1_after_root ? sp : 0;
         }
-        uint8_t tc = 0;
+        uint32_t tc = 0;
         // roots: degree in [max_qdeg, cap) (subgraph_matching.cuh:1086-1098),
         // enough domain vertices for the other dend-1 positions and at least
         // one level-1 vertex
@@ -3357,78 +3390,134 @@ __global__ void k_classify(const PairDev *__restrict__ pairs, const uint64_t *__
         } else if (root_ok && D + 1 >= (uint32_t)pd.pl.dend) {
             tc = D <= cfg.small_max ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
         }
-        tier[t] = tc;
+        tier[t] = (uint8_t)tc;
         dom[t] = D;
+        if (!tc)
+            continue;
         if (pd.sup) {
-            if (tc)
-                atomicAdd(&s_sup[tc - 1], 1u);
+            atomicAdd(&s_sup[tc - 1], 1u);
             continue;
         }
         if (tc == 4) {
             const uint32_t rn = pd.pl.rows_needed, rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
-            atomicAdd(large_words, (unsigned long long)large_root_words(D, rlo, pd.pl.nbhd != kNbNone));
+            atomicAdd(reinterpret_cast<unsigned long long *>(misc + kMiscLarge),
+                      (unsigned long long)large_root_words(D, rlo, pd.pl.nbhd != kNbNone));
         }
-        if (tc) {
-            mx[tc - 1] = max(mx[tc - 1], D);
-            const uint32_t slot = depth_slot(pd.pl, tc, pd.en.out != nullptr);
-            atomicAdd(&s_hist[(tc - 1) * kSlots + slot], 1u);
-            if (tc == 1 && D <= cfg.tiny_max)
-                atomicAdd(&s_tiny[slot], 1u);
-        }
+        mx[tc - 1] = max(mx[tc - 1], D);
+        const uint32_t slot = depth_slot(pd.pl, tc, pd.en.out != nullptr);
+        atomicAdd(&s_hist[((tc - 1) * kSlots + slot) * kDomClasses + dom_class(tc, D)], 1u);
     }
 #pragma unroll
     for (int k = 0; k < kTiers; ++k) {
         const uint32_t m = __reduce_max_sync(kFull, mx[k]);
         if ((threadIdx.x & 31) == 0 && m)
-            atomicMax(&tier_max[k], m);
+            atomicMax(&misc[k], m);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kTiers * kSlots; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < kBuckets; i += blockDim.x)
         if (s_hist[i])
-            atomicAdd(&tier_depth[i], s_hist[i]);
-    for (int i = threadIdx.x; i < kSlots; i += blockDim.x)
-        if (s_tiny[i])
-            atomicAdd(&tiny_depth[i], s_tiny[i]);
+            atomicAdd(&misc[kMiscBuckets + i], s_hist[i]);
     if (threadIdx.x < kTiers && s_sup[threadIdx.x])
-        atomicAdd(&sup_tiers[threadIdx.x], s_sup[threadIdx.x]);
+        atomicAdd(&misc[kMiscSup + threadIdx.x], s_sup[threadIdx.x]);
 }
 
-// Sort keys of every flattened vertex for all item lists at once:
-// (tier, depth slot, domain order) -- small roots by domain ascending, medium and
-// large ones by domain descending (heaviest first), list-walker roots by
-// depth only; non-roots last.
-__global__ void k_list_keys(const uint8_t *__restrict__ tier, const uint32_t *__restrict__ dom,
-                            const PairDev *__restrict__ pairs, const uint64_t *__restrict__ offs, uint32_t npairs,
-                            uint64_t N, uint32_t *keys, uint32_t *vals) {
-    constexpr uint32_t kDomMask = (1u << 24) - 1u;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t tc = tier[t];
-        uint32_t key = 0xffffffffu, p = 0;
-        if (tc) {
-            p = find_pair(offs, npairs, t);
-            if (pairs[p].sup)
-                tc = 0; // takes no items
+// Bucket counts -> offsets (in place), roots per (tier, slot) and tiny roots
+// per slot. One block.
+__global__ void __launch_bounds__(1024) k_list_offsets(unsigned *misc, uint32_t tiny_max) {
+    constexpr uint32_t kPer = (kBuckets + 1023) / 1024;
+    __shared__ uint32_t s_warp[32];
+    unsigned *cnt = misc + kMiscBuckets;
+    const uint32_t i0 = threadIdx.x * kPer, i1 = min(i0 + kPer, kBuckets);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+        c[k] = i0 + k < i1 ? cnt[i0 + k] : 0u;
+        sum += c[k];
+        if (c[k]) {
+            const uint32_t ts = (i0 + k) / kDomClasses; // tier * kSlots + slot
+            atomicAdd(&misc[kMiscSlots + ts], c[k]);
+            if (ts < (uint32_t)kSlots && (i0 + k) % kDomClasses <= tiny_max)
+                atomicAdd(&misc[kMiscTiny + ts], c[k]);
         }
-        if (tc) {
-            const uint32_t slot = depth_slot(pairs[p].pl, tc, pairs[p].en.out != nullptr);
-            const uint32_t d = min(dom[t], kDomMask);
-            const uint32_t dk = tc == 1 ? d : (tc == 5 ? 0u : kDomMask - d);
-            key = ((tc - 1) << 29) | (slot << 24) | dk;
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, inc, o);
+        if (lane >= o)
+            inc += y;
+    }
+    if (lane == 31)
+        s_warp[wp] = inc;
+    __syncthreads();
+    uint32_t base = inc - sum;
+    for (int w = 0; w < wp; ++w)
+        base += s_warp[w];
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+        if (i0 + k < i1) {
+            cnt[i0 + k] = base;
+            base += c[k];
         }
-        keys[t] = key;
-        vals[t] = (uint32_t)t;
+}
+
+// Items (pair << 32 | root) of every root at its bucket's next place; one
+// atomic per warp and bucket.
+__global__ void __launch_bounds__(256) k_list_fill(const PairDev *__restrict__ pairs,
+                                                   const uint64_t *__restrict__ offs, uint32_t npairs, uint64_t N,
+                                                   const uint8_t *__restrict__ tier, const uint32_t *__restrict__ dom,
+                                                   unsigned *misc, uint64_t *items) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < N; t0 += step) {
+        const uint64_t t = t0 + (uint64_t)lane;
+        uint32_t bucket = 0xffffffffu, p = 0;
+        if (t < N) {
+            const uint32_t tc = tier[t];
+            if (tc) {
+                p = find_pair(offs, npairs, t);
+                const PairDev &pd = pairs[p];
+                if (!pd.sup)
+                    bucket = ((tc - 1) * kSlots + depth_slot(pd.pl, tc, pd.en.out != nullptr)) * kDomClasses +
+                             dom_class(tc, dom[t]);
+            }
+        }
+        const unsigned peers = __match_any_sync(kFull, bucket);
+        const int first = __ffs(peers) - 1;
+        uint32_t at = 0;
+        if (lane == first && bucket != 0xffffffffu)
+            at = atomicAdd(&misc[kMiscBuckets + bucket], (uint32_t)__popc(peers));
+        at = __shfl_sync(kFull, at, first) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        if (bucket != 0xffffffffu)
+            items[at] = ((uint64_t)p << 32) | (uint64_t)(t - offs[p]);
     }
 }
 
-// Sorted flattened indices of the roots -> items (pair << 32 | root).
-__global__ void k_make_items(const uint32_t *__restrict__ sorted, uint32_t n, const uint64_t *__restrict__ offs,
-                             uint32_t npairs, uint64_t *items) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t t = sorted[i];
-        const uint32_t p = find_pair(offs, npairs, t);
-        items[i] = ((uint64_t)p << 32) | (uint64_t)(t - offs[p]);
+// The device copy of a call's pairs for up to kPackPairs of them: they travel
+// as a kernel argument (a copy from pageable host memory would wait for the
+// stream) and the same launch clears the planning block.
+constexpr uint32_t kPackPairs = 4;
+struct PairPack {
+    PairDev p[kPackPairs];
+    uint64_t offs[kPackPairs + 1];
+};
+static_assert(sizeof(PairPack) <= 3500, "a kernel argument");
+__global__ void k_put_pairs(const __grid_constant__ PairPack pk, uint32_t np, PairDev *pairs, uint64_t *offs,
+                            unsigned *misc) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    if (blockIdx.x == 0) {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(&pk.p[0]);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(pairs);
+        for (uint32_t i = threadIdx.x; i < np * (uint32_t)(sizeof(PairDev) / 4); i += blockDim.x)
+            dst[i] = src[i];
+        if (threadIdx.x <= np)
+            offs[threadIdx.x] = pk.offs[threadIdx.x];
     }
+    for (uint32_t i = t; i < kMiscWords; i += nt)
+        misc[i] = 0;
 }
+static_assert(sizeof(PairDev) % 4 == 0, "copied by words");
 
 // Arena words, row chunks and level-1 tasks of each listed large root
 // (D, j0 from k_gather_dom).
@@ -3751,6 +3840,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     std::vector<PairDev> hp;
     std::vector<uint64_t> offs{0};
     std::vector<Graph *> dropped;
+    bool built_any = false;
     // Pairs counted from degrees and triangle counts: whole counts only (the
     // sums are not per root). Their view is an ascending one whose peel
     // removes no more than theirs would: peeled vertices are in no match, and
@@ -3796,6 +3886,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 qdeg = it->second;
         }
         BEEP_TRY(get_view(ctx, ps.g, qdeg, asc, false, &v, &built));
+        built_any = built_any || built;
         lp->views.push_back(v);
         st.peel_rounds = v->peel_rounds; // view-build launches are counted where they happen
         if (v->n == 0)
@@ -3867,38 +3958,44 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     bool items = false; // some pair's roots go through the tiers
     for (auto &pd : hp)
         items = items || !pd.sup;
-    uint32_t *d_dom, *d_sel = nullptr, *d_keys = nullptr, *d_keys2 = nullptr;
+    uint32_t *d_dom, *d_sel = nullptr, *d_keys = nullptr;
     unsigned *d_misc;
+    uint64_t *all_items = nullptr;
     BEEP_TRY(lp->alloc(d_dom, N));
-    if (items) {
-        BEEP_TRY(lp->alloc(d_sel, N));
-        BEEP_TRY(lp->alloc(d_keys, N));
-        BEEP_TRY(lp->alloc(d_keys2, N));
+    BEEP_TRY(lp->alloc(d_misc, kMiscWords));
+    if (np <= kPackPairs) {
+        PairPack pk;
+        std::memset(&pk, 0, sizeof(pk));
+        std::copy(hp.begin(), hp.end(), pk.p);
+        std::copy(offs.begin(), offs.end(), pk.offs);
+        k_put_pairs<<<8, 256, 0, s>>>(pk, np, lp->d_pairs, lp->d_offs, d_misc);
+        BEEP_CUDA_TRY(cudaGetLastError());
+        st.kernel_launches += 1;
+    } else {
+        BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_pairs, hp.data(), np * sizeof(PairDev), cudaMemcpyHostToDevice, s));
+        BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_offs, offs.data(), (np + 1) * 8, cudaMemcpyHostToDevice, s));
+        BEEP_CUDA_TRY(cudaMemsetAsync(d_misc, 0, kMiscWords * 4, s));
     }
-    BEEP_TRY(lp->alloc(d_misc, 256));
-    BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_pairs, hp.data(), np * sizeof(PairDev), cudaMemcpyHostToDevice, s));
-    BEEP_CUDA_TRY(cudaMemcpyAsync(lp->d_offs, offs.data(), (np + 1) * 8, cudaMemcpyHostToDevice, s));
-    BEEP_CUDA_TRY(cudaMemsetAsync(d_misc, 0, 256 * 4, s));
-    const int gv = std::max(1, (int)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->num_sms * 32));
-    // d_misc: [0, 8) largest domain per tier, [8, 8 + kTiers * kSlots) roots
-    // per (tier, depth slot), [120, 120 + kSlots) tiny small-tier roots per
-    // slot, [144, 146) arena words of the large tier (u64)
-    // and [148, 148 + kTiers) roots per tier of the pairs that take no items
-    constexpr int kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144, kMiscSup = 148;
-    static_assert(kMiscSlots + kTiers * kSlots <= kMiscTiny && kMiscTiny + kSlots <= kMiscLarge, "d_misc layout");
     TierCfg cfg = tiers;
     cfg.tiny_max = std::min<uint32_t>(cfg.tiny_max, kTinyMaxD);
     cfg.small_max = std::min<uint32_t>(cfg.small_max, kSmallMaxD);
     cfg.med_a_max = std::min<uint32_t>(cfg.med_a_max, kMediumAMaxD);
     cfg.med_max = std::min<uint32_t>(cfg.med_max, kMediumMaxD);
-    k_classify<<<gv, 256, 0, s>>>(lp->d_pairs, lp->d_offs, np, N, cfg, lp->d_tier, d_dom, d_misc,
-                                  d_misc + kMiscSlots, d_misc + kMiscTiny,
-                                  reinterpret_cast<unsigned long long *>(d_misc + kMiscLarge), d_misc + kMiscSup);
+    // (few blocks: each clears and flushes the bucket counts)
+    const int gc = std::max(1, (int)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->num_sms * 4));
+    k_classify<<<gc, 256, 0, s>>>(lp->d_pairs, lp->d_offs, np, N, cfg, lp->d_tier, d_dom, d_misc);
     BEEP_CUDA_TRY(cudaGetLastError());
     st.kernel_launches += 1;
-    unsigned h_misc[kMiscLarge + 2] = {0};
-    if (items) { // the tiers' sizes decide the launches
+    unsigned h_misc[kMiscBuckets] = {0};
+    if (items) { // the lists; the tiers' sizes decide the launches
+        BEEP_TRY(lp->alloc(all_items, N));
+        k_list_offsets<<<1, 1024, 0, s>>>(d_misc, cfg.tiny_max);
+        BEEP_CUDA_TRY(cudaGetLastError());
         BEEP_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
+        const int gf = std::max(1, (int)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->num_sms * 16));
+        k_list_fill<<<gf, 256, 0, s>>>(lp->d_pairs, lp->d_offs, np, N, lp->d_tier, d_dom, d_misc, all_items);
+        BEEP_CUDA_TRY(cudaGetLastError());
+        st.kernel_launches += 2;
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
     }
     if (!sups.empty())
@@ -3970,25 +4067,13 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         return BEEP_OK;
     };
 
-    // All item lists by one sort of (tier, depth, domain order) keys over the
-    // flattened vertices; tier k's list is a contiguous run of the result.
-    uint64_t *all_items = nullptr;
+    // tier k's list is a contiguous run of the items
     uint32_t list_off[kTiers + 1] = {0};
     for (int k = 0; k < kTiers; ++k)
         list_off[k + 1] = list_off[k] + tier_n[k];
-    BEEP_TRY(lp->alloc(all_items, list_off[kTiers]));
-    if (list_off[kTiers] > 0) {
-        k_list_keys<<<gv, 256, 0, s>>>(lp->d_tier, d_dom, lp->d_pairs, lp->d_offs, np, N, d_keys, d_sel);
-        BEEP_CUDA_TRY(cudaGetLastError());
-        size_t tb = 0;
-        BEEP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, d_keys, d_keys2, d_sel, d_dom, N, 0, 32, s));
-        BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
-        BEEP_CUDA_TRY(
-            cub::DeviceRadixSort::SortPairs(ctx->scratch.ptr, tb, d_keys, d_keys2, d_sel, d_dom, N, 0, 32, s));
-        k_make_items<<<std::max(1u, std::min(list_off[kTiers] / 256 + 1, 4096u)), 256, 0, s>>>(
-            d_dom, list_off[kTiers], lp->d_offs, np, all_items);
-        BEEP_CUDA_TRY(cudaGetLastError());
-        st.kernel_launches += 2;
+    if (tier_n[3] > 0 || tier_n[4] > 0) { // domains and level-1 starts of listed roots
+        BEEP_TRY(lp->alloc(d_keys, std::max(tier_n[3], tier_n[4])));
+        BEEP_TRY(lp->alloc(d_sel, std::max(tier_n[3], tier_n[4])));
     }
     auto make_list = [&](int k, uint64_t *&list) -> beep_status {
         list = all_items + list_off[k];
@@ -3997,8 +4082,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
 
     // large tier, one batch planned on the device when every root's bitmap
     // fits the arena at once (the arena words were summed by k_classify)
-    size_t arena_cap = 0;
-    if (tier_n[3] > 0) {
+    size_t arena_cap = (size_t)256 << 20;
+    if (tier_n[3] > 0 && large_words * 4 > arena_cap) { // the free memory is asked for only when it matters
         size_t free_b = 0, total_b = 0;
         BEEP_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         arena_cap = std::max<size_t>((size_t)256 << 20, std::min<size_t>((size_t)48 << 30, free_b / 2));
@@ -4041,13 +4126,12 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         size_t tb = 0, tb2 = 0;
         BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb, words, boff + 1, nl, s));
         BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb2, chunks, cstart + 1, nl, s));
-        BEEP_TRY(ctx->grow(ctx->scratch, std::max(tb, tb2) + 1024));
-        tb = ctx->scratch.bytes;
-        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(ctx->scratch.ptr, tb, words, boff + 1, nl, s));
-        tb = ctx->scratch.bytes;
-        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(ctx->scratch.ptr, tb, chunks, cstart + 1, nl, s));
-        tb = ctx->scratch.bytes;
-        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(ctx->scratch.ptr, tb, tasks, tstart + 1, nl, s));
+        uint8_t *tmp = nullptr; // the plan's own: the context's scratch may serve another stream's plan
+        tb = std::max(tb, tb2);
+        BEEP_TRY(lp->alloc(tmp, tb));
+        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, words, boff + 1, nl, s));
+        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, chunks, cstart + 1, nl, s));
+        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, tasks, tstart + 1, nl, s));
         BEEP_CUDA_TRY(cudaMemsetAsync(boff, 0, 8, s));
         BEEP_CUDA_TRY(cudaMemsetAsync(cstart, 0, 4, s));
         BEEP_CUDA_TRY(cudaMemsetAsync(tstart, 0, 4, s));
@@ -4327,10 +4411,10 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         st.kernel_launches += 2;
         BEEP_CUDA_TRY(cudaGetLastError());
         size_t tb = 0;
-        BEEP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, tasks, tstart, nl + 1, s));
-        BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
-        // tasks[nl] is not written: scan nl entries, then the total into tstart[nl]
-        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(ctx->scratch.ptr, tb, tasks, tstart + 1, nl, s));
+        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb, tasks, tstart + 1, nl, s));
+        uint8_t *tmp = nullptr;
+        BEEP_TRY(lp->alloc(tmp, tb));
+        BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, tasks, tstart + 1, nl, s));
         BEEP_CUDA_TRY(cudaMemsetAsync(tstart, 0, 4, s));
         uint32_t first = 0;
         for (int sl = 0; sl < kSlots; ++sl) {
@@ -4437,7 +4521,12 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     lp->nexit = (uint32_t)lp->recs.size();
     BEEP_TRY(lp->alloc(lp->d_exit, 2 * (size_t)lp->nexit));
     BEEP_TRY(ctx->host_results(lp->host_words(), &lp->h_counts));
-    BEEP_CUDA_TRY(cudaStreamSynchronize(s)); // planning buffers are final
+    // A view built here is cached on its graph, and its build used the
+    // context's scratch: other streams (another slot of a server, another
+    // context) may use both once this call returns. Otherwise nothing waits:
+    // the host arrays copied above were pageable, consumed by the copies.
+    if (built_any)
+        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
     tr.mark("lists");
     *out = std::move(lp);
     return BEEP_OK;
