@@ -3025,12 +3025,15 @@ __device__ __forceinline__ uint32_t sup_row_of(const uint32_t *__restrict__ rp, 
     return lo;
 }
 
-// Row of entry e0 + lane for the lanes with e0 + lane < m (no row is empty,
-// so it is within 31 rows of e0's).
+// Row of entry e in [e0, e0 + 32), e < m: within 32 rows of e0's unless some
+// are empty (a view has no empty row, a caller's CSR may).
 __device__ __forceinline__ uint32_t sup_warp_row(const uint32_t *__restrict__ rp, uint32_t n, uint32_t e0,
                                                  uint32_t e) {
     const uint32_t u0 = sup_row_of(rp, 0, n, e0);
-    return sup_row_of(rp, u0, min(n, u0 + 32), e);
+    uint64_t step = 32;
+    while (n - u0 > step && rp[u0 + step] <= e)
+        step <<= 1;
+    return sup_row_of(rp, u0, (uint32_t)min(u0 + step, (uint64_t)n), e);
 }
 
 constexpr int kSupWarps = 8;
@@ -3659,6 +3662,26 @@ template <int D, bool ENUM> beep_status set_medium_attr(size_t smem) {
     BEEP_TRY(raise_smem_limit((const void *)k_medium<D, ENUM, 0>, smem));
     BEEP_TRY(raise_smem_limit((const void *)k_medium<D, ENUM, 32>, smem));
     return BEEP_OK;
+}
+
+// Block size, shared memory and blocks per SM of a medium launch (sub-tier 0:
+// thread walker, 1: warp walker) over domains of up to maxD vertices.
+struct MediumShape {
+    int block, per_sm;
+    size_t smem;
+};
+MediumShape medium_shape(int sub, uint32_t maxD) {
+    // 32-bit words per row: 8 (4 x 64 bits) in the thread-mode sub-tier;
+    // clique rows take an odd number
+    const uint32_t W = clique_stride(sub == 0 ? 2 * kThreadNW : (maxD + 31) / 32);
+    const size_t pad = (maxD + 4) & ~3u;
+    // the domain hash: nslots ids, nslots 16-bit indices and the filter
+    const size_t nslots = hash_slots(maxD);
+    MediumShape ms;
+    ms.smem = (4 * pad + nslots + nslots / 2 + nslots / 4 + (size_t)maxD * W) * 4;
+    ms.block = sub == 0 ? 256 : 1024;
+    ms.per_sm = std::max(1, (int)std::min<size_t>(2048 / ms.block, (200 * 1024) / (ms.smem + 1024)));
+    return ms;
 }
 
 template <bool ENUM>
@@ -4332,15 +4355,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         uint64_t *list = nullptr;
         BEEP_TRY(make_list(k, list));
         const uint32_t maxD = tier_max[k];
-        // 32-bit words per row: 8 (4 x 64 bits) in the thread-mode sub-tier;
-        // clique rows take an odd number
-        const uint32_t W = clique_stride(sub == 0 ? 2 * kThreadNW : (maxD + 31) / 32);
-        const size_t pad = (maxD + 4) & ~3u;
-        // the domain hash: nslots ids, nslots 16-bit indices and the filter
-        const size_t nslots = hash_slots(maxD);
-        const size_t smem = (4 * pad + nslots + nslots / 2 + nslots / 4 + (size_t)maxD * W) * 4;
-        const int block = sub == 0 ? 256 : 1024;
-        const int per_sm = std::max(1, (int)std::min<size_t>(2048 / block, (200 * 1024) / (smem + 1024)));
+        const MediumShape ms = medium_shape(sub, maxD);
+        const size_t smem = ms.smem;
+        const int block = ms.block, per_sm = ms.per_sm;
         uint32_t first = 0;
         for (int sl = 0; sl < kSlots; ++sl) {
             const uint32_t cnt = tier_depth[k * kSlots + sl];
@@ -4976,10 +4993,12 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[BEEP_NOALLOC_SC
 
 struct NoAllocCtrl {
     unsigned long long count;    // the match count ...
-    unsigned long long overflow; // ... and its overflow flag (the word after it)
+    unsigned long long overflow; // ... and its overflow flag (the word after it),
+    unsigned long long nb[4];    // then a pair counter's statistics words
     unsigned int cursor;
     unsigned int max_domain;
     unsigned int bad_csr;        // bit 0: row pointers, bit 1: column entries
+    unsigned int cursors[4];     // work cursors of the tier launches
 };
 static_assert(sizeof(NoAllocCtrl) <= kNoAllocCtrlBytes, "control block");
 
@@ -5020,7 +5039,7 @@ __device__ __forceinline__ bool csr_is_root(const DevPlan &pl, uint32_t deg, uin
 // of the valid rows. Entries of a row are read only when its pointers are
 // valid, so a bad CSR is reported, never read out of bounds.
 __global__ void k_noalloc_maxdom(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ col, int64_t n,
-                                 int64_t m, DevPlan pl, uint32_t min_deg, NoAllocCtrl *ctrl) {
+                                 int64_t m, DevPlan pl, uint32_t min_deg, NoAllocCtrl *ctrl, uint32_t *split) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     uint32_t mx = 0, bad = 0;
@@ -5040,6 +5059,8 @@ __global__ void k_noalloc_maxdom(const uint32_t *__restrict__ rp, const uint32_t
             csr_root_domain(rp, col, pl, (uint32_t)v, beg, D, j0, deg);
             if (csr_is_root(pl, deg, D, j0, min_deg))
                 mx = max(mx, D);
+            if (split)
+                split[v] = lower_bound_g(col, b, e, (uint32_t)v) - b;
         }
     }
     mx = __reduce_max_sync(kFull, mx);
@@ -5094,18 +5115,18 @@ __device__ __forceinline__ void csr_build_rows(const uint32_t *__restrict__ rp, 
     __syncthreads();
 }
 
-// Block per root over every vertex (the medium-tier kernel reading the
-// caller's CSR); rows in shared memory up to smem_maxD, else in this block's
-// slice of the scratch array.
+// Block per root, over every vertex or over a list of roots; rows in shared
+// memory up to smem_maxD, else in this block's slice of the scratch array.
 template <int DEND>
 __global__ void __launch_bounds__(512) k_noalloc_count(const uint32_t *__restrict__ rp,
                                                        const uint32_t *__restrict__ col, int64_t n, DevPlan pl,
                                                        uint32_t min_deg, unsigned char *scratch,
-                                                       uint64_t slice_words, uint32_t smem_maxD) {
+                                                       uint32_t *slices, uint64_t slice_words, uint32_t smem_maxD,
+                                                       const uint64_t *__restrict__ list, uint32_t nlist) {
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t s_v, s_j;
     NoAllocCtrl *ctrl = reinterpret_cast<NoAllocCtrl *>(scratch);
-    uint32_t *slice = reinterpret_cast<uint32_t *>(scratch + kNoAllocCtrlBytes) + (uint64_t)blockIdx.x * slice_words;
+    uint32_t *slice = slices + (uint64_t)blockIdx.x * slice_words;
     const uint32_t pad = (smem_maxD + 4) & ~3u;
     uint32_t *sA = sm, *s_hb = sm + pad, *s_pre = sm + 2 * pad, *srows = sm + 3 * pad;
     const int lane = threadIdx.x & 31;
@@ -5116,9 +5137,11 @@ __global__ void __launch_bounds__(512) k_noalloc_count(const uint32_t *__restric
         if (threadIdx.x == 0)
             s_v = atomicAdd(&ctrl->cursor, 1u);
         __syncthreads();
-        const uint32_t v = s_v;
-        if ((int64_t)v >= n)
+        uint32_t v = s_v;
+        if (list ? v >= nlist : (int64_t)v >= n)
             break;
+        if (list)
+            v = item_root(list[v]);
         uint32_t beg, D, j0, deg;
         csr_root_domain(rp, col, pl, v, beg, D, j0, deg);
         if (csr_is_root(pl, deg, D, j0, min_deg)) {
@@ -5210,9 +5233,36 @@ extern "C" beep_status beep_count_noalloc(int device, void *cuda_stream, int64_t
     BEEP_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device));
     BEEP_CUDA_TRY(cudaMemsetAsync(scratch, 0, kNoAllocCtrlBytes, s));
     const uint32_t min_deg = (uint32_t)plan.info.max_qdeg;
+    // The tier kernels read the caller's CSR as a view in vertex-id order: the
+    // split points, the root classification and the item lists are laid out in
+    // the scratch array, 17 bytes a vertex (up to 3.9 million vertices);
+    // larger graphs take a block per vertex. (Diamonds, R-MAT s15 ef6: 3.42 ->
+    // 0.55 ms.)
+    unsigned char *const arena = static_cast<unsigned char *>(scratch) + kNoAllocCtrlBytes;
+    size_t used = 0;
+    auto take = [&](size_t bytes) {
+        unsigned char *p = arena + used;
+        used += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    PairDev *d_pair = reinterpret_cast<PairDev *>(take(sizeof(PairDev)));
+    uint64_t *d_offs = reinterpret_cast<uint64_t *>(take(16));
+    unsigned *d_misc = reinterpret_cast<unsigned *>(take(kMiscWords * 4));
+    SupView *d_sup = reinterpret_cast<SupView *>(take(sizeof(SupView)));
+    const size_t fixed = used;
+    const bool tiered = (uint64_t)n * 17 + 4 * 256 + fixed <= kNoAllocArenaWords * 4;
+    uint32_t *d_split = nullptr, *d_dom = nullptr;
+    uint8_t *d_tier = nullptr;
+    uint64_t *d_items = nullptr;
+    if (tiered) {
+        d_split = reinterpret_cast<uint32_t *>(take((size_t)n * 4));
+        d_dom = reinterpret_cast<uint32_t *>(take((size_t)n * 4));
+        d_tier = take((size_t)n);
+        d_items = reinterpret_cast<uint64_t *>(take((size_t)n * 8));
+    }
     if (n > 0) {
         const int g0 = (int)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)num_sms * 16));
-        k_noalloc_maxdom<<<g0, 256, 0, s>>>(rp, col, n, m, pl, min_deg, ctrl);
+        k_noalloc_maxdom<<<g0, 256, 0, s>>>(rp, col, n, m, pl, min_deg, ctrl, d_split);
         BEEP_CUDA_TRY(cudaGetLastError());
     }
     uint32_t h_ctrl[2] = {0, 0}; // max_domain, bad_csr
@@ -5230,29 +5280,156 @@ extern "C" beep_status beep_count_noalloc(int device, void *cuda_stream, int64_t
         return BEEP_OK;
     }
     const uint32_t smem_maxD = (uint32_t)kMediumMaxD;
-    const uint64_t arena_words = kNoAllocArenaWords;
-    uint64_t slice_words = 0;
-    int grid = num_sms;
-    if (maxD > smem_maxD) {
-        slice_words = noalloc_slice_words(maxD);
-        if (maxD > BEEP_NOALLOC_MAX_DOMAIN)
-            return fail(BEEP_ERR_UNSUPPORTED,
-                        "beep_count_noalloc: the largest search domain has " + std::to_string(maxD) +
-                            " vertices; its bitmap needs " + std::to_string(slice_words * 4) +
-                            " bytes, more than the " + std::to_string(BEEP_NOALLOC_SCRATCH_BYTES) +
-                            "-byte scratch of the allocation-free path (domains up to " +
-                            std::to_string(BEEP_NOALLOC_MAX_DOMAIN) + " vertices); use beep_count");
-        grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms, arena_words / slice_words));
+    const uint64_t slice_words = maxD > smem_maxD ? noalloc_slice_words(maxD) : 0;
+    if (maxD > BEEP_NOALLOC_MAX_DOMAIN)
+        return fail(BEEP_ERR_UNSUPPORTED,
+                    "beep_count_noalloc: the largest search domain has " + std::to_string(maxD) +
+                        " vertices; its bitmap needs " + std::to_string(slice_words * 4) +
+                        " bytes, more than the " + std::to_string(BEEP_NOALLOC_SCRATCH_BYTES) +
+                        "-byte scratch of the allocation-free path (domains up to " +
+                        std::to_string(BEEP_NOALLOC_MAX_DOMAIN) + " vertices); use beep_count");
+    unsigned char *scr = static_cast<unsigned char *>(scratch);
+    const ViewDev view{rp, col, d_split, nullptr};
+    unsigned long long h_out[6] = {0, 0, 0, 0, 0, 0}; // a pair counter
+    auto finish = [&]() -> beep_status {
+        BEEP_CUDA_TRY(cudaMemcpyAsync(h_out, &ctrl->count, sizeof(h_out), cudaMemcpyDeviceToHost, s));
+        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+        const unsigned long long st = h_out[2] - h_out[4], c = h_out[0] + st;
+        if (h_out[1] || h_out[3] || h_out[5] || h_out[2] < h_out[4] || c < st || c >= kCountLimit) {
+            *out_count = BEEP_COUNT_OVERFLOW;
+            return fail(BEEP_ERR_OVERFLOW,
+                        "beep_count_noalloc: the count is at least BEEP_COUNT_LIMIT (2^64 - 2^52)");
+        }
+        *out_count = c;
+        return BEEP_OK;
+    };
+    // degree and triangle-count forms, where their counters fit the scratch
+    const bool sup_cnt = pl.support == kSupDiamond || pl.support == kSupBook3 || pl.support == kSupWedgeIso ||
+                         pl.support == kSupTwoEdges;
+    const size_t sup_words = sup_cnt ? (size_t)m : 0, sup_tv = pl.support == kSupTwoEdges ? (size_t)n : 0;
+    if (tiered && pl.support &&
+        fixed + (size_t)n * 4 + 256 + sup_words * 4 + 256 + sup_tv * 8 + 256 <= kNoAllocArenaWords * 4) {
+        used = fixed;
+        take((size_t)n * 4); // the split points
+        SupView sv;
+        std::memset(&sv, 0, sizeof(sv));
+        sv.v = view;
+        sv.n = (uint32_t)n;
+        sv.out[pl.support] = &ctrl->count;
+        if (sup_words) {
+            sv.cnt = reinterpret_cast<uint32_t *>(take(sup_words * 4));
+            BEEP_CUDA_TRY(cudaMemsetAsync(sv.cnt, 0, sup_words * 4, s));
+        }
+        if (sup_tv) {
+            sv.tv = reinterpret_cast<unsigned long long *>(take(sup_tv * 8));
+            BEEP_CUDA_TRY(cudaMemsetAsync(sv.tv, 0, sup_tv * 8, s));
+        }
+        BEEP_CUDA_TRY(cudaMemcpyAsync(d_sup, &sv, sizeof(sv), cudaMemcpyHostToDevice, s));
+        const uint64_t nchunks = ((uint64_t)m + 31) / 32;
+        const int gk = (int)std::max<int64_t>(
+            1, std::min<int64_t>((int64_t)((nchunks + kSupWarps - 1) / kSupWarps), (int64_t)num_sms * 8));
+        if (pl.support < kSupStar2) {
+            k_sup_triangles<<<gk, kSupWarps * 32, 0, s>>>(d_sup, 1, nchunks, nullptr);
+            BEEP_CUDA_TRY(cudaGetLastError());
+        }
+        if (sup_words) {
+            k_sup_edges<<<gk, 256, 0, s>>>(d_sup, 1, nchunks);
+            BEEP_CUDA_TRY(cudaGetLastError());
+        }
+        if (sup_tv || pl.support >= kSupStar2) {
+            k_sup_vertices<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms * 4), 256, 0, s>>>(d_sup, 1);
+            BEEP_CUDA_TRY(cudaGetLastError());
+        }
+        return finish();
     }
+    uint32_t *slices = reinterpret_cast<uint32_t *>(scr + kNoAllocCtrlBytes);
+    uint64_t arena_words = kNoAllocArenaWords;
+    const uint64_t *big = nullptr; // the roots with domains above smem_maxD, when they are listed
+    uint32_t nbig = 0;
+    if (tiered && used + slice_words * 4 <= kNoAllocArenaWords * 4) {
+        slices = reinterpret_cast<uint32_t *>(arena + used);
+        arena_words -= used / 4;
+        PairPack pk;
+        std::memset(&pk, 0, sizeof(pk));
+        PairDev &pd = pk.p[0];
+        pd.v = view;
+        pd.pl = pl;
+        pd.count = &ctrl->count;
+        pd.min_deg = min_deg;
+        pd.cap_deg = 0xffffffffu;
+        pd.shard_mod = 1;
+        pk.offs[1] = (uint64_t)n;
+        k_put_pairs<<<8, 256, 0, s>>>(pk, 1, d_pair, d_offs, d_misc);
+        BEEP_CUDA_TRY(cudaGetLastError());
+        TierCfg cfg;
+        const int gc = (int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms * 4);
+        k_classify<<<gc, 256, 0, s>>>(d_pair, d_offs, 1, (uint64_t)n, cfg, d_tier, d_dom, d_misc);
+        k_list_offsets<<<1, 1024, 0, s>>>(d_misc, cfg.tiny_max);
+        BEEP_CUDA_TRY(cudaGetLastError());
+        unsigned h_misc[kMiscBuckets] = {0};
+        BEEP_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
+        k_list_fill<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms * 16), 256, 0, s>>>(
+            d_pair, d_offs, 1, (uint64_t)n, d_tier, d_dom, d_misc, d_items);
+        BEEP_CUDA_TRY(cudaGetLastError());
+        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+        uint32_t tier_n[4] = {0, 0, 0, 0}, tiny = 0;
+        for (int k = 0; k < 4; ++k)
+            for (int d = 0; d < kSlots; ++d)
+                tier_n[k] += h_misc[kMiscSlots + k * kSlots + d];
+        for (int d = 0; d < kSlots; ++d)
+            tiny += h_misc[kMiscTiny + d];
+        const uint32_t parts = walk_parts(pl.dend, false);
+        // the long blocks first; all on the caller's stream
+        for (int sub = 1; sub >= 0; --sub) {
+            const uint32_t cnt = tier_n[1 + sub];
+            if (!cnt)
+                continue;
+            const uint64_t *list = d_items + tier_n[0] + (sub ? tier_n[1] : 0);
+            const MediumShape ms = medium_shape(sub, h_misc[1 + sub]);
+            const int grid = num_sms * ms.per_sm;
+            unsigned *cur = &ctrl->cursors[sub];
+#define BEEP_CASE(DD)                                                                                              \
+    case DD:                                                                                                       \
+        BEEP_TRY((set_medium_attr<DD, false>(ms.smem)));                                                           \
+        if (sub == 0)                                                                                              \
+            k_medium<DD, false, 0><<<grid, ms.block, ms.smem, s>>>(d_pair, list, cnt, parts, cur,                  \
+                                                                   h_misc[1 + sub], nullptr);                      \
+        else                                                                                                       \
+            k_medium<DD, false, 32><<<grid, ms.block, ms.smem, s>>>(d_pair, list, cnt, parts, cur,                 \
+                                                                    h_misc[1 + sub], nullptr);                     \
+        break;
+            BEEP_DEPTH_SWITCH(pl.dend, BEEP_CASE)
+#undef BEEP_CASE
+            BEEP_CUDA_TRY(cudaGetLastError());
+        }
+        for (int part = 0; part < 2; ++part) {
+            const uint32_t cnt = part == 0 ? tiny : tier_n[0] - tiny;
+            if (!cnt)
+                continue;
+            const int group = part == 0 ? 8 : 32, per_block = kSmallWarps * 32 / group;
+            const uint32_t np = part == 0 ? 1u : parts;
+            const int grid = (int)std::min<int64_t>(((int64_t)cnt * np + per_block - 1) / per_block,
+                                                    (int64_t)num_sms * 8);
+            BEEP_TRY(launch_small<false>(pl.dend, group, grid, s, d_pair, d_items + (part ? tiny : 0), cnt, np,
+                                         nullptr));
+        }
+        big = d_items + tier_n[0] + tier_n[1] + tier_n[2];
+        nbig = tier_n[3];
+        if (nbig == 0)
+            return finish();
+    }
+    int grid = num_sms;
+    if (maxD > smem_maxD)
+        grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms, arena_words / slice_words));
     const size_t pad = (smem_maxD + 4) & ~3u;
     const size_t smem = (3 * pad + (size_t)smem_maxD * ((smem_maxD + 31) / 32)) * 4;
-    unsigned char *scr = static_cast<unsigned char *>(scratch);
     switch (pl.dend) {
 #define BEEP_CASE(DD)                                                                                              \
     case DD:                                                                                                       \
         BEEP_CUDA_TRY(cudaFuncSetAttribute(k_noalloc_count<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
                                            (int)smem));                                                            \
-        k_noalloc_count<DD><<<grid, 512, smem, s>>>(rp, col, n, pl, min_deg, scr, slice_words, smem_maxD);          \
+        k_noalloc_count<DD><<<grid, 512, smem, s>>>(rp, col, n, pl, min_deg, scr, slices, slice_words, smem_maxD,   \
+                                                    big, nbig);                                                    \
         break;
         BEEP_CASE(3)
         BEEP_CASE(4)
@@ -5267,13 +5444,5 @@ extern "C" beep_status beep_count_noalloc(int device, void *cuda_stream, int64_t
         return fail(BEEP_ERR_UNSUPPORTED, "depth out of range");
     }
     BEEP_CUDA_TRY(cudaGetLastError());
-    unsigned long long c[2] = {0, 0}; // count, overflow flag
-    BEEP_CUDA_TRY(cudaMemcpyAsync(c, &ctrl->count, sizeof(c), cudaMemcpyDeviceToHost, s));
-    BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-    if (c[1]) {
-        *out_count = BEEP_COUNT_OVERFLOW;
-        return fail(BEEP_ERR_OVERFLOW, "beep_count_noalloc: the count is at least BEEP_COUNT_LIMIT (2^64 - 2^52)");
-    }
-    *out_count = c[0];
-    return BEEP_OK;
+    return finish();
 }
