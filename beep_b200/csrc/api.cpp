@@ -5,6 +5,8 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include <omp.h>
+
 #include "internal.h"
 
 namespace beep {
@@ -41,11 +43,73 @@ beep_status bind(beep_ctx *ctx) {
 template <typename T> beep_status upload(Ctx *ctx, DevBuf &dst, const T *src, size_t count) {
     BEEP_TRY(ctx->grow(dst, std::max<size_t>(count, 1) * sizeof(T)));
     if (count)
-        BEEP_CUDA_TRY(cudaMemcpyAsync(dst.ptr, src, count * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
+        BEEP_TRY(staged_copy(ctx, dst.ptr, const_cast<T *>(src), count * sizeof(T), true));
     return BEEP_OK;
 }
 
+void parallel_memcpy(void *dst, const void *src, size_t bytes) {
+    constexpr int64_t kSlice = 256 << 10;
+    const int64_t n = ((int64_t)bytes + kSlice - 1) / kSlice;
+    const int threads = (int)std::min<int64_t>({n, 8, (int64_t)omp_get_num_procs()});
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int64_t i = 0; i < n; ++i)
+        std::memcpy(static_cast<char *>(dst) + i * kSlice, static_cast<const char *>(src) + i * kSlice,
+                    std::min<size_t>(kSlice, bytes - (size_t)(i * kSlice)));
+}
+
 } // namespace
+
+beep_status staged_copy(Ctx *ctx, void *dev, void *host, size_t bytes, bool to_device) {
+    cudaStream_t s = ctx->stream;
+    const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    bool staged = bytes >= ((size_t)1 << 20);
+    if (staged) {
+        cudaPointerAttributes at;
+        staged = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+    }
+    for (int i = 0; i < 2 && staged; ++i) {
+        if (!ctx->stage[i] && cudaMallocHost(&ctx->stage[i], Ctx::kStageBytes) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->stage[i] = nullptr;
+            staged = false; // no pinned memory: the driver's own staging
+        }
+        if (staged && !ctx->stage_ev[i])
+            BEEP_CUDA_TRY(cudaEventCreateWithFlags(&ctx->stage_ev[i], cudaEventDisableTiming));
+    }
+    if (!staged) {
+        BEEP_CUDA_TRY(to_device ? cudaMemcpyAsync(dev, host, bytes, kind, s) : cudaMemcpyAsync(host, dev, bytes, kind, s));
+        if (!to_device)
+            BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+        return BEEP_OK;
+    }
+    char *h = static_cast<char *>(host), *d = static_cast<char *>(dev);
+    const size_t nch = (bytes + Ctx::kStageBytes - 1) / Ctx::kStageBytes;
+    auto len = [&](size_t c) { return std::min(Ctx::kStageBytes, bytes - c * Ctx::kStageBytes); };
+    if (to_device) {
+        for (size_t c = 0; c < nch; ++c) {
+            const int b = (int)(c & 1);
+            BEEP_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[b])); // the chunk's last transfer
+            parallel_memcpy(ctx->stage[b], h + c * Ctx::kStageBytes, len(c));
+            BEEP_CUDA_TRY(cudaMemcpyAsync(d + c * Ctx::kStageBytes, ctx->stage[b], len(c), kind, s));
+            BEEP_CUDA_TRY(cudaEventRecord(ctx->stage_ev[b], s));
+        }
+        return BEEP_OK;
+    }
+    for (size_t c = 0; c <= nch; ++c) {
+        if (c < nch) { // a chunk is free here: copies to the host drain before the call returns
+            const int b = (int)(c & 1);
+            BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->stage[b], d + c * Ctx::kStageBytes, len(c), kind, s));
+            BEEP_CUDA_TRY(cudaEventRecord(ctx->stage_ev[b], s));
+        }
+        if (c > 0) {
+            const int b = (int)((c - 1) & 1);
+            BEEP_CUDA_TRY(cudaEventSynchronize(ctx->stage_ev[b]));
+            parallel_memcpy(h + (c - 1) * Ctx::kStageBytes, ctx->stage[b], len(c - 1));
+        }
+    }
+    return BEEP_OK;
+}
 } // namespace beep
 
 namespace beep {
@@ -148,7 +212,7 @@ beep_status beep_ctx_create(int device, void *stream, beep_ctx **out) {
         }
     }
     if (e == cudaSuccess)
-        e = cudaMallocHost(&c->impl.h_pinned, 64);
+        e = cudaMallocHost(&c->impl.h_pinned, Ctx::kPinnedBytes);
     if (e == cudaSuccess) {
         // per-call buffers come from a pool of this context that keeps its memory
         cudaMemPoolProps props;
@@ -182,6 +246,12 @@ void ctx_free(beep_ctx *ctx) {
         cudaFreeHost(ctx->impl.h_pinned);
     if (ctx->impl.h_results)
         cudaFreeHost(ctx->impl.h_results);
+    for (int i = 0; i < 2; ++i) {
+        if (ctx->impl.stage[i])
+            cudaFreeHost(ctx->impl.stage[i]);
+        if (ctx->impl.stage_ev[i])
+            cudaEventDestroy(ctx->impl.stage_ev[i]);
+    }
     ctx->impl.release_side();
     if (ctx->impl.pool)
         cudaMemPoolDestroy(ctx->impl.pool);
@@ -317,11 +387,10 @@ beep_status beep_graph_csr(const beep_graph *g, int32_t *row_ptr, int32_t *col_i
     if (!g || !row_ptr || (g->impl.m > 0 && !col_ind))
         return fail(BEEP_ERR_INVALID_ARG, "beep_graph_csr: bad arguments");
     BEEP_TRY(bind(g->ctx));
-    cudaStream_t s = g->ctx->impl.stream;
-    BEEP_CUDA_TRY(cudaMemcpyAsync(row_ptr, g->impl.row_ptr.ptr, (size_t)(g->impl.n + 1) * 4, cudaMemcpyDeviceToHost, s));
+    Ctx *ctx = &g->ctx->impl;
+    BEEP_TRY(staged_copy(ctx, g->impl.row_ptr.ptr, row_ptr, (size_t)(g->impl.n + 1) * 4, false));
     if (g->impl.m > 0)
-        BEEP_CUDA_TRY(cudaMemcpyAsync(col_ind, g->impl.col.ptr, (size_t)g->impl.m * 4, cudaMemcpyDeviceToHost, s));
-    BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+        BEEP_TRY(staged_copy(ctx, g->impl.col.ptr, col_ind, (size_t)g->impl.m * 4, false));
     return BEEP_OK;
 }
 
@@ -468,7 +537,7 @@ beep_status beep_enumerate(beep_ctx *ctx, beep_graph *g, const beep_query *q, ui
     BEEP_TRY(compile_plan(q->impl.qn, q->impl.row_ptr, q->impl.col, BEEP_MODE_SGM, &p));
     const size_t K = (size_t)p.info.K;
     DevBuf dout;
-    BEEP_TRY(dout.reserve(std::max<uint64_t>(k, 1) * K * 4));
+    BEEP_TRY(ctx->impl.grow(dout, std::max<uint64_t>(k, 1) * K * 4));
     EnumRequest er;
     er.k = k;
     er.d_out = dout.as<int32_t>();
@@ -494,8 +563,9 @@ beep_status beep_enumerate(beep_ctx *ctx, beep_graph *g, const beep_query *q, ui
     }
     const uint64_t got = std::min<uint64_t>(k, st.count);
     if (got)
-        BEEP_CUDA_TRY(cudaMemcpyAsync(out_tuples, dout.ptr, got * K * 4, cudaMemcpyDeviceToHost, ctx->impl.stream));
-    BEEP_CUDA_TRY(cudaStreamSynchronize(ctx->impl.stream));
+        BEEP_TRY(staged_copy(&ctx->impl, dout.ptr, out_tuples, got * K * 4, false));
+    else
+        BEEP_CUDA_TRY(cudaStreamSynchronize(ctx->impl.stream));
     *n_out = got;
     if (total_count)
         *total_count = st.count;

@@ -4014,12 +4014,14 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         BEEP_TRY(lp->alloc(all_items, N));
         k_list_offsets<<<1, 1024, 0, s>>>(d_misc, cfg.tiny_max);
         BEEP_CUDA_TRY(cudaGetLastError());
-        BEEP_CUDA_TRY(cudaMemcpyAsync(h_misc, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
+        static_assert(sizeof(h_misc) <= Ctx::kPinnedBytes, "the pinned mirror");
+        BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, d_misc, sizeof(h_misc), cudaMemcpyDeviceToHost, s));
         const int gf = std::max(1, (int)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->num_sms * 16));
         k_list_fill<<<gf, 256, 0, s>>>(lp->d_pairs, lp->d_offs, np, N, lp->d_tier, d_dom, d_misc, all_items);
         BEEP_CUDA_TRY(cudaGetLastError());
         st.kernel_launches += 2;
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+        std::memcpy(h_misc, ctx->h_pinned, sizeof(h_misc));
     }
     if (!sups.empty())
         lp->d_sup_tiers = d_misc + kMiscSup; // read back with the counts

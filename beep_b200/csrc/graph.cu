@@ -117,39 +117,70 @@ __global__ void k_check_chunks(const uint32_t *__restrict__ rp, const uint32_t *
         atomicOr(bad, flag);
 }
 
-__global__ void k_csr_keys(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ col, int64_t n,
-                           uint64_t *keys) {
+// Edge keys (src << bits | dst), ids below 2^bits; self loops become the
+// largest value of 2 bits bits (itself a loop, so no edge has it), which sorts
+// last. flags[0] |= 1: a loop, 2: an id that does not fit.
+__global__ void k_csr_keys(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ col, int64_t n, int bits,
+                           uint64_t *keys, unsigned *flags) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const uint64_t loop = ~0ull >> (64 - 2 * bits);
+    unsigned f = 0;
     for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const uint32_t b = rp[v], e = rp[v + 1];
         for (uint32_t i = b + lane; i < e; i += 32) {
             const uint32_t w = col[i];
-            keys[i] = (w == (uint32_t)v) ? ~0ull : (((uint64_t)v << 32) | w);
+            const bool lp = w == (uint32_t)v, bad = (int64_t)w >= n;
+            f |= (lp ? 1u : 0u) | (bad ? 2u : 0u);
+            keys[i] = lp || bad ? loop : (((uint64_t)v << bits) | w);
         }
     }
+    f = __reduce_or_sync(kFull, f);
+    if (lane == 0 && f)
+        atomicOr(flags, f);
 }
 
-__global__ void k_edge_keys(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, int64_t ne,
-                            uint64_t *keys, unsigned *max_id) {
+__global__ void k_max_id(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, int64_t ne,
+                         unsigned *max_id) {
     uint32_t mx = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t s = src[i], d = dst[i];
-        keys[i] = (s == d) ? ~0ull : (((uint64_t)s << 32) | d);
-        mx = max(mx, max(s, d));
-    }
-    for (int o = 16; o > 0; o >>= 1)
-        mx = max(mx, __shfl_xor_sync(kFull, mx, o));
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (int64_t)gridDim.x * blockDim.x)
+        mx = max(mx, max(src[i], dst[i]));
+    mx = __reduce_max_sync(kFull, mx);
     if ((threadIdx.x & 31) == 0)
         atomicMax(max_id, mx);
 }
 
-// Keys are sorted and unique; the self-loop sentinel (~0) sorts last.
-__global__ void k_keys_to_coo(const uint64_t *__restrict__ keys, int64_t m, uint32_t *col, uint32_t *deg) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = keys[i];
-        col[i] = (uint32_t)k;
-        atomicAdd(&deg[k >> 32], 1u);
+__global__ void k_edge_keys(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, int64_t ne, int bits,
+                            uint64_t *keys, unsigned *flags) {
+    const uint64_t loop = ~0ull >> (64 - 2 * bits);
+    unsigned f = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t s = src[i], d = dst[i];
+        f |= s == d ? 1u : 0u;
+        keys[i] = s == d ? loop : (((uint64_t)s << bits) | d);
+    }
+    f = __reduce_or_sync(kFull, f);
+    if ((threadIdx.x & 31) == 0 && f)
+        atomicOr(flags, f);
+}
+
+// Sorted unique keys -> columns, and row pointers by a binary search per vertex.
+__global__ void k_keys_to_csr(const uint64_t *__restrict__ keys, int64_t m, int64_t n, int bits, uint32_t *col,
+                              uint32_t *rp) {
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    const uint64_t low = (1ull << bits) - 1ull;
+    for (int64_t i = t0; i < m; i += nt)
+        col[i] = (uint32_t)(keys[i] & low);
+    for (int64_t v = t0; v <= n; v += nt) {
+        int64_t lo = 0, hi = m;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if ((int64_t)(keys[mid] >> bits) < v)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        rp[v] = (uint32_t)lo;
     }
 }
 
@@ -174,10 +205,18 @@ __global__ void k_degree_stats(const uint32_t *__restrict__ rp, int64_t n, unsig
 
 // ---- peeling --------------------------------------------------------------
 
-__global__ void k_peel_init(const uint32_t *__restrict__ rp, int64_t n, uint32_t *deg, uint8_t *alive) {
+// Everything a view build starts from: degrees, live marks, no ranks, empty
+// row cursors, and `words` zeroed words at zero[].
+__global__ void k_view_init(const uint32_t *__restrict__ rp, int64_t n, uint32_t *deg, uint8_t *alive, uint32_t *rank,
+                            uint32_t *cur, uint32_t *zero, uint32_t words) {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x)
+            zero[i] = 0;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         deg[v] = rp[v + 1] - rp[v];
         alive[v] = 1;
+        rank[v] = 0xffffffffu;
+        cur[v] = 0;
     }
 }
 
@@ -312,6 +351,8 @@ __global__ void k_rank(const uint32_t *__restrict__ sorted_ids, int64_t n_alive,
         rank[v] = (uint32_t)i;
         new_deg[i] = deg[v];
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        new_deg[n_alive] = 0; // the scan's last entry
 }
 
 // ---- relabelled rows --------------------------------------------------------
@@ -661,15 +702,46 @@ struct Carve {
     }
 };
 
-// Sorted unique u64 keys -> CSR in g.
-beep_status keys_to_graph(Ctx *ctx, Graph *g, uint64_t *keys, uint64_t *keys_tmp, int64_t nkeys, int64_t n) {
+// Scratch of one build from the context's pool, freed in the stream's order.
+struct PoolBuf {
+    Ctx *ctx;
+    void *ptr = nullptr;
+    explicit PoolBuf(Ctx *c) : ctx(c) {}
+    PoolBuf(const PoolBuf &) = delete;
+    PoolBuf &operator=(const PoolBuf &) = delete;
+    ~PoolBuf() {
+        if (ptr)
+            cudaFreeAsync(ptr, ctx->stream);
+    }
+    beep_status reserve(size_t bytes) {
+        cudaError_t e = cudaMallocFromPoolAsync(&ptr, std::max<size_t>(bytes, 16), ctx->pool, ctx->stream);
+        if (e != cudaSuccess) {
+            ptr = nullptr;
+            return fail(BEEP_ERR_OUT_OF_MEMORY, "device pool allocation of " + std::to_string(bytes) +
+                                                    " bytes: " + cudaGetErrorString(e));
+        }
+        return BEEP_OK;
+    }
+};
+
+// bits of an id below n (at least 1)
+inline int id_bits(int64_t n) {
+    int b = 1;
+    while (b < 32 && ((int64_t)1 << b) < n)
+        ++b;
+    return b;
+}
+
+// u64 keys of 2 bits bits -> CSR in g: sorted over those bits only (5 radix
+// passes instead of 8 at 2^18 vertices), made unique, split at a binary search
+// per vertex. flags: k_csr_keys / k_edge_keys' word.
+beep_status keys_to_graph(Ctx *ctx, Graph *g, uint64_t *keys, uint64_t *keys_tmp, int64_t nkeys, int64_t n, int bits,
+                          const unsigned *flags) {
     cudaStream_t s = ctx->stream;
-    // sort
-    int end_bit = 64;
     size_t tb = 0;
-    BEEP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys_tmp, nkeys, 0, end_bit, s));
+    BEEP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys_tmp, nkeys, 0, 2 * bits, s));
     BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
-    BEEP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(ctx->scratch.ptr, tb, keys, keys_tmp, nkeys, 0, end_bit, s));
+    BEEP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(ctx->scratch.ptr, tb, keys, keys_tmp, nkeys, 0, 2 * bits, s));
     // unique
     BEEP_TRY(ctx->grow(ctx->counter, 64));
     unsigned long long *d_num = ctx->counter.as<unsigned long long>();
@@ -677,62 +749,61 @@ beep_status keys_to_graph(Ctx *ctx, Graph *g, uint64_t *keys, uint64_t *keys_tmp
     BEEP_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, tb, keys_tmp, keys, d_num, nkeys, s));
     BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
     BEEP_CUDA_TRY(cub::DeviceSelect::Unique(ctx->scratch.ptr, tb, keys_tmp, keys, d_num, nkeys, s));
-    unsigned long long h_num = 0;
-    BEEP_CUDA_TRY(cudaMemcpyAsync(&h_num, d_num, sizeof(h_num), cudaMemcpyDeviceToHost, s));
+    volatile unsigned long long *h = ctx->h_pinned;
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, d_num, 8, cudaMemcpyDeviceToHost, s));
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned + 1, flags, 4, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-    int64_t m = (int64_t)h_num;
-    if (m > 0) {
-        uint64_t last = 0;
-        BEEP_CUDA_TRY(cudaMemcpyAsync(&last, keys + (m - 1), sizeof(last), cudaMemcpyDeviceToHost, s));
-        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-        if (last == ~0ull)
-            --m; // self-loop sentinel
-    }
+    const unsigned f = (unsigned)h[1];
+    if (f & 2u)
+        return fail(BEEP_ERR_INVALID_ARG, "column index >= n");
+    const int64_t m = (int64_t)h[0] - (f & 1u ? 1 : 0); // without the loops' key
     if (m >= (int64_t)0xffffffffll)
         return fail(BEEP_ERR_UNSUPPORTED, "graph has 2^32 or more directed edges");
     g->n = n;
     g->m = m;
     BEEP_TRY(ctx->grow(g->row_ptr, (size_t)(n + 1) * 4));
     BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
-    uint32_t *deg = g->row_ptr.as<uint32_t>();
-    BEEP_CUDA_TRY(cudaMemsetAsync(deg, 0, (size_t)(n + 1) * 4, s));
-    if (m > 0) {
-        k_keys_to_coo<<<grid_for(m, 256, ctx->num_sms), 256, 0, s>>>(keys, m, g->col.as<uint32_t>(), deg);
-        ++ctx->launches;
-    }
+    k_keys_to_csr<<<grid_for(std::max(m, n + 1), 256, ctx->num_sms), 256, 0, s>>>(keys, m, n, bits,
+                                                                                  g->col.as<uint32_t>(),
+                                                                                  g->row_ptr.as<uint32_t>());
+    ++ctx->launches;
     BEEP_CUDA_TRY(cudaGetLastError());
-    tb = 0;
-    BEEP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, deg, deg, n + 1, s));
-    BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
-    BEEP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(ctx->scratch.ptr, tb, deg, deg, n + 1, s));
     return BEEP_OK;
+}
+
+// Degree statistics into the context's counter words: sum of squares, maximum.
+beep_status launch_stats(Ctx *ctx, const uint32_t *rp, int64_t n) {
+    cudaStream_t s = ctx->stream;
+    unsigned long long *d = ctx->counter.as<unsigned long long>();
+    if (n > 0)
+        k_degree_stats<<<grid_for(n, 256, ctx->num_sms), 256, 0, s>>>(rp, n, d, reinterpret_cast<unsigned *>(d + 1));
+    BEEP_CUDA_TRY(cudaGetLastError());
+    return BEEP_OK;
+}
+
+// cutoff = ceil(mean + 6 sd) over all n vertices (include/utils.cuh:241-260)
+void set_stats(Graph *g, unsigned long long sumsq, uint32_t maxdeg) {
+    g->max_degree = (int64_t)maxdeg;
+    g->cutoff = 0;
+    if (g->n > 0) {
+        const double n = (double)g->n;
+        const double mean = (double)g->m / n;
+        double var = (double)sumsq / n - mean * mean;
+        if (var < 0)
+            var = 0;
+        g->cutoff = (uint32_t)std::ceil(mean + 6.0 * std::sqrt(var));
+    }
+    g->views.clear();
 }
 
 beep_status finish_graph(Ctx *ctx, Graph *g) {
     cudaStream_t s = ctx->stream;
     BEEP_TRY(ctx->grow(ctx->counter, 64));
-    unsigned long long *d = ctx->counter.as<unsigned long long>();
-    BEEP_CUDA_TRY(cudaMemsetAsync(d, 0, 16, s));
-    if (g->n > 0)
-        k_degree_stats<<<grid_for(g->n, 256, ctx->num_sms), 256, 0, s>>>(g->row_ptr.as<uint32_t>(), g->n, d,
-                                                                         reinterpret_cast<unsigned *>(d + 1));
-    BEEP_CUDA_TRY(cudaGetLastError());
-    unsigned long long h[2] = {0, 0};
-    BEEP_CUDA_TRY(cudaMemcpyAsync(h, d, 16, cudaMemcpyDeviceToHost, s));
+    BEEP_CUDA_TRY(cudaMemsetAsync(ctx->counter.ptr, 0, 16, s));
+    BEEP_TRY(launch_stats(ctx, g->row_ptr.as<uint32_t>(), g->n));
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, ctx->counter.ptr, 16, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-    g->max_degree = (int64_t)(uint32_t)h[1];
-    // cutoff = ceil(mean + 6 sd) over all n vertices (include/utils.cuh:241-260)
-    if (g->n > 0) {
-        const double n = (double)g->n;
-        const double mean = (double)g->m / n;
-        double var = (double)h[0] / n - mean * mean;
-        if (var < 0)
-            var = 0;
-        g->cutoff = (uint32_t)std::ceil(mean + 6.0 * std::sqrt(var));
-    } else {
-        g->cutoff = 0;
-    }
-    g->views.clear();
+    set_stats(g, ctx->h_pinned[0], (uint32_t)ctx->h_pinned[1]);
     return BEEP_OK;
 }
 
@@ -744,11 +815,14 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
     if (n < 0 || m < 0 || n >= (int64_t)0xffffffffll || m >= (int64_t)0xffffffffll)
         return fail(BEEP_ERR_INVALID_ARG, "graph size out of range");
     PhaseTrace tr("graph", s);
-    // Fast path: rows already strictly increasing with no self loop.
+    // Fast path: rows already strictly increasing with no self loop. The check,
+    // the degree statistics (which read only the row pointers) and the last
+    // row pointer come back in one read: counter words [0, 16) statistics,
+    // [32, 36) flags, [36, 40) chunks.
     BEEP_TRY(ctx->grow(ctx->counter, 64));
     unsigned *d_bad = reinterpret_cast<unsigned *>(ctx->counter.as<char>() + 32);
     unsigned *d_nchunks = reinterpret_cast<unsigned *>(ctx->counter.as<char>() + 36);
-    BEEP_CUDA_TRY(cudaMemsetAsync(d_bad, 0, 8, s));
+    BEEP_CUDA_TRY(cudaMemsetAsync(ctx->counter.ptr, 0, 64, s));
     if (n > 0) {
         BEEP_TRY(ctx->grow(ctx->scratch2, chunk_capacity(n, m) * sizeof(RowChunk)));
         RowChunk *chunks = ctx->scratch2.as<RowChunk>();
@@ -759,53 +833,47 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
         ctx->launches += 2;
     }
     BEEP_CUDA_TRY(cudaGetLastError());
-    unsigned h_bad = 0;
-    uint32_t h_m_end = 0;
-    BEEP_CUDA_TRY(cudaMemcpyAsync(&h_bad, d_bad, 4, cudaMemcpyDeviceToHost, s));
-    BEEP_CUDA_TRY(cudaMemcpyAsync(&h_m_end, d_rp + n, 4, cudaMemcpyDeviceToHost, s));
+    BEEP_TRY(launch_stats(ctx, d_rp, n));
+    // the graph's own copy, made before the check's result is known
+    BEEP_TRY(ctx->grow(g->row_ptr, (size_t)(n + 1) * 4));
+    BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
+    if (g->row_ptr.ptr != (const void *)d_rp)
+        BEEP_CUDA_TRY(cudaMemcpyAsync(g->row_ptr.ptr, d_rp, (size_t)(n + 1) * 4, cudaMemcpyDeviceToDevice, s));
+    if (m > 0 && g->col.ptr != (const void *)d_col)
+        BEEP_CUDA_TRY(cudaMemcpyAsync(g->col.ptr, d_col, (size_t)m * 4, cudaMemcpyDeviceToDevice, s));
+    const unsigned *h32 = reinterpret_cast<const unsigned *>(ctx->h_pinned);
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, ctx->counter.ptr, 40, cudaMemcpyDeviceToHost, s));
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned + 6, d_rp + n, 4, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+    const unsigned h_bad = h32[8];
+    const uint32_t h_m_end = h32[12];
     if ((int64_t)h_m_end != m)
         return fail(BEEP_ERR_INVALID_ARG, "row_ptr[n] != m");
     if (h_bad & 2u)
         return fail(BEEP_ERR_INVALID_ARG, "row_ptr is not non-decreasing within [0, m]");
     tr.mark("check");
     if (!h_bad) {
+        const unsigned long long sumsq = ctx->h_pinned[0];
+        const uint32_t maxdeg = (uint32_t)ctx->h_pinned[1];
         g->n = n;
         g->m = m;
-        BEEP_TRY(ctx->grow(g->row_ptr, (size_t)(n + 1) * 4));
-        BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
-        if (g->row_ptr.ptr != (const void *)d_rp)
-            BEEP_CUDA_TRY(cudaMemcpyAsync(g->row_ptr.ptr, d_rp, (size_t)(n + 1) * 4, cudaMemcpyDeviceToDevice, s));
-        if (m > 0 && g->col.ptr != (const void *)d_col)
-            BEEP_CUDA_TRY(cudaMemcpyAsync(g->col.ptr, d_col, (size_t)m * 4, cudaMemcpyDeviceToDevice, s));
-        tr.mark("copy");
-        beep_status st = finish_graph(ctx, g);
-        tr.mark("stats");
-        return st;
+        set_stats(g, sumsq, maxdeg);
+        return BEEP_OK;
     }
     // Slow path: sort + unique packed (src, dst) keys. Out-of-range ids fail.
-    DevBuf keys, keys2;
+    PoolBuf keys(ctx), keys2(ctx);
     BEEP_TRY(keys.reserve((size_t)(m > 0 ? m : 1) * 8));
     BEEP_TRY(keys2.reserve((size_t)(m > 0 ? m : 1) * 8));
+    const int bits = id_bits(n);
+    unsigned *d_flags = reinterpret_cast<unsigned *>(ctx->counter.as<char>() + 40);
     if (n > 0) {
-        k_csr_keys<<<grid_for(n * 32, 256, ctx->num_sms), 256, 0, s>>>(d_rp, d_col, n, keys.as<uint64_t>());
+        k_csr_keys<<<grid_for(n * 32, 256, ctx->num_sms), 256, 0, s>>>(d_rp, d_col, n, bits,
+                                                                        static_cast<uint64_t *>(keys.ptr), d_flags);
         ++ctx->launches;
     }
     BEEP_CUDA_TRY(cudaGetLastError());
-    BEEP_TRY(keys_to_graph(ctx, g, keys.as<uint64_t>(), keys2.as<uint64_t>(), m, n));
-    // validate ids
-    if (g->m > 0) {
-        uint32_t maxc = 0;
-        size_t tb = 0;
-        unsigned *d_max = reinterpret_cast<unsigned *>(ctx->counter.as<char>() + 40);
-        BEEP_CUDA_TRY(cub::DeviceReduce::Max(nullptr, tb, g->col.as<uint32_t>(), d_max, g->m, s));
-        BEEP_TRY(ctx->grow(ctx->scratch, tb + 1024));
-        BEEP_CUDA_TRY(cub::DeviceReduce::Max(ctx->scratch.ptr, tb, g->col.as<uint32_t>(), d_max, g->m, s));
-        BEEP_CUDA_TRY(cudaMemcpyAsync(&maxc, d_max, 4, cudaMemcpyDeviceToHost, s));
-        BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-        if ((int64_t)maxc >= n)
-            return fail(BEEP_ERR_INVALID_ARG, "column index >= n");
-    }
+    BEEP_TRY(keys_to_graph(ctx, g, static_cast<uint64_t *>(keys.ptr), static_cast<uint64_t *>(keys2.ptr), m, n, bits,
+                           d_flags));
     return finish_graph(ctx, g);
 }
 
@@ -814,22 +882,30 @@ beep_status graph_build_from_device_edges(Ctx *ctx, Graph *g, int64_t ne, const 
     cudaStream_t s = ctx->stream;
     if (ne < 0 || ne >= (int64_t)0xffffffffll)
         return fail(BEEP_ERR_INVALID_ARG, "edge count out of range");
-    DevBuf keys, keys2;
+    PoolBuf keys(ctx), keys2(ctx);
     BEEP_TRY(keys.reserve((size_t)(ne > 0 ? ne : 1) * 8));
     BEEP_TRY(keys2.reserve((size_t)(ne > 0 ? ne : 1) * 8));
     BEEP_TRY(ctx->grow(ctx->counter, 64));
     unsigned *d_max = reinterpret_cast<unsigned *>(ctx->counter.as<char>() + 48);
-    BEEP_CUDA_TRY(cudaMemsetAsync(d_max, 0, 4, s));
+    unsigned *d_flags = d_max + 1;
+    BEEP_CUDA_TRY(cudaMemsetAsync(d_max, 0, 8, s));
     if (ne > 0) {
-        k_edge_keys<<<grid_for(ne, 256, ctx->num_sms), 256, 0, s>>>(d_src, d_dst, ne, keys.as<uint64_t>(), d_max);
+        k_max_id<<<grid_for(ne, 256, ctx->num_sms), 256, 0, s>>>(d_src, d_dst, ne, d_max);
         ++ctx->launches;
     }
     BEEP_CUDA_TRY(cudaGetLastError());
-    unsigned h_max = 0;
-    BEEP_CUDA_TRY(cudaMemcpyAsync(&h_max, d_max, 4, cudaMemcpyDeviceToHost, s));
+    BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, d_max, 4, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaStreamSynchronize(s));
-    int64_t n = ne > 0 ? (int64_t)h_max + 1 : 0;
-    BEEP_TRY(keys_to_graph(ctx, g, keys.as<uint64_t>(), keys2.as<uint64_t>(), ne, n));
+    const int64_t n = ne > 0 ? (int64_t)(uint32_t)ctx->h_pinned[0] + 1 : 0;
+    const int bits = id_bits(n);
+    if (ne > 0) {
+        k_edge_keys<<<grid_for(ne, 256, ctx->num_sms), 256, 0, s>>>(d_src, d_dst, ne, bits,
+                                                                    static_cast<uint64_t *>(keys.ptr), d_flags);
+        ++ctx->launches;
+    }
+    BEEP_CUDA_TRY(cudaGetLastError());
+    BEEP_TRY(keys_to_graph(ctx, g, static_cast<uint64_t *>(keys.ptr), static_cast<uint64_t *>(keys2.ptr), ne, n, bits,
+                           d_flags));
     return finish_graph(ctx, g);
 }
 
@@ -845,9 +921,10 @@ beep_status build_view(Ctx *ctx, Graph *g, int32_t min_qdeg, int32_t asc, View *
     const int64_t nn = n > 0 ? n : 1;
     const size_t cap = chunk_capacity(n, m);
     const size_t mm = m > 0 ? (size_t)m : 1;
+    constexpr size_t kZeroWords = 2 * kPeelMaxRounds + kVsWords + 4;
     size_t need = Carve::need({(size_t)nn * 4, (size_t)nn, (size_t)nn * 4, (size_t)nn * 4, (size_t)nn * 4,
-                               (size_t)nn * 4, (size_t)nn * 4, (size_t)nn * 4, mm * 4, cap * sizeof(RowChunk), 16,
-                               (size_t)nn * 4, kPeelMaxRounds * 8, kVsWords * 4, ((size_t)nn + 1) * 4});
+                               (size_t)nn * 4, (size_t)nn * 4, ((size_t)nn + 1) * 4, mm * 4, cap * sizeof(RowChunk),
+                               (size_t)nn * 4, kZeroWords * 4, (size_t)nn * 4, ((size_t)nn + 1) * 4});
     BEEP_TRY(ctx->grow(ctx->scratch2, need));
     Carve cv(ctx->scratch2.ptr);
     uint32_t *deg = cv.take<uint32_t>(nn);
@@ -855,29 +932,29 @@ beep_status build_view(Ctx *ctx, Graph *g, int32_t min_qdeg, int32_t asc, View *
     uint32_t *rank = cv.take<uint32_t>(nn);
     uint32_t *pkey = cv.take<uint32_t>(nn), *pid = cv.take<uint32_t>(nn);
     uint32_t *pkey2 = cv.take<uint32_t>(nn), *pid2 = cv.take<uint32_t>(nn);
-    uint32_t *new_deg = cv.take<uint32_t>(nn);
+    uint32_t *new_deg = cv.take<uint32_t>(nn + 1);
     uint32_t *hub_tmp = cv.take<uint32_t>(mm); // the hub rows' other merge buffer
     RowChunk *chunks = cv.take<RowChunk>(cap);
-    unsigned *d_nchunks = cv.take<unsigned>(4); // [0] chunk count, [1] row sort cursor
     uint32_t *peel_list = cv.take<uint32_t>(nn);
-    unsigned long long *peel_removed = cv.take<unsigned long long>(kPeelMaxRounds);
-    uint32_t *vstat = cv.take<uint32_t>(kVsWords);
+    // words that start at zero: the peel's counts, the class statistics, the
+    // chunk count and the row sort's cursor
+    uint32_t *zero = cv.take<uint32_t>(kZeroWords);
+    unsigned long long *peel_removed = reinterpret_cast<unsigned long long *>(zero);
+    uint32_t *vstat = zero + 2 * kPeelMaxRounds;
+    unsigned *d_nchunks = vstat + kVsWords; // [0] chunk count, [1] row sort cursor
+    uint32_t *cur = cv.take<uint32_t>(nn);  // long rows' fill cursors
     uint32_t *htp = cv.take<uint32_t>((size_t)nn + 1); // first tile of every hub row
     const uint32_t ucap = (uint32_t)std::min<size_t>(cap, 0xffffffffu);
 
     PhaseTrace tr("view", s);
     const int gv = grid_for(n, 256, ctx->num_sms);
-    if (n > 0) {
-        k_peel_init<<<gv, 256, 0, s>>>(rp, n, deg, alive);
-        ++ctx->launches;
-    }
+    k_view_init<<<gv, 256, 0, s>>>(rp, n, deg, alive, rank, cur, zero, (uint32_t)kZeroWords);
+    ++ctx->launches;
     BEEP_CUDA_TRY(cudaGetLastError());
     // Iterated peel, all rounds in one cooperative launch (no host round trip
     // per round).
-    BEEP_CUDA_TRY(cudaMemsetAsync(vstat, 0, kVsWords * 4, s));
     int *d_rounds = reinterpret_cast<int *>(vstat + kVsRounds);
     if (min_qdeg > 1 && n > 0) {
-        BEEP_CUDA_TRY(cudaMemsetAsync(peel_removed, 0, kPeelMaxRounds * 8, s));
         int per_sm = 0;
         BEEP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_fused, 256, 0));
         // two blocks per SM at most: enough threads for these elementwise
@@ -909,7 +986,7 @@ beep_status build_view(Ctx *ctx, Graph *g, int32_t min_qdeg, int32_t asc, View *
     BEEP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(ctx->scratch.ptr, tb, pkey, pkey2, pid, pid2, n, 0, hb, s));
     // rows per class (their sum: the vertices that kept an edge), hub tiles,
     // peel rounds
-    static_assert(kVsWords * 4 <= 64, "the pinned mirror holds 64 bytes");
+    static_assert(kVsWords * 4 <= Ctx::kPinnedBytes, "the pinned mirror");
     uint32_t *hv = reinterpret_cast<uint32_t *>(ctx->h_pinned);
     BEEP_CUDA_TRY(cudaMemcpyAsync(hv, vstat, kVsWords * 4, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaStreamSynchronize(s));
@@ -926,8 +1003,8 @@ beep_status build_view(Ctx *ctx, Graph *g, int32_t min_qdeg, int32_t asc, View *
     BEEP_TRY(ctx->grow(v->row_ptr, (size_t)(na + 1) * 4));
     BEEP_TRY(ctx->grow(v->orig, (size_t)(na > 0 ? na : 1) * 4));
     BEEP_TRY(ctx->grow(v->split, (size_t)(na > 0 ? na : 1) * 4));
-    BEEP_CUDA_TRY(cudaMemsetAsync(rank, 0xff, (size_t)nn * 4, s));
-    BEEP_CUDA_TRY(cudaMemsetAsync(new_deg, 0, (size_t)nn * 4, s));
+    if (na == 0)
+        BEEP_CUDA_TRY(cudaMemsetAsync(new_deg, 0, 4, s));
     if (na > 0) {
         k_rank<<<grid_for(na, 256, ctx->num_sms), 256, 0, s>>>(pid2, na, v->orig.as<uint32_t>(), rank, deg,
                                                                new_deg);
@@ -945,11 +1022,8 @@ beep_status build_view(Ctx *ctx, Graph *g, int32_t min_qdeg, int32_t asc, View *
     BEEP_TRY(ctx->grow(v->col, (size_t)(m > 0 ? m : 1) * 4));
     uint32_t *vcol = v->col.as<uint32_t>();
     if (m > 0 && na > 0) {
-        // new_deg is free after the scan: the long rows' fill cursors
-        BEEP_CUDA_TRY(cudaMemsetAsync(new_deg, 0, (size_t)na * 4, s));
-        BEEP_CUDA_TRY(cudaMemsetAsync(d_nchunks, 0, 8, s));
         k_view_fill<<<gv, 256, 0, s>>>(rp, col, rank, n, nrp, vcol, chunks, d_nchunks, ucap);
-        k_view_fill_chunks<<<ctx->num_sms * 8, 256, 0, s>>>(col, rank, chunks, d_nchunks, ucap, nrp, new_deg, vcol);
+        k_view_fill_chunks<<<ctx->num_sms * 8, 256, 0, s>>>(col, rank, chunks, d_nchunks, ucap, nrp, cur, vcol);
         ctx->launches += 2;
         BEEP_CUDA_TRY(cudaGetLastError());
     }

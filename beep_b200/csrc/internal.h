@@ -236,7 +236,15 @@ struct Ctx {
     DevBuf scratch2;
     DevBuf arena;        // neighbourhood bitmaps of large roots
     DevBuf counter;      // u64 counters
-    unsigned long long *h_pinned = nullptr; // pinned host mirror of small results
+    // pinned host mirror of small results (a copy to pageable memory blocks in
+    // the driver and cannot be queued behind other work)
+    static constexpr size_t kPinnedBytes = 4096;
+    unsigned long long *h_pinned = nullptr;
+    // two pinned chunks through which copies from and to pageable memory are
+    // staged (staged_copy), and the events of their last transfers
+    static constexpr size_t kStageBytes = (size_t)4 << 20;
+    void *stage[2] = {nullptr, nullptr};
+    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     uint64_t launches = 0; // kernels of this library launched on the context
     cudaMemPool_t pool = nullptr; // stream-ordered pool for per-call buffers
     // grow b (a buffer of this context or of an object it builds) from the pool on the context's stream
@@ -291,6 +299,14 @@ struct Ctx {
         return BEEP_OK;
     }
 };
+
+// Copies between the device and host memory of any kind, on ctx->stream.
+// Pageable memory of 1 MB and more goes through the context's pinned chunks,
+// several host threads filling or draining one chunk while the other's
+// transfer runs: the driver's own path moves about 10 GB/s on one thread, and
+// a fresh destination's page faults are taken by all threads. A copy to the
+// host is complete on return.
+beep_status staged_copy(Ctx *ctx, void *dev, void *host, size_t bytes, bool to_device);
 
 // device entry points (device.cu)
 beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m, const uint32_t *d_row_ptr,

@@ -382,7 +382,7 @@ beep_status beep_serve_create(beep_ctx *ctx, const beep_serve_options *opt, beep
             S.reserve = opt->hbm_reserve_bytes;
         S.count_options = opt->count_options & BEEP_OPT_REFERENCE_ROOT_CAP;
     }
-    cudaError_t e = cudaMallocHost(&S.ctx.h_pinned, 64);
+    cudaError_t e = cudaMallocHost(&S.ctx.h_pinned, Ctx::kPinnedBytes);
     // buffers come from the user context's pool (the server holds a
     // reference to that context, so the pool outlives everything built here,
     // including the views it caches in the graphs)
