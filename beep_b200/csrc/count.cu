@@ -1473,8 +1473,28 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
         __syncwarp(gmask);
     }
     cnt = group_sum<G>(cnt, gmask);
-    if (glane == 0)
-        flush_count(pr.count, cnt);
+    // the block's groups mostly end on the same pair: one atomic for a run of
+    // equal counters (a group each was up to 38,000 atomics on one address)
+    __shared__ unsigned long long s_cnt[NG], *s_ptr[NG];
+    if (glane == 0) {
+        s_cnt[gid] = cnt;
+        s_ptr[gid] = cur == 0xffffffffu ? nullptr : pr.count;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long *ptr = nullptr, acc = 0;
+        for (int i = 0; i < NG; ++i) {
+            if (s_ptr[i] != ptr) {
+                if (ptr)
+                    flush_count(ptr, acc);
+                ptr = s_ptr[i];
+                acc = 0;
+            }
+            acc = sat_add(acc, s_cnt[i]);
+        }
+        if (ptr)
+            flush_count(ptr, acc);
+    }
     if (lane == 0)
         record_exit(exit_t);
 }
@@ -1976,6 +1996,7 @@ constexpr uint32_t kLargeSmemA = 48 * 1024; // domain entries staged in shared m
 // Rows of at least kListMinW words also get non-zero-word lists of
 // W / 8 entries (rounded down to 32): 1 + W / 8 more words a row, under 13%.
 constexpr uint32_t kListMinW = 256;
+constexpr uint32_t kC4StripMaxW = 512; // widest rows counted in strips (4-wheel, statistics)
 __host__ __device__ __forceinline__ uint32_t list_cap(uint32_t W) { return W >= kListMinW ? (W / 8) & ~31u : 0u; }
 
 // Arena words of one large root: rows [rlo, D) of W = ceil(D / 32) words,
@@ -2068,7 +2089,8 @@ __global__ void __launch_bounds__(256) k_large_lists(const PairDev *__restrict__
         uint32_t beg, D, j0;
         pair_domain(pr, item_root(it), beg, D, j0);
         const uint32_t W = (D + 31) >> 5, cap = list_cap(W);
-        if (cap == 0)
+        const DevPlan &pl = pairs[item_pair(it)].pl;
+        if (cap == 0 || ((pl.wheel4 || pl.nbhd) && W <= kC4StripMaxW)) // strips read no lists
             continue;
         const uint32_t rlo = pair_rlo(pr, D, j0);
         const uint32_t *rows = arena + bt.off[b];
@@ -2277,7 +2299,6 @@ __device__ __forceinline__ void wheel4_task(const uint32_t *__restrict__ bm, con
 // below a. Strips keep the tasks of a hub's neighbourhood short: its largest a
 // have thousands of b and a dozen strips.
 // Task t of a root: strip s holds the a in [1024 s, D), largest first.
-constexpr uint32_t kC4StripMaxW = 512;
 __host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D) {
     const uint32_t S = (D + 1023) / 1024;
     return S * D - 512 * S * (S - 1);
@@ -2789,9 +2810,10 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
         const uint32_t *deg = rows + nb_deg_offset(D, 0);
         const unsigned long long E = *reinterpret_cast<const unsigned long long *>(rows + nb_edges_offset(D, 0)) / 2;
         if (nbhd_strips(form, D)) {
-            // the forms' per-edge terms by bit-sliced counters; forms without
-            // them (wedge, two edges) and wider rows take nbhd_task
-            const uint32_t S = (D + 1023) / 1024, ti = t - bt.tstart[b], st = ti % S, u = j0 + ti / S;
+            // the forms' per-edge terms by bit-sliced counters, the largest
+            // (and most connected) u first; forms without them (wedge, two
+            // edges) and wider rows take nbhd_task
+            const uint32_t S = (D + 1023) / 1024, ti = t - bt.tstart[b], st = ti % S, u = D - 1 - ti / S;
             uint16_t *ib = s_ib[threadIdx.x >> 5];
             const unsigned long long du = deg[u], rest = D - 3;
             switch (form) {
@@ -2829,7 +2851,7 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
 
 // ---------------------------------------------------------------------------
 // queries without a central vertex: list walker. The neighbourhood bitmaps
-// above need every position adjacent to the root; here a thread takes one
+// above need every position adjacent to the root; here eight lanes take one
 // (root, level-1 vertex) task and walks the rest of the matching order over
 // the view's sorted neighbour lists: a position's candidates are the entries
 // of the shortest list among its back-edge positions (the root included)
@@ -2873,8 +2895,14 @@ __device__ __forceinline__ void gen_emit(const GenRegs &g, const uint32_t (&x)[k
     t[g.order[P]] = (int32_t)g.v.orig[w];
 }
 
+// Lanes per (root, level-1 vertex) task: each takes every kGenLanes-th
+// candidate of level 2. A walk is a chain of dependent loads, and a lane per
+// task left the chain of a task's whole subtree on one lane and (ER graph of
+// 20,011 vertices) fewer warps than the GPU holds.
+constexpr uint32_t kGenLanes = 8;
+
 template <int P, int DEND, bool ENUM>
-__device__ void gen_walk(const GenRegs &g, uint32_t (&x)[kMaxQ], unsigned long long &cnt) {
+__device__ void gen_walk(const GenRegs &g, uint32_t (&x)[kMaxQ], unsigned long long &cnt, uint32_t sub) {
     if constexpr (P >= DEND) {
         return;
     } else {
@@ -2899,7 +2927,9 @@ __device__ void gen_walk(const GenRegs &g, uint32_t (&x)[kMaxQ], unsigned long l
                     de = e;
                 }
             }
-        for (uint32_t k = lower_bound_g(g.v.col, db, de, lo); k < de; ++k) {
+        constexpr uint32_t step = P == 2 ? kGenLanes : 1u;
+        // (64-bit: the last stride may pass 2^32)
+        for (uint64_t k = (uint64_t)lower_bound_g(g.v.col, db, de, lo) + (P == 2 ? sub : 0u); k < de; k += step) {
             if constexpr (ENUM) {
                 if (g.en.out && *(const volatile unsigned long long *)g.en.n >= g.en.k)
                     return;
@@ -2921,14 +2951,14 @@ __device__ void gen_walk(const GenRegs &g, uint32_t (&x)[kMaxQ], unsigned long l
                 ++cnt;
             } else {
                 x[P] = w;
-                gen_walk<P + 1, DEND, ENUM>(g, x, cnt);
+                gen_walk<P + 1, DEND, ENUM>(g, x, cnt, 0u);
             }
         }
     }
 }
 
 // Items of one depth; tstart[i] - tstart[0] = first task of item i
-// (tstart[n] - tstart[0] tasks in all). Warps take 32 tasks at a time.
+// (tstart[n] - tstart[0] tasks in all). Warps take 32 / kGenLanes tasks at a time.
 template <int DEND, bool ENUM>
 __global__ void __launch_bounds__(256) k_general(const PairDev *__restrict__ pairs, const uint64_t *__restrict__ items,
                                                  const uint32_t *__restrict__ tstart, uint32_t nitems,
@@ -2941,11 +2971,11 @@ __global__ void __launch_bounds__(256) k_general(const PairDev *__restrict__ pai
     for (;;) {
         uint32_t t0 = 0;
         if (lane == 0)
-            t0 = atomicAdd(cursor, 32u);
+            t0 = atomicAdd(cursor, 32u / kGenLanes);
         t0 = __shfl_sync(kFull, t0, 0);
         if (t0 >= total)
             break;
-        const uint32_t t = t0 + (uint32_t)lane;
+        const uint32_t t = t0 + (uint32_t)lane / kGenLanes;
         if (t >= total)
             continue;
         const uint32_t b = find_batch(tstart, nitems, t + base0);
@@ -2962,9 +2992,15 @@ __global__ void __launch_bounds__(256) k_general(const PairDev *__restrict__ pai
         uint32_t x[kMaxQ];
         x[0] = r;
         x[1] = g.v.col[g.v.rp[r] + j0 + (t + base0 - tstart[b])];
-        gen_walk<2, DEND, ENUM>(g, x, cnt);
+        gen_walk<2, DEND, ENUM>(g, x, cnt, (uint32_t)lane % kGenLanes);
     }
-    if (count_ptr)
+    // one atomic per warp where its lanes end on the same pair (a lane each was
+    // 300,000 atomics on one address)
+    int same = 0;
+    __match_all_sync(kFull, (unsigned long long)count_ptr, &same);
+    if (same)
+        cnt = warp_sum(cnt);
+    if (count_ptr && (!same || lane == 0))
         flush_count(count_ptr, cnt);
 }
 
@@ -3333,13 +3369,16 @@ __host__ __device__ __forceinline__ uint32_t dom_class(uint32_t tier, uint32_t D
         return D < 63 ? D : 63; // at most kSmallMaxD = 64
     if (tier == 2 || tier == 3)
         return 63 - (D / 16 < 63 ? D / 16 : 63); // at most kMediumMaxD = 1024
-    if (tier == 4) { // half-octaves
+    if (tier == 4) { // eighths of an octave from 2^10 (coarser classes cost the 4-wheel 12%)
 #ifdef __CUDA_ARCH__
         const uint32_t lg = 31u - (uint32_t)__clz((int)D);
 #else
         const uint32_t lg = 31u - (uint32_t)__builtin_clz(D);
 #endif
-        return 63 - (2 * lg + ((D >> (lg - 1)) & 1u));
+        if (lg < 10)
+            return 63; // tuned limits may leave smaller domains to this tier
+        const uint32_t c = 8 * (lg - 10) + ((D >> (lg - 3)) & 7u);
+        return 63 - (c < 63 ? c : 63);
     }
     return 0;
 }
@@ -3749,13 +3788,20 @@ struct LaunchRec {
     int tail_slot = -1;       // stats tail this launch's exit spread counts to (0 small, 1 medium, 2 large)
 };
 
+// Blocks of k_large_rows: as many as fit beside each other with the domain
+// list staged in shared memory (one block of 512 threads per SM left the SM a
+// quarter full, and the pass waits on dependent loads).
+static int large_rows_grid(const Ctx *ctx, size_t smemA) {
+    return ctx->num_sms * (int)std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / (smemA + 5 * 1024)));
+}
+
 // The degree pass of the neighbourhood-statistics roots a kLargeRows record builds.
 static LaunchRec nbdeg_rec(const LaunchRec &rows) {
     LaunchRec r = rows;
     r.kind = LaunchRec::kLargeNbDeg;
     r.block = 256;
     r.smem = 0;
-    r.grid = rows.grid * 4;
+    r.grid = std::max(rows.grid, 592); // whole SMs' worth of 256-thread blocks
     r.cursor = nullptr;
     return r;
 }
@@ -3766,7 +3812,7 @@ static LaunchRec lists_rec(const LaunchRec &rows) {
     r.kind = LaunchRec::kLargeLists;
     r.block = 256;
     r.smem = 0;
-    r.grid = rows.grid * 4;
+    r.grid = std::max(rows.grid, 592); // whole SMs' worth of 256-thread blocks
     r.cursor = nullptr;
     return r;
 }
@@ -4171,7 +4217,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         st.bitmap_bytes += large_words * 4;
         LaunchRec lr;
         lr.kind = LaunchRec::kLargeRows;
-        lr.grid = ctx->num_sms;
+        lr.grid = large_rows_grid(ctx, smemA);
         lr.block = 512;
         lr.smem = smemA;
         lr.bt = Batch{list, reinterpret_cast<const uint64_t *>(boff), cstart, tstart, nl};
@@ -4312,7 +4358,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             st.bitmap_bytes += words * 4;
             LaunchRec lr;
             lr.kind = LaunchRec::kLargeRows;
-            lr.grid = ctx->num_sms;
+            lr.grid = large_rows_grid(ctx, smemA);
             lr.block = 512;
             lr.smem = smemA;
             lr.bt = Batch{d_bitem, d_boff, d_cs, d_ts, nbt};
