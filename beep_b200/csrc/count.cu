@@ -1144,6 +1144,9 @@ __device__ __forceinline__ uint32_t pair_rlo(const PairRegs &pr, uint32_t D, uin
 // registers (five blocks per SM, no spills), a few percent faster on C2.
 // ---------------------------------------------------------------------------
 constexpr int kSmallWarps = 8;
+// blocks of a small launch per SM: several times what is resident, so that
+// blocks that drew short roots make room for the next ones
+constexpr int kSmallBlocksPerSm = 32;
 constexpr int kTinyMaxD = 16;
 
 // A walk of depth 6 or more multiplies a root's work by its density at every
@@ -1153,6 +1156,10 @@ constexpr int kTinyMaxD = 16;
 // builds the rows again (a small share of its walk) and takes every parts-th
 // chunk of the walk. (6- and 7-cliques there together: 193 -> 31 ms.)
 constexpr uint32_t kSplitMinD = 24;
+// parts of a root of D vertices (of at most `parts`): 8 vertices each
+__device__ __forceinline__ uint32_t root_parts(uint32_t parts, uint32_t D) {
+    return parts == 1 || D <= kSplitMinD ? 1u : min(parts, D / 8);
+}
 inline uint32_t walk_parts(int dend, bool enumerate) { return enumerate || dend < 6 ? 1u : (dend == 6 ? 8u : 32u); }
 
 template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigned long long v, unsigned gmask) {
@@ -1409,10 +1416,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
         uint32_t beg, D, j0;
         pair_domain(pr, r, beg, D, j0);
         const uint32_t rlo = pair_rlo(pr, D, j0);
-        const bool split = parts > 1 && D > kSplitMinD && pr.lp.free_from > 2;
-        if (part > 0 && !split) // the root's first part takes it whole
+        const uint32_t nparts = pr.lp.free_from > 2 ? root_parts(parts, D) : 1u;
+        if (part >= nparts)
             continue;
-        const uint32_t nparts = split ? parts : 1u;
         for (uint32_t i = glane; i < D; i += G) {
             A[i] = pr.v.col[beg + i];
             rows[i] = 0;
@@ -1658,6 +1664,60 @@ __device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, u
     }
 }
 
+// Prefixes x[1..P], one per lane (valid or not), extended a level at a time to
+// x[1..DEND-3], whose completions clique_walk counts: the children of all 32
+// lanes are numbered and taken 32 at a time, so every lane has one however the
+// candidates are spread (a lane walking its own subtree left most of the warp
+// idle: 7-cliques, R-MAT s14 ef12, 28.9 ms). Warp-wide.
+template <int P, int DEND>
+__device__ __forceinline__ void clique_expand(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t (&x)[kMaxQ],
+                                              bool valid, int lane, unsigned long long &cnt) {
+    if constexpr (P >= DEND - 3) {
+        if (valid)
+            clique_walk<P, DEND>(rows, RS, W, x, cnt);
+        __syncwarp();
+    } else {
+        uint32_t c = 0;
+        if (valid)
+            for (uint32_t k = x[P] >> 5; k < W; ++k)
+                c += (uint32_t)__popc(clique_word<P>(rows, RS, x, k));
+        uint32_t inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o)
+                inc += y;
+        }
+        const uint32_t T = __shfl_sync(kFull, inc, 31);
+        for (uint32_t base = 0; base < T; base += 32) {
+            const uint32_t t = base + (uint32_t)lane;
+            uint32_t own = 0; // lanes whose children end at or before t
+#pragma unroll
+            for (uint32_t step = 16; step; step >>= 1)
+                if (__shfl_sync(kFull, inc, (int)(own + step - 1)) <= t)
+                    own += step;
+            uint32_t j = t - __shfl_sync(kFull, inc - c, (int)own);
+            uint32_t y[kMaxQ];
+#pragma unroll
+            for (int q = 1; q <= P; ++q)
+                y[q] = __shfl_sync(kFull, x[q], (int)own);
+            const bool ok = t < T;
+            if (ok) {
+                uint32_t k = y[P] >> 5, w = clique_word<P>(rows, RS, y, k);
+                for (uint32_t pc = (uint32_t)__popc(w); j >= pc; pc = (uint32_t)__popc(w)) {
+                    j -= pc;
+                    w = clique_word<P>(rows, RS, y, ++k);
+                }
+                for (; j; --j)
+                    w &= w - 1;
+                y[P + 1] = (k << 5) + (uint32_t)(__ffs(w) - 1);
+            }
+            __syncwarp();
+            clique_expand<P + 1, DEND>(rows, RS, W, y, ok, lane, cnt);
+        }
+    }
+}
+
 // Every clique of a root's domain graph (block-wide): warps take 32 (x1, x2)
 // edges at a time from s_j, chunks part, part + parts, ..; s_cnt: D + 1 words.
 template <int DEND>
@@ -1685,6 +1745,7 @@ __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, u
         const uint32_t t = (__shfl_sync(kFull, c, 0) << 5) + (uint32_t)lane;
         if (t - (uint32_t)lane >= T)
             break;
+        uint32_t x[kMaxQ];
         if (t < T) {
             uint32_t a = 0, b = D; // last i with s_cnt[i] <= t
             while (b - a > 1) {
@@ -1694,7 +1755,6 @@ __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, u
                 else
                     b = mid;
             }
-            uint32_t x[kMaxQ];
             x[1] = a;
             uint32_t j = t - s_cnt[a], k = a >> 5, w = rows[a * RS + k];
             for (uint32_t pc = (uint32_t)__popc(w); j >= pc; pc = (uint32_t)__popc(w)) {
@@ -1704,9 +1764,12 @@ __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, u
             for (; j; --j)
                 w &= w - 1;
             x[2] = (k << 5) + (uint32_t)(__ffs(w) - 1);
-            clique_walk<2, DEND>(rows, RS, W, x, cnt);
+            if constexpr (DEND <= 5)
+                clique_walk<2, DEND>(rows, RS, W, x, cnt);
         }
         __syncwarp();
+        if constexpr (DEND > 5)
+            clique_expand<2, DEND>(rows, RS, W, x, t < T, lane, cnt);
     }
 }
 
@@ -1784,12 +1847,11 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         uint32_t beg, D, j0;
         pair_domain(pr, r, beg, D, j0);
         const uint32_t rlo = pair_rlo(pr, D, j0);
-        const bool split = parts > 1 && D > kSplitMinD;
-        if (part > 0 && !split) { // block-uniform: the root's first part takes it whole
+        const uint32_t nparts = root_parts(parts, D);
+        if (part >= nparts) { // block-uniform
             __syncthreads();
             continue;
         }
-        const uint32_t nparts = split ? parts : 1u;
         const uint32_t W = (D + 31) >> 5;
         // 32-bit words per row
         const uint32_t row_words = clique ? clique_stride(W) : (G == 0 ? 2 * kThreadNW : W);
@@ -3430,7 +3492,12 @@ __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pa
                 D -= j0; // level-1 tasks of the list walker
             }
         } else if (root_ok && D + 1 >= (uint32_t)pd.pl.dend) {
-            tc = D <= cfg.small_max ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
+            // (6-cliques and larger: the medium tier's expansion from
+            // kSplitMinD vertices on, where the small tier's lanes diverge)
+            const uint32_t smax = pd.pl.clique && pd.pl.dend >= 6 && pd.en.out == nullptr
+                                      ? min(cfg.small_max, kSplitMinD)
+                                      : cfg.small_max;
+            tc = D <= smax ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
         }
         tier[t] = (uint8_t)tc;
         dom[t] = D;
@@ -4164,7 +4231,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     uint32_t *wsc = nullptr;
     uint32_t wstride = 0;
     {
-        if (tier_depth[3 * kSlots + kWheelSlot] > 0 || tier_depth[3 * kSlots + kNbhdSlot] > 0) {
+        // (roots counted in strips need none)
+        if ((tier_depth[3 * kSlots + kWheelSlot] > 0 || tier_depth[3 * kSlots + kNbhdSlot] > 0) &&
+            (tier_max[3] + 31) / 32 > kC4StripMaxW) {
             wstride = (4 * ((tier_max[3] + 31) / 32) + 31) & ~31u;
             const size_t words = (size_t)ctx->num_sms * kLargeDfsBlocksPerSm * 8 * wstride;
             BEEP_TRY(lp->alloc(wsc, words));
@@ -4451,7 +4520,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 r.group = group;
                 r.parts = part == 0 ? 1u : walk_parts(r.dend, r.enumerate);
                 r.grid = (int)std::min<int64_t>(((int64_t)cnt * r.parts + per_block - 1) / per_block,
-                                                (int64_t)ctx->num_sms * 8);
+                                                (int64_t)ctx->num_sms * kSmallBlocksPerSm);
                 r.block = kSmallWarps * 32;
                 r.items = list + first;
                 r.n = cnt;
@@ -5457,7 +5526,7 @@ extern "C" beep_status beep_count_noalloc(int device, void *cuda_stream, int64_t
             const int group = part == 0 ? 8 : 32, per_block = kSmallWarps * 32 / group;
             const uint32_t np = part == 0 ? 1u : parts;
             const int grid = (int)std::min<int64_t>(((int64_t)cnt * np + per_block - 1) / per_block,
-                                                    (int64_t)num_sms * 8);
+                                                    (int64_t)num_sms * kSmallBlocksPerSm);
             BEEP_TRY(launch_small<false>(pl.dend, group, grid, s, d_pair, d_items + (part ? tiny : 0), cnt, np,
                                          nullptr));
         }
