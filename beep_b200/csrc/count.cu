@@ -1273,28 +1273,6 @@ __device__ __forceinline__ unsigned long long c4_pairs(uint32_t (&s)[NS], int L,
     return tot;
 }
 
-// Appends the set bits of this lane's word w (word index k) to ib in order,
-// group-wide (G lanes, mask gmask); returns the group's total.
-template <int G>
-__device__ __forceinline__ uint32_t c4_indices(uint32_t w, uint32_t k, uint16_t *ib, int glane, unsigned gmask) {
-    const uint32_t n = (uint32_t)__popc(w);
-    uint32_t inc = n;
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(gmask, inc, o, G);
-        if (glane >= o)
-            inc += y;
-    }
-    uint32_t at = inc - n;
-    while (w) {
-        ib[at++] = (uint16_t)((k << 5) + (uint32_t)(__ffs(w) - 1));
-        w &= w - 1;
-    }
-    const uint32_t total = __shfl_sync(gmask, inc, G - 1, G);
-    __syncwarp(gmask);
-    return total;
-}
-
 // What the counters of one vertex a are summed into. b runs over row(a), c over
 // the columns; n_c counts the b whose row holds c.
 enum C4Mode : int {
@@ -1327,6 +1305,65 @@ template <int MODE> __device__ __forceinline__ uint32_t c4_input(uint32_t w, uin
     const uint32_t bw = b >> 5;
     return k > bw ? w : (k == bw ? w & ~((2u << (b & 31)) - 1u) : 0u);
 }
+// 16-bit entries of a group's index list: D, in 16-byte steps.
+__host__ __device__ __forceinline__ uint32_t c4_list(uint32_t D) { return (D + 7) & ~7u; }
+
+// Appends the set bits of this lane's word w (word index k) to ib in order,
+// group-wide (G lanes, mask gmask); returns the group's total.
+template <int G>
+__device__ __forceinline__ uint32_t c4_indices(uint32_t w, uint32_t k, uint16_t *ib, int glane, unsigned gmask) {
+    const uint32_t n = (uint32_t)__popc(w);
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(gmask, inc, o, G);
+        if (glane >= o)
+            inc += y;
+    }
+    uint32_t at = inc - n;
+    while (w) {
+        ib[at++] = (uint16_t)((k << 5) + (uint32_t)(__ffs(w) - 1));
+        w &= w - 1;
+    }
+    const uint32_t total = __shfl_sync(gmask, inc, G - 1, G);
+    __syncwarp(gmask);
+    return total;
+}
+
+// Adds rows ib[0, nb) of column `col` (row b at col + b * RS) to the counters:
+// eight indices by one 16-byte load and eight unpredicated row loads a step;
+// only the last step, of fewer than eight, is masked. Every lane's column is
+// readable (callers clamp it to the row and mask the sums), so the loop holds
+// no bounds test.
+template <int MODE, int NS>
+__device__ __forceinline__ void c4_add_rows(uint32_t (&s)[NS], const uint32_t *col, uint32_t RS, uint32_t k,
+                                            const uint16_t *ib, uint32_t nb) {
+    uint32_t i = 0;
+    for (; i + 8 <= nb; i += 8) {
+        const uint4 p = *reinterpret_cast<const uint4 *>(ib + i);
+        const uint32_t pk[4] = {p.x, p.y, p.z, p.w};
+        uint32_t d[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t b = q & 1 ? pk[q >> 1] >> 16 : pk[q >> 1] & 0xffffu;
+            d[q] = c4_input<MODE>(col[(size_t)b * RS], k, b);
+        }
+        c4_add8<NS>(s, d);
+    }
+    if (i < nb) {
+        uint32_t d[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            d[q] = 0;
+            if (i + q < nb) {
+                const uint32_t b = ib[i + q];
+                d[q] = c4_input<MODE>(col[(size_t)b * RS], k, b);
+            }
+        }
+        c4_add8<NS>(s, d);
+    }
+}
+
 // The mode's sum over the counters of slices [0, L) in the columns of mask.
 template <int MODE, int NS>
 __device__ __forceinline__ unsigned long long c4_sum(uint32_t (&s)[NS], int L, uint32_t mask) {
@@ -1355,18 +1392,8 @@ __device__ __forceinline__ unsigned long long c4_group(const uint32_t *rows, uin
 #pragma unroll
     for (int i = 0; i < NS; ++i)
         s[i] = 0;
-    for (uint32_t i = 0; i < nb; i += 8) {
-        uint32_t d[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            d[q] = 0;
-            if (cm && i + q < nb) {
-                const uint32_t b = ib[i + q];
-                d[q] = c4_input<MODE>(rows[(size_t)b * RS + k], k, b);
-            }
-        }
-        c4_add8<NS>(s, d);
-    }
+    const uint32_t kc = min(k, W - 1);
+    c4_add_rows<MODE, NS>(s, rows + kc, RS, kc, ib, nb);
     __syncwarp(gmask); // ib is rewritten by the group's next call
     return nb ? c4_sum<MODE, NS>(s, 32 - __clz((int)nb), cm) : 0ull;
 }
@@ -1546,7 +1573,7 @@ __device__ __forceinline__ void nbhd_medium(int form, const uint32_t *rows, uint
                                             unsigned long long &plus, unsigned long long &minus) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    uint16_t *ib = ib_all + (threadIdx.x / G) * (size_t)((D + 1) & ~1u);
+    uint16_t *ib = ib_all + (threadIdx.x / G) * (size_t)c4_list(D);
     if (threadIdx.x == 0) {
         s_misc[0] = 0;
         s_misc[1] = j0;
@@ -1924,7 +1951,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 static_assert(2 * kThreadNW == 8, "8 words a row");
                 const int gl = lane & 7;
                 const unsigned gm = 0xffu << (lane & 24);
-                uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 3) * (size_t)((D + 1) & ~1u);
+                uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 3) * (size_t)c4_list(D);
                 for (;;) {
                     uint32_t j = 0;
                     if (gl == 0)
@@ -1999,7 +2026,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 if constexpr (G == 32) {
                     if (wheel) { // block-uniform; rows of the whole domain
                         uint16_t *ib =
-                            reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 5) * (size_t)((D + 1) & ~1u);
+                            reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 5) * (size_t)c4_list(D);
                         cnt = sat_add(cnt, c4_group<kC4Cycles, 32, 11>(rows, W, W, D - 1 - j, ib, glane, gmask));
                         continue;
                     }
@@ -2381,7 +2408,8 @@ template <int MODE>
 __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restrict__ bm, uint32_t W, uint32_t a,
                                                        uint32_t st, uint16_t *ib, int lane) {
     const uint32_t k = 32 * st + (uint32_t)lane;
-    const uint32_t *ra = bm + (size_t)a * W, *col = bm + k;
+    const uint32_t kc = min(k, W - 1);
+    const uint32_t *ra = bm + (size_t)a * W, *col = bm + kc;
     const uint32_t cm = k < W ? c4_c_bits<MODE>(ra[k], k, a) : 0u;
     if (!__ballot_sync(kFull, cm != 0))
         return 0;
@@ -2396,18 +2424,7 @@ __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restric
         const uint32_t wi = w0 + (uint32_t)lane;
         const uint32_t nb = c4_indices<32>(wi < wend ? c4_b_bits<MODE>(ra[wi], wi, a) : 0u, wi, ib, lane, kFull);
         total += nb;
-        for (uint32_t i = 0; i < nb; i += 8) {
-            uint32_t d[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                d[q] = 0;
-                if (cm && i + q < nb) {
-                    const uint32_t b = ib[i + q];
-                    d[q] = c4_input<MODE>(col[(size_t)b * W], k, b);
-                }
-            }
-            c4_add8<kC4MaxSlices>(s, d);
-        }
+        c4_add_rows<MODE, kC4MaxSlices>(s, col, W, kc, ib, nb);
         __syncwarp();
     }
     return total ? c4_sum<MODE, kC4MaxSlices>(s, 32 - __clz((int)total), cm) : 0ull;
@@ -2614,7 +2631,7 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
     // and on exit)
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
-    __shared__ uint16_t s_ib[8][1024];
+    __shared__ __align__(16) uint16_t s_ib[8][1024];
     PairRegs pr;
     uint32_t cur = 0xffffffffu;
     unsigned long long cnt = 0;
@@ -2833,7 +2850,7 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
     // [2 Wm, 3 Wm)
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
-    __shared__ uint16_t s_ib[8][1024];
+    __shared__ __align__(16) uint16_t s_ib[8][1024];
     PairRegs pr;
     uint32_t cur = 0xffffffffu;
     int form = kNbNone;
