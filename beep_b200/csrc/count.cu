@@ -1653,8 +1653,36 @@ __device__ __forceinline__ uint32_t clique_word(const uint32_t *rows, uint32_t R
     return w;
 }
 
-// Ways to complete x[1..P] to x[1..DEND-1].
-template <int P, int DEND>
+// Edges inside the candidates that follow x[1..NP], rows of at most 8 words:
+// the candidate words stay in registers, so each is ANDed once (in the general
+// form below once per word pair) and a vertex's bit is found once for all
+// words.
+template <int NP>
+__device__ __forceinline__ uint32_t clique_edges8(const uint32_t *rows, uint32_t RS, uint32_t W,
+                                                  const uint32_t (&x)[kMaxQ]) {
+    uint32_t S[8], n = 0;
+    const uint32_t k0 = x[NP] >> 5;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+        S[k] = k >= k0 && k < W ? clique_word<NP>(rows, RS, x, k) : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t *rk = rows + (k << 5) * RS;
+        for (uint32_t b = S[k]; b;) { // y < z in word k: b without y is the candidates above y
+            const uint32_t *ry = rk + (uint32_t)(__ffs(b) - 1) * RS;
+            b &= b - 1;
+            n += (uint32_t)__popc(ry[k] & b);
+#pragma unroll
+            for (uint32_t w = k + 1; w < 8; ++w)
+                if (S[w])
+                    n += (uint32_t)__popc(ry[w] & S[w]);
+        }
+    }
+    return n;
+}
+
+// Ways to complete x[1..P] to x[1..DEND-1]. NARROW: rows of at most 8 words.
+template <int P, int DEND, bool NARROW>
 __device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t (&x)[kMaxQ],
                                             unsigned long long &cnt) {
     uint32_t n = 0;
@@ -1662,6 +1690,8 @@ __device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, u
         for (uint32_t k = x[P] >> 5; k < W; ++k)
             n += (uint32_t)__popc(clique_word<P>(rows, RS, x, k));
         cnt += n;
+    } else if constexpr (P == DEND - 3 && NARROW) {
+        cnt += clique_edges8<P>(rows, RS, W, x);
     } else if constexpr (P == DEND - 3) {
         for (uint32_t k = x[P] >> 5; k < W; ++k) {
             const uint32_t sk = clique_word<P>(rows, RS, x, k);
@@ -1686,7 +1716,7 @@ __device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, u
         for (uint32_t k = x[P] >> 5; k < W; ++k)
             for (uint32_t b = clique_word<P>(rows, RS, x, k); b; b &= b - 1) {
                 x[P + 1] = (k << 5) + (uint32_t)(__ffs(b) - 1);
-                clique_walk<P + 1, DEND>(rows, RS, W, x, cnt);
+                clique_walk<P + 1, DEND, NARROW>(rows, RS, W, x, cnt);
             }
     }
 }
@@ -1696,12 +1726,12 @@ __device__ __forceinline__ void clique_walk(const uint32_t *rows, uint32_t RS, u
 // lanes are numbered and taken 32 at a time, so every lane has one however the
 // candidates are spread (a lane walking its own subtree left most of the warp
 // idle: 7-cliques, R-MAT s14 ef12, 28.9 ms). Warp-wide.
-template <int P, int DEND>
+template <int P, int DEND, bool NARROW>
 __device__ __forceinline__ void clique_expand(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t (&x)[kMaxQ],
                                               bool valid, int lane, unsigned long long &cnt) {
     if constexpr (P >= DEND - 3) {
         if (valid)
-            clique_walk<P, DEND>(rows, RS, W, x, cnt);
+            clique_walk<P, DEND, NARROW>(rows, RS, W, x, cnt);
         __syncwarp();
     } else {
         uint32_t c = 0;
@@ -1740,14 +1770,14 @@ __device__ __forceinline__ void clique_expand(const uint32_t *rows, uint32_t RS,
                 y[P + 1] = (k << 5) + (uint32_t)(__ffs(w) - 1);
             }
             __syncwarp();
-            clique_expand<P + 1, DEND>(rows, RS, W, y, ok, lane, cnt);
+            clique_expand<P + 1, DEND, NARROW>(rows, RS, W, y, ok, lane, cnt);
         }
     }
 }
 
 // Every clique of a root's domain graph (block-wide): warps take 32 (x1, x2)
 // edges at a time from s_j, chunks part, part + parts, ..; s_cnt: D + 1 words.
-template <int DEND>
+template <int DEND, bool NARROW>
 __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
                                             uint32_t *s_cnt, uint32_t *s_j, uint32_t part, uint32_t parts,
                                             unsigned long long &cnt) {
@@ -1792,11 +1822,11 @@ __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, u
                 w &= w - 1;
             x[2] = (k << 5) + (uint32_t)(__ffs(w) - 1);
             if constexpr (DEND <= 5)
-                clique_walk<2, DEND>(rows, RS, W, x, cnt);
+                clique_walk<2, DEND, NARROW>(rows, RS, W, x, cnt);
         }
         __syncwarp();
         if constexpr (DEND > 5)
-            clique_expand<2, DEND>(rows, RS, W, x, t < T, lane, cnt);
+            clique_expand<2, DEND, NARROW>(rows, RS, W, x, t < T, lane, cnt);
     }
 }
 
@@ -1937,7 +1967,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         bool clique_done = false;
         if constexpr (DEND >= 4 && !ENUM) {
             if (clique) {
-                clique_root<DEND>(rows, row_words, W, D, s_pre, &s_j, part, nparts, cnt);
+                clique_root<DEND, G == 0>(rows, row_words, W, D, s_pre, &s_j, part, nparts, cnt);
                 clique_done = true;
             }
         }
@@ -3509,10 +3539,10 @@ __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pa
                 D -= j0; // level-1 tasks of the list walker
             }
         } else if (root_ok && D + 1 >= (uint32_t)pd.pl.dend) {
-            // (6-cliques and larger: the medium tier's expansion from
-            // kSplitMinD vertices on, where the small tier's lanes diverge)
+            // (6-cliques and larger: the medium tier's expansion above
+            // kTinyMaxD vertices, where the small tier's lanes diverge)
             const uint32_t smax = pd.pl.clique && pd.pl.dend >= 6 && pd.en.out == nullptr
-                                      ? min(cfg.small_max, kSplitMinD)
+                                      ? min(cfg.small_max, (uint32_t)kTinyMaxD)
                                       : cfg.small_max;
             tc = D <= smax ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
         }
