@@ -2424,19 +2424,26 @@ __host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D) {
 }
 static_assert((kC4StripMaxW * 32) >> kC4MaxSlices == 0, "a count fits the slices");
 
+// A hub's paw strips run over all its neighbours b (its 4-wheel strips do too,
+// but start first and are not the longest launch): 0.5 ms for one of 12,000.
+constexpr uint32_t kPawParts = 4;
 __host__ __device__ __forceinline__ bool nbhd_strips(int nbhd, uint32_t D) {
     return nbhd >= kNbTriIso && (D + 31) / 32 <= kC4StripMaxW;
 }
 __host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, const DevPlan &pl) {
-    if (nbhd_strips(pl.nbhd, D))
-        return (D - j0) * ((D + 1023) / 1024); // (u, strip) pairs
+    if (nbhd_strips(pl.nbhd, D)) // (u, strip) pairs, in parts
+        return (D - j0) * ((D + 1023) / 1024) * (pl.nbhd == kNbPaw ? kPawParts : 1u);
     return pl.wheel4 && (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D - j0;
 }
 
 // One strip of vertex a: this lane's part of the mode's sum.
+// (part of parts: every parts-th 1,024 of the b's, for the modes that are
+// linear in the counters)
 template <int MODE>
 __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restrict__ bm, uint32_t W, uint32_t a,
-                                                       uint32_t st, uint16_t *ib, int lane) {
+                                                       uint32_t st, uint16_t *ib, int lane, uint32_t part = 0,
+                                                       uint32_t parts = 1) {
+    static_assert(MODE >= 0 && MODE <= 3, "a C4Mode");
     const uint32_t k = 32 * st + (uint32_t)lane;
     const uint32_t kc = min(k, W - 1);
     const uint32_t *ra = bm + (size_t)a * W, *col = bm + kc;
@@ -2450,7 +2457,7 @@ __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restric
     uint32_t total = 0;
     // the b's: all of row(a), below a, or (paw, c > b) up to the strip's last word
     const uint32_t wend = MODE == kC4Diamond ? W : (MODE == kC4Paw ? min(W, 32 * st + 32) : (a >> 5) + 1);
-    for (uint32_t w0 = 0; w0 < wend; w0 += 32) {
+    for (uint32_t w0 = 32 * part; w0 < wend; w0 += 32 * parts) {
         const uint32_t wi = w0 + (uint32_t)lane;
         const uint32_t nb = c4_indices<32>(wi < wend ? c4_b_bits<MODE>(ra[wi], wi, a) : 0u, wi, ib, lane, kFull);
         total += nb;
@@ -2922,7 +2929,8 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
             // the forms' per-edge terms by bit-sliced counters, the largest
             // (and most connected) u first; forms without them (wedge, two
             // edges) and wider rows take nbhd_task
-            const uint32_t S = (D + 1023) / 1024, ti = t - bt.tstart[b], st = ti % S, u = D - 1 - ti / S;
+            const uint32_t S = (D + 1023) / 1024, pp = form == kNbPaw ? kPawParts : 1u, tt = t - bt.tstart[b];
+            const uint32_t part = tt % pp, ti = tt / pp, st = ti % S, u = D - 1 - ti / S;
             uint16_t *ib = s_ib[threadIdx.x >> 5];
             const unsigned long long du = deg[u], rest = D - 3;
             switch (form) {
@@ -2938,7 +2946,7 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
             }
             case kNbPaw:
                 if (du >= 2)
-                    plus = sat_add(plus, sat_mul(c4_strip<kC4Paw>(rows, W, u, st, ib, lane), du - 2));
+                    plus = sat_add(plus, sat_mul(c4_strip<kC4Paw>(rows, W, u, st, ib, lane, part, pp), du - 2));
                 break;
             default: // kNbDiamond
                 plus = sat_add(plus, c4_strip<kC4Diamond>(rows, W, u, st, ib, lane));
@@ -3501,6 +3509,23 @@ constexpr uint32_t kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144, kMiscSup =
 static_assert(kMiscSlots + kTiers * kSlots <= kMiscTiny && kMiscTiny + kSlots <= kMiscLarge, "planning block");
 constexpr uint32_t kMiscWords = kMiscBuckets + kBuckets;
 
+// Largest domain of a plan's roots that the small tier takes (at most; the
+// call's limits may be lower). A warp builds such a root's rows with dependent
+// loads: near 64 vertices that takes as long as a launch's whole small tier,
+// and a block of the medium tier does it sooner. Counting calls, ms with the
+// limit at 64 / 48 / 32: 4-cliques on a power-law graph of 100,003 vertices
+// .373 / .306 / .303 and on R-MAT s20 ef3 .82 / .83 / .89, so 48; 5-cliques on
+// the first .91 / .67 / .60 and on one of 32,768 .80 / .55 / .45, so 32.
+// Larger cliques gain from the medium tier's expansion at any size beyond the
+// 8-lane groups', the 4-wheel and the statistics from its counters.
+__host__ __device__ __forceinline__ uint32_t small_limit(const DevPlan &pl, bool enumerating) {
+    if (enumerating)
+        return kSmallMaxD;
+    if (pl.clique)
+        return pl.dend == 4 ? 48u : (pl.dend == 5 ? 32u : (uint32_t)kTinyMaxD);
+    return pl.wheel4 || pl.nbhd ? 32u : (uint32_t)kSmallMaxD;
+}
+
 // tier[t] for flattened vertex t; dom[t] = its domain size.
 __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pairs,
                                                   const uint64_t *__restrict__ offs, uint32_t npairs, uint64_t N,
@@ -3539,11 +3564,7 @@ __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pa
                 D -= j0; // level-1 tasks of the list walker
             }
         } else if (root_ok && D + 1 >= (uint32_t)pd.pl.dend) {
-            // (6-cliques and larger: the medium tier's expansion above
-            // kTinyMaxD vertices, where the small tier's lanes diverge)
-            const uint32_t smax = pd.pl.clique && pd.pl.dend >= 6 && pd.en.out == nullptr
-                                      ? min(cfg.small_max, (uint32_t)kTinyMaxD)
-                                      : cfg.small_max;
+            const uint32_t smax = min(cfg.small_max, small_limit(pd.pl, pd.en.out != nullptr));
             tc = D <= smax ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
         }
         tier[t] = (uint8_t)tc;
