@@ -18,8 +18,10 @@
 //     vertices, minus bits below the symmetry bound) while the enumeration
 //     state lives in registers, unrolled over the compile-time depth;
 //   - the next candidate comes from __ballot_sync + __ffs across the warp;
-//   - the last level is a popcount (as in the reference); free suffixes and
-//     the 4-wheel are counted in closed form.
+//   - the last level is a popcount (as in the reference); free suffixes, the
+//     4-wheel and the neighbourhood statistics are counted in closed form.
+// Patterns whose count is a sum of degrees and triangle counts need neither
+// roots nor bitmaps (SupForm).
 // Tiers by domain size D (limits are runtime parameters, defaults shown):
 //   small   D <= 64   a group of 8 or 32 lanes per root, 64-bit rows in shared
 //                     memory, a lane per level-1 vertex or (level-1, level-2)
@@ -1079,6 +1081,14 @@ constexpr uint32_t kAux = 8;
 // words of a pair's counter: (count, flag), (statistics plus, flag), (minus, flag)
 constexpr uint32_t kPairWords = 6;
 
+// Forms counted from a root's rows alone: the 4-wheel and the neighbourhood
+// statistics (NbhdForm). The pairs of a call that take such forms on the same
+// view are counted together: the first of them has the items and the counters
+// of all (fmask, fcount), the others have none, so a root's rows are built
+// once for all its forms.
+constexpr int kFormWheel = 0; // 1 .. 6: NbhdForm
+constexpr int kForms = 7;
+
 struct PairDev {
     ViewDev v;
     const uint32_t *g_rp, *g_col; // the graph's deduplicated input CSR (input ids)
@@ -1087,7 +1097,10 @@ struct PairDev {
     EnumDev en;                // enumeration output (out == nullptr: none)
     uint32_t min_deg;          // roots: degree >= max_qdeg ...
     uint32_t cap_deg;          // ... and < cap_deg (reference root cap, else 2^32-1)
-    uint32_t sup;              // counted from degrees and triangle counts (SupForm): no items
+    uint32_t sup;              // no items: counted from degrees and triangle counts (SupForm), or
+                               // (kSupForms) at another pair's roots
+    uint32_t fmask;            // bit f: form f is counted at this pair's roots; 0: the plan is walked
+    unsigned long long *fcount[kForms]; // ... into these pair counters
     uint32_t shard_mod;        // > 1: only roots whose input id % shard_mod == shard_rem
     uint32_t shard_rem;
 };
@@ -1170,52 +1183,9 @@ template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigne
 }
 
 // ---------------------------------------------------------------------------
-// the 4-wheel in closed form on shared-memory rows (small and medium tiers)
+// forms counted from shared-memory rows (small and medium tiers)
 // ---------------------------------------------------------------------------
-// The same count as wheel4_task (large tier) for one x1 = a: U = OR of the
-// rows of a's neighbours above a, then C(|row(a) & row(x3) above a|, 2) for
-// every x3 of U above a. Rows of the whole domain (rlo = 0).
-// One thread, rows of NW 64-bit words: row(a) and U stay in registers.
-template <int NW>
-__device__ __forceinline__ unsigned long long wheel4_thread(const uint64_t *rows, uint32_t a) {
-    uint64_t ra[NW], U[NW];
-    const uint32_t aw = a >> 6;
-    const uint64_t above = ~((2ull << (a & 63)) - 1ull); // bits of word aw above a
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-        const uint64_t w = rows[(size_t)a * NW + k];
-        ra[k] = (uint32_t)k > aw ? w : ((uint32_t)k == aw ? (w & above) : 0ull);
-        U[k] = 0;
-    }
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-        uint64_t w = ra[k];
-        while (w) {
-            const uint32_t b = (uint32_t)k * 64 + (uint32_t)(__ffsll((long long)w) - 1);
-            w &= w - 1;
-#pragma unroll
-            for (int kk = 0; kk < NW; ++kk)
-                U[kk] |= rows[(size_t)b * NW + kk];
-        }
-    }
-    unsigned long long cnt = 0;
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-        uint64_t u = (uint32_t)k > aw ? U[k] : ((uint32_t)k == aw ? (U[k] & above) : 0ull);
-        while (u) {
-            const uint32_t c = (uint32_t)k * 64 + (uint32_t)(__ffsll((long long)u) - 1);
-            u &= u - 1;
-            uint32_t n = 0;
-#pragma unroll
-            for (int kk = 0; kk < NW; ++kk)
-                n += (uint32_t)__popcll(ra[kk] & rows[(size_t)c * NW + kk]);
-            cnt = sat_add(cnt, (unsigned long long)n * (n - (n ? 1u : 0u)) / 2);
-        }
-    }
-    return cnt;
-}
-
-// Wider rows: bit-sliced counters. A lane owns one word column (32 domain
+// Bit-sliced counters. A lane owns one word column (32 domain
 // vertices c) and counts, for one vertex a, the b of row(a) below a whose row
 // holds c -- |row(a) & row(c) below a| for all 32 c at once: slice k of the
 // counters holds bit k of each. Eight row words at a time go through carry-
@@ -1378,6 +1348,85 @@ __device__ __forceinline__ unsigned long long c4_sum(uint32_t (&s)[NS], int L, u
     }
 }
 
+// The sums a root's forms add to: the 4-wheel's count, then the statistics'
+// positive and negative sums (words 0, 2 and 4 of a pair's counter).
+constexpr int kFormSums = 9; // wheel, wedge +, two edges + -, triangle +, path + -, paw +, diamond +
+__host__ __device__ constexpr int form_of_sum(int i) {
+    return i == 0 ? kFormWheel : (i == 1 ? (int)kNbWedgeIso : (i <= 3 ? (int)kNbTwoEdges
+           : (i == 4 ? (int)kNbTriIso : (i <= 6 ? (int)kNbPath4 : (i == 7 ? (int)kNbPaw : (int)kNbDiamond)))));
+}
+__host__ __device__ constexpr int word_of_sum(int i) { return i == 0 ? 0 : (i == 3 || i == 6 ? 4 : 2); }
+
+// Adds word w to 64 counters of 6 slices (at most 63 rows).
+__device__ __forceinline__ void c4_add64(uint64_t (&s)[6], uint64_t w) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const uint64_t t = s[k] & w;
+        s[k] ^= w;
+        w = t;
+        if (!w)
+            break;
+    }
+}
+__device__ __forceinline__ unsigned long long c4_pairs64(const uint64_t (&s)[6], uint64_t mask) {
+    unsigned long long tot = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const uint64_t x = s[k] & mask;
+        tot += (unsigned long long)__popcll(x) * (((1ull << (2 * k)) - (1ull << k)) / 2);
+#pragma unroll
+        for (int j = 0; j < k; ++j)
+            tot += (unsigned long long)__popcll(s[j] & x) << (j + k);
+    }
+    return tot;
+}
+__device__ __forceinline__ unsigned long long c4_total64(const uint64_t (&s)[6], uint64_t mask) {
+    unsigned long long tot = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        tot += (unsigned long long)__popcll(s[k] & mask) << k;
+    return tot;
+}
+
+// Vertex u's part of every form of fmask, one thread, rows of one 64-bit word:
+// the counters over the neighbours below u give the 4-wheel and the triangles
+// whose middle vertex is u, those over all neighbours the paw and the diamond
+// (for u at or after sp, the root's place in its list).
+__device__ __forceinline__ void forms_thread(uint32_t fmask, const uint64_t *rows, uint32_t D, uint32_t u, uint32_t sp,
+                                             unsigned long long (&acc)[kFormSums]) {
+    const uint64_t r = rows[u], below = r & ((1ull << u) - 1ull), above = r & ~((2ull << u) - 1ull);
+    const unsigned long long du = (unsigned long long)__popcll(r), rest = D >= 3 ? D - 3 : 0;
+    if (fmask >> kNbWedgeIso & 1u)
+        acc[1] = sat_add(acc[1], binom2(du) * rest);
+    if (fmask >> kNbTwoEdges & 1u)
+        acc[3] = sat_add(acc[3], binom2(du));
+    if (fmask >> kNbPath4 & 1u) // paths x - u - w - y over the edges (u, w > u); the closed ones below
+        for (uint64_t b = above; b; b &= b - 1)
+            acc[5] = sat_add(acc[5], (du - 1) * (unsigned long long)(__popcll(rows[__ffsll((long long)b) - 1]) - 1));
+    if (!(fmask & ~(1u << kNbWedgeIso | 1u << kNbTwoEdges)))
+        return;
+    uint64_t s[6] = {0, 0, 0, 0, 0, 0};
+    for (uint64_t b = below; b; b &= b - 1)
+        c4_add64(s, rows[__ffsll((long long)b) - 1]);
+    if (fmask >> kFormWheel & 1u)
+        acc[0] = sat_add(acc[0], c4_pairs64(s, (1ull << u) - 1ull));
+    if (fmask & (1u << kNbTriIso | 1u << kNbPath4)) {
+        const unsigned long long t = c4_total64(s, above);
+        if (fmask >> kNbTriIso & 1u)
+            acc[4] = sat_add(acc[4], t * rest);
+        if (fmask >> kNbPath4 & 1u)
+            acc[6] = sat_add(acc[6], 3 * t);
+    }
+    if (!(fmask & (1u << kNbPaw | 1u << kNbDiamond)) || u < sp)
+        return;
+    for (uint64_t b = above; b; b &= b - 1)
+        c4_add64(s, rows[__ffsll((long long)b) - 1]);
+    if (fmask >> kNbPaw & 1u && du >= 2)
+        acc[7] = sat_add(acc[7], c4_total64(s, r) / 2 * (du - 2));
+    if (fmask >> kNbDiamond & 1u)
+        acc[8] = sat_add(acc[8], c4_pairs64(s, above));
+}
+
 // Rows in shared memory, W <= G words each (stride RS): a group of G lanes
 // takes vertex a; this lane's part of the sum is returned. ib: D 16-bit
 // entries of the group's own.
@@ -1417,7 +1466,22 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
     uint32_t cur = 0xffffffffu;
     EnumCtx ec;
     unsigned long long cnt = 0;
-    bool wheel = false; // the 4-wheel's closed form (counts)
+    uint32_t fmask = 0; // forms counted from the rows (counts)
+    unsigned long long acc[kFormSums];
+#pragma unroll
+    for (int i = 0; i < kFormSums; ++i)
+        acc[i] = 0;
+    auto flush_forms = [&]() {
+#pragma unroll
+        for (int i = 0; i < kFormSums; ++i) {
+            if (!(fmask >> form_of_sum(i) & 1u)) // group-uniform
+                continue;
+            const unsigned long long v = group_sum<G>(acc[i], gmask);
+            if (glane == 0)
+                flush_count(pairs[cur].fcount[form_of_sum(i)] + word_of_sum(i), v);
+            acc[i] = 0;
+        }
+    };
     // largest domains first (the list rises): the last roots taken are short
     for (uint64_t vi = blockIdx.x * NG + gid; vi < (uint64_t)nitems * parts; vi += gridDim.x * NG) {
         const uint32_t ri = (uint32_t)(vi / parts), part = (uint32_t)(vi - (uint64_t)ri * parts);
@@ -1428,11 +1492,13 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
             if (glane == 0)
                 flush_count(pr.count, cnt);
             cnt = 0;
+            if constexpr (DEND == 5 && !ENUM)
+                flush_forms();
             cur = p;
             load_pair(pairs, p, pr);
             if constexpr (ENUM)
                 make_ec(ec, pairs[p].en, pairs[p].pl, pr.v);
-            wheel = DEND == 5 && !ENUM && pairs[p].pl.wheel4;
+            fmask = DEND == 5 && !ENUM ? pairs[p].fmask : 0u;
         }
         if constexpr (ENUM) { // k tuples reserved: skip the root before its rows are built
             unsigned full = glane == 0 ? (unsigned)enum_full(ec) : 0u;
@@ -1464,9 +1530,22 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
             ec.A = A;
             ec.root = r;
         }
-        if (wheel) { // group-uniform; rows of the whole domain
-            for (uint32_t j = j0 + glane; j < D; j += G)
-                cnt = sat_add(cnt, wheel4_thread<1>(rows, j));
+        if (fmask) { // group-uniform; rows of the whole domain
+            if constexpr (DEND == 5 && !ENUM) {
+                if (fmask >> kNbTwoEdges & 1u) { // C(E, 2) once a root
+                    uint32_t d = 0;
+                    for (uint32_t j = glane; j < D; j += G)
+                        d += (uint32_t)__popcll(rows[j]);
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1)
+                        d += __shfl_xor_sync(gmask, d, o, G);
+                    if (glane == 0)
+                        acc[2] = sat_add(acc[2], binom2(d / 2));
+                }
+                const uint32_t sp = pr.v.split[r];
+                for (uint32_t j = glane; j < D; j += G)
+                    forms_thread(fmask, rows, D, j, sp, acc);
+            }
         } else if (DEND == 3 || pr.lp.free_from <= 2) { // group-uniform
             for (uint32_t j = j0 + glane; j < D; j += G) {
                 uint32_t x[kMaxQ];
@@ -1505,6 +1584,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
         }
         __syncwarp(gmask);
     }
+    if constexpr (DEND == 5 && !ENUM)
+        flush_forms();
     cnt = group_sum<G>(cnt, gmask);
     // the block's groups mostly end on the same pair: one atomic for a run of
     // equal counters (a group each was up to 38,000 atomics on one address)
@@ -1621,6 +1702,27 @@ __device__ __forceinline__ void nbhd_medium(int form, const uint32_t *rows, uint
         default:
             break;
         }
+    }
+}
+
+// The 4-wheel the same way, the largest (and most connected) vertices first.
+template <int G, int NS>
+__device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
+                                             uint32_t *s_misc, uint16_t *ib_all, unsigned long long &cnt) {
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    uint16_t *ib = ib_all + (threadIdx.x / G) * (size_t)c4_list(D);
+    if (threadIdx.x == 0)
+        s_misc[1] = 0;
+    __syncthreads();
+    for (;;) {
+        uint32_t j = 0;
+        if (gl == 0)
+            j = atomicAdd(&s_misc[1], 1u);
+        j = __shfl_sync(gm, j, 0, G);
+        if (j >= D)
+            break;
+        cnt = sat_add(cnt, c4_group<kC4Cycles, G, NS>(rows, RS, W, D - 1 - j, ib, gl, gm));
     }
 }
 
@@ -1861,10 +1963,8 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
     uint32_t cur = 0xffffffffu;
     EnumCtx ec;
     unsigned long long cnt = 0;
-    bool wheel = false; // the 4-wheel's closed form (counts)
+    uint32_t fmask = 0; // forms counted from the rows (counts)
     bool clique = false; // upper rows, clique_root (counts)
-    int nbform = kNbNone; // a neighbourhood-statistics form (counts)
-    unsigned long long nb_plus = 0, nb_minus = 0;
     for (;;) {
         if (threadIdx.x == 0)
             s_ri = atomicAdd(cursor, 1u);
@@ -1876,20 +1976,14 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         const uint32_t p = item_pair(it), r = item_root(it);
         if (p != cur) { // block-uniform
             cnt = warp_sum(cnt);
-            nb_plus = warp_sum(nb_plus);
-            nb_minus = warp_sum(nb_minus);
-            if (lane == 0) {
+            if (lane == 0)
                 flush_count(pr.count, cnt);
-                flush_count(pr.count + 2, nb_plus);
-                flush_count(pr.count + 4, nb_minus);
-            }
-            cnt = nb_plus = nb_minus = 0;
+            cnt = 0;
             cur = p;
             load_pair(pairs, p, pr);
             if constexpr (ENUM)
                 make_ec(ec, pairs[p].en, pairs[p].pl, pr.v);
-            wheel = DEND == 5 && !ENUM && pairs[p].pl.wheel4;
-            nbform = (DEND == 5 && !ENUM) ? (int)pairs[p].pl.nbhd : (int)kNbNone;
+            fmask = DEND == 5 && !ENUM ? pairs[p].fmask : 0u;
             clique = DEND >= 4 && !ENUM && pairs[p].pl.clique;
         }
         if constexpr (ENUM) { // k tuples reserved: skip the root before its rows are built
@@ -1951,16 +2045,37 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
             ec.A = A;
             ec.root = r;
         }
-        bool stats_done = false; // counted by the neighbourhood statistics
+        bool stats_done = false; // counted from the rows
         if constexpr (DEND == 5 && !ENUM) {
-            if (nbform) { // block-uniform; rows of the whole domain
-                // the domain list's place takes the degrees, the row
-                // builder's arrays the index lists (as for the 4-wheel)
+            if (fmask) { // block-uniform; rows of the whole domain
+                // groups of 8 lanes (rows of 8 words) or a warp take the
+                // vertices of one form after the other. The domain list's
+                // place takes the degrees, the row builder's arrays (free
+                // again) the groups' index lists: (3 pad + 1.75 nslots) words
+                // hold 64 bytes a vertex, D rounded up to 8
+                constexpr int GG = G == 0 ? 8 : 32, NS = G == 0 ? 9 : 11;
+                static_assert(2 * kThreadNW == 8, "8 words a row");
+                const uint32_t RS = G == 0 ? 8u : W, sp = pr.v.split[r];
                 uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb);
-                if constexpr (G == 0)
-                    nbhd_medium<8, 9>(nbform, rows, 8, 8, D, j0, A, s_nb, ib, nb_plus, nb_minus);
-                else
-                    nbhd_medium<32, 11>(nbform, rows, W, W, D, j0, A, s_nb, ib, nb_plus, nb_minus);
+                for (uint32_t fm = fmask; fm; fm &= fm - 1) {
+                    const int f = __ffs((int)fm) - 1;
+                    unsigned long long c = 0, plus = 0, minus = 0;
+                    if (f == kFormWheel)
+                        wheel_medium<GG, NS>(rows, RS, RS, D, s_nb, ib, c);
+                    else
+                        nbhd_medium<GG, NS>(f, rows, RS, RS, D, f == kNbPaw || f == kNbDiamond ? sp : 0u, A, s_nb, ib,
+                                            plus, minus);
+                    c = warp_sum(c);
+                    plus = warp_sum(plus);
+                    minus = warp_sum(minus);
+                    if (lane == 0) {
+                        unsigned long long *out = pairs[cur].fcount[f];
+                        flush_count(out, c);
+                        flush_count(out + 2, plus);
+                        flush_count(out + 4, minus);
+                    }
+                    __syncthreads(); // the next form reuses the lists and the cursor
+                }
                 stats_done = true;
             }
         }
@@ -1974,24 +2089,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         if (stats_done || clique_done) {
         } else if constexpr (G == 0) {
             const uint64_t *r64 = reinterpret_cast<const uint64_t *>(rows);
-            if (wheel) { // block-uniform; rows of the whole domain
-                // 8 lanes per vertex, rows of 8 words; index lists in the
-                // space of the row builder's arrays (free again):
-                // (3 pad + 1.75 nslots) words >= 17 maxD against 32 groups x D / 2
-                static_assert(2 * kThreadNW == 8, "8 words a row");
-                const int gl = lane & 7;
-                const unsigned gm = 0xffu << (lane & 24);
-                uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 3) * (size_t)c4_list(D);
-                for (;;) {
-                    uint32_t j = 0;
-                    if (gl == 0)
-                        j = atomicAdd(&s_j, 1u);
-                    j = __shfl_sync(gm, j, 0, 8);
-                    if (j >= D)
-                        break;
-                    cnt = sat_add(cnt, c4_group<kC4Cycles, 8, 9>(rows, 8, 8, D - 1 - j, ib, gl, gm));
-                }
-            } else if (DEND == 3 || pr.lp.free_from <= 2) { // block-uniform
+            if (DEND == 3 || pr.lp.free_from <= 2) { // block-uniform
                 // level 2 is the last or is counted in closed form: O(1) per level-1 vertex
                 while (part == 0) {
                     const uint32_t j = atomicAdd(&s_j, 1u);
@@ -2053,14 +2151,6 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 j = __shfl_sync(gmask, j, 0, G);
                 if (j >= D)
                     break;
-                if constexpr (G == 32) {
-                    if (wheel) { // block-uniform; rows of the whole domain
-                        uint16_t *ib =
-                            reinterpret_cast<uint16_t *>(s_hb) + (threadIdx.x >> 5) * (size_t)c4_list(D);
-                        cnt = sat_add(cnt, c4_group<kC4Cycles, 32, 11>(rows, W, W, D - 1 - j, ib, glane, gmask));
-                        continue;
-                    }
-                }
                 uint32_t x[kMaxQ];
                 x[1] = j;
                 dfs_warp<2, DEND, ENUM, G>(pr.lp, rows, rlo, W, D, x, cnt, glane, ec, gmask);
@@ -2069,13 +2159,8 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
         __syncthreads();
     }
     cnt = warp_sum(cnt);
-    nb_plus = warp_sum(nb_plus);
-    nb_minus = warp_sum(nb_minus);
-    if (lane == 0) {
+    if (lane == 0)
         flush_count(pr.count, cnt);
-        flush_count(pr.count + 2, nb_plus);
-        flush_count(pr.count + 4, nb_minus);
-    }
     if (threadIdx.x == 0)
         record_exit(exit_t);
 }
@@ -2098,17 +2183,16 @@ constexpr uint32_t kCursorBlock = 256;   // work cursors allocated at a time
 constexpr uint32_t kWheelGroupMin = 16;  // 4-wheel pair phase by 8-lane groups from this x1 list length
 constexpr uint32_t kMaxDonLaunches = 64; // walk launches of a call with a donation queue
 // Depth slot of a root in the tier lists: its plan's depth, except the large
-// tier's 4-wheel roots, which take slot 2 (no plan has depth 2) and run on
-// k_large_wheel.
+// tier's roots of the forms counted from rows (4-wheel, statistics), which
+// take slot 2 (no plan has depth 2) and run on k_large_wheel and k_large_nbhd.
 constexpr uint32_t kWheelSlot = 2;
 constexpr int kDepthsConst = 11; // dend 0..10
 // Slots kDepthsConst.. hold the same depths for enumerating pairs, which run
 // in launches of their own (the walk that writes tuples, with no closed
 // forms), so that counting pairs of the same call keep theirs.
-constexpr uint32_t kNbhdSlot = 1; // the large tier's roots of neighbourhood-statistics plans
 __host__ __device__ __forceinline__ uint32_t depth_slot(const DevPlan &pl, uint32_t tier, bool enumerating) {
     return (enumerating ? (uint32_t)kDepthsConst : 0u) +
-           ((tier == 4 && pl.wheel4) ? kWheelSlot : ((tier == 4 && pl.nbhd) ? kNbhdSlot : (uint32_t)pl.dend));
+           (tier == 4 && (pl.wheel4 || pl.nbhd) ? kWheelSlot : (uint32_t)pl.dend);
 }
 constexpr uint32_t kLargeSmemA = 48 * 1024; // domain entries staged in shared memory
 
@@ -2135,8 +2219,8 @@ __host__ __device__ __forceinline__ uint64_t large_root_words(uint32_t D, uint32
     return ((nb ? nb_edges_offset(D, rlo) + 2 : nb_deg_offset(D, rlo)) + 31) & ~(uint64_t)31;
 }
 
-// Tasks of a large root's walk: its level-1 vertices, or (vertex, strip) pairs.
-__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, const DevPlan &pl);
+// Tasks of a large root for form f: its vertices, or (vertex, strip) pairs.
+__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f);
 
 __device__ __forceinline__ uint32_t find_batch(const uint32_t *__restrict__ start, uint32_t nb, uint32_t t) {
     // last b with start[b] <= t
@@ -2208,8 +2292,7 @@ __global__ void __launch_bounds__(256) k_large_lists(const PairDev *__restrict__
         uint32_t beg, D, j0;
         pair_domain(pr, item_root(it), beg, D, j0);
         const uint32_t W = (D + 31) >> 5, cap = list_cap(W);
-        const DevPlan &pl = pairs[item_pair(it)].pl;
-        if (cap == 0 || ((pl.wheel4 || pl.nbhd) && W <= kC4StripMaxW)) // strips read no lists
+        if (cap == 0 || (pairs[item_pair(it)].fmask && W <= kC4StripMaxW)) // strips read no lists
             continue;
         const uint32_t rlo = pair_rlo(pr, D, j0);
         const uint32_t *rows = arena + bt.off[b];
@@ -2430,10 +2513,11 @@ constexpr uint32_t kPawParts = 4;
 __host__ __device__ __forceinline__ bool nbhd_strips(int nbhd, uint32_t D) {
     return nbhd >= kNbTriIso && (D + 31) / 32 <= kC4StripMaxW;
 }
-__host__ __device__ __forceinline__ uint32_t large_tasks(uint32_t D, uint32_t j0, const DevPlan &pl) {
-    if (nbhd_strips(pl.nbhd, D)) // (u, strip) pairs, in parts
-        return (D - j0) * ((D + 1023) / 1024) * (pl.nbhd == kNbPaw ? kPawParts : 1u);
-    return pl.wheel4 && (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D - j0;
+__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f) {
+    if (f == kFormWheel)
+        return (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D;
+    const uint32_t n = f == kNbPaw || f == kNbDiamond ? D - sp : D;
+    return nbhd_strips(f, D) ? n * ((D + 1023) / 1024) * (f == kNbPaw ? kPawParts : 1u) : n;
 }
 
 // One strip of vertex a: this lane's part of the mode's sum.
@@ -2466,6 +2550,11 @@ __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restric
     }
     return total ? c4_sum<MODE, kC4MaxSlices>(s, 32 - __clz((int)total), cm) : 0ull;
 }
+
+// The strips' state (15 slices, 8 row words, addresses) just fits 64 registers,
+// four blocks an SM (three: 5.6 ms against 5.0 on R-MAT s16 ef28); the kernels
+// keep only the pair's index across tasks and look its counters up again.
+constexpr int kStripBlocksPerSm = 4;
 
 // 4-wheel task t of a root.
 __device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, uint32_t W, uint32_t D, uint32_t t,
@@ -2657,7 +2746,7 @@ __global__ void __launch_bounds__(256, (!ENUM && DEND <= 5) ? 3 : 1) k_large_dfs
 // The large tier's 4-wheel roots (classified into depth slot kWheelSlot):
 // every warp takes (root, x1) tasks from the cursor and runs wheel4_task on
 // its own scratch, wstride words at wsc + warp * wstride.
-__global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__ pairs, Batch bt,
+__global__ void __launch_bounds__(256, kStripBlocksPerSm) k_large_wheel(const PairDev *__restrict__ pairs, Batch bt,
                                                      const uint32_t *arena, unsigned *cursor, uint32_t *wsc,
                                                      uint32_t wstride, unsigned long long *exit_t) {
     const int lane = threadIdx.x & 31;
@@ -2669,7 +2758,6 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
     __shared__ __align__(16) uint16_t s_ib[8][1024];
-    PairRegs pr;
     uint32_t cur = 0xffffffffu;
     unsigned long long cnt = 0;
     for (;;) {
@@ -2685,14 +2773,13 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
         const uint32_t p = item_pair(it), r = item_root(it);
         if (p != cur) {
             cnt = warp_sum(cnt);
-            if (lane == 0)
-                flush_count(pr.count, cnt);
+            if (lane == 0 && cur != 0xffffffffu)
+                flush_count(pairs[cur].fcount[kFormWheel], cnt);
             cnt = 0;
             cur = p;
-            load_pair(pairs, p, pr);
         }
-        uint32_t beg, D, j0;
-        pair_domain(pr, r, beg, D, j0);
+        const uint32_t *rp = pairs[p].v.rp;
+        const uint32_t D = rp[r + 1] - rp[r]; // every neighbour
         const uint32_t W = (D + 31) >> 5;
         const uint32_t *rows = arena + bt.off[b]; // rows of the whole domain: rlo == 0
         if (W <= kC4StripMaxW) {
@@ -2703,12 +2790,12 @@ __global__ void __launch_bounds__(256) k_large_wheel(const PairDev *__restrict__
         rl.cap = list_cap(W);
         rl.nzc = rows + (size_t)D * W;
         rl.nzl = rl.nzc + D;
-        wheel4_task(rows, rl, W, j0 + (t - bt.tstart[b]), ws, ws + 3 * (size_t)Wm, ws + Wm, ws + 2 * (size_t)Wm, lane,
+        wheel4_task(rows, rl, W, t - bt.tstart[b], ws, ws + 3 * (size_t)Wm, ws + Wm, ws + 2 * (size_t)Wm, lane,
                     cnt);
     }
     cnt = warp_sum(cnt);
-    if (lane == 0)
-        flush_count(pr.count, cnt);
+    if (lane == 0 && cur != 0xffffffffu)
+        flush_count(pairs[cur].fcount[kFormWheel], cnt);
     if (lane == 0)
         record_exit(exit_t);
 }
@@ -2733,7 +2820,7 @@ __global__ void __launch_bounds__(256) k_large_nbdeg(const PairDev *__restrict__
     for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
         const uint32_t b = find_batch(bt.cstart, bt.nb, c);
         const uint64_t it = bt.item[b];
-        if (pairs[item_pair(it)].pl.nbhd == kNbNone)
+        if (!(pairs[item_pair(it)].fmask & ~(1u << kFormWheel)))
             continue;
         PairRegs pr;
         load_pair(pairs, item_pair(it), pr);
@@ -2872,10 +2959,10 @@ __device__ __forceinline__ void nbhd_task(int form, const uint32_t *__restrict__
     __syncwarp(); // la reused by the warp's next task
 }
 
-// The large tier's roots of neighbourhood-statistics plans (depth slot
-// kNbhdSlot): every warp takes (root, u) tasks from the cursor. The task of
+// Statistics form `form` of the large tier's roots that have it (the others
+// have no tasks): every warp takes (root, u) tasks from the cursor. The task of
 // the root's first domain vertex also adds the root-level term.
-__global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ pairs, Batch bt,
+__global__ void __launch_bounds__(256, kStripBlocksPerSm) k_large_nbhd(const PairDev *__restrict__ pairs, Batch bt, int form,
                                                     const uint32_t *arena, unsigned *cursor, uint32_t *wsc,
                                                     uint32_t wstride, unsigned long long *exit_t) {
     const int lane = threadIdx.x & 31;
@@ -2888,9 +2975,7 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
     const uint32_t Wm = wstride / 4;
     uint32_t *ws = wsc + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wstride;
     __shared__ __align__(16) uint16_t s_ib[8][1024];
-    PairRegs pr;
     uint32_t cur = 0xffffffffu;
-    int form = kNbNone;
     unsigned long long plus = 0, minus = 0;
     for (;;) {
         uint32_t t = 0;
@@ -2906,17 +2991,15 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
         if (p != cur) {
             plus = warp_sum(plus);
             minus = warp_sum(minus);
-            if (lane == 0) {
-                flush_count(pr.count + 2, plus);
-                flush_count(pr.count + 4, minus);
+            if (lane == 0 && cur != 0xffffffffu) {
+                flush_count(pairs[cur].fcount[form] + 2, plus);
+                flush_count(pairs[cur].fcount[form] + 4, minus);
             }
             plus = minus = 0;
             cur = p;
-            load_pair(pairs, p, pr);
-            form = pairs[p].pl.nbhd;
         }
-        uint32_t beg, D, j0;
-        pair_domain(pr, r, beg, D, j0);
+        const uint32_t *rp = pairs[p].v.rp;
+        const uint32_t D = rp[r + 1] - rp[r]; // every neighbour
         const uint32_t W = (D + 31) >> 5;
         const uint32_t *rows = arena + bt.off[b]; // rows of the whole domain: rlo == 0
         RowLists rl;
@@ -2954,16 +3037,18 @@ __global__ void __launch_bounds__(256) k_large_nbhd(const PairDev *__restrict__ 
             }
             continue;
         }
-        const uint32_t u = j0 + (t - bt.tstart[b]);
+        const uint32_t u =
+            (form == kNbPaw || form == kNbDiamond ? pairs[p].v.split[r] : 0u) + (t - bt.tstart[b]);
         nbhd_task(form, rows, rl, deg, E, W, D, u, t == bt.tstart[b], ws + 2 * (size_t)Wm, lane, plus, minus);
     }
     plus = warp_sum(plus);
     minus = warp_sum(minus);
-    if (lane == 0) {
-        flush_count(pr.count + 2, plus);
-        flush_count(pr.count + 4, minus);
-        record_exit(exit_t);
+    if (lane == 0 && cur != 0xffffffffu) {
+        flush_count(pairs[cur].fcount[form] + 2, plus);
+        flush_count(pairs[cur].fcount[form] + 4, minus);
     }
+    if (lane == 0)
+        record_exit(exit_t);
 }
 
 // ---------------------------------------------------------------------------
@@ -3578,7 +3663,7 @@ __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pa
         if (tc == 4) {
             const uint32_t rn = pd.pl.rows_needed, rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
             atomicAdd(reinterpret_cast<unsigned long long *>(misc + kMiscLarge),
-                      (unsigned long long)large_root_words(D, rlo, pd.pl.nbhd != kNbNone));
+                      (unsigned long long)large_root_words(D, rlo, (pd.fmask & ~(1u << kFormWheel)) != 0));
         }
         mx[tc - 1] = max(mx[tc - 1], D);
         const uint32_t slot = depth_slot(pd.pl, tc, pd.en.out != nullptr);
@@ -3703,12 +3788,21 @@ __global__ void k_large_meta(const PairDev *__restrict__ pairs, const uint64_t *
                              unsigned long long *words, uint32_t *chunks, uint32_t *tasks) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
         const uint32_t D = D_in[i], j0 = j0_in[i];
-        const DevPlan &pl = pairs[item_pair(items[i])].pl;
-        const uint32_t rn = (uint32_t)pl.rows_needed;
+        const PairDev &pd = pairs[item_pair(items[i])];
+        const uint32_t rn = (uint32_t)pd.pl.rows_needed;
         const uint32_t rlo = rn == 2 ? 0u : (rn == 1 ? j0 : D);
-        words[i] = large_root_words(D, rlo, pl.nbhd != kNbNone);
+        words[i] = large_root_words(D, rlo, (pd.fmask & ~(1u << kFormWheel)) != 0);
         chunks[i] = (D + kRowsPerChunk - 1) / kRowsPerChunk;
-        tasks[i] = large_tasks(D, j0, pl);
+        tasks[i] = pd.fmask ? 0u : D - j0; // (forms: k_form_tasks)
+    }
+}
+
+// Tasks of every listed large root for form f.
+__global__ void k_form_tasks(const PairDev *__restrict__ pairs, const uint64_t *__restrict__ items, uint32_t nl,
+                             const uint32_t *__restrict__ D_in, int f, uint32_t *tasks) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
+        const PairDev &pd = pairs[item_pair(items[i])];
+        tasks[i] = pd.fmask >> f & 1u ? form_tasks(D_in[i], pd.v.split[item_root(items[i])], f) : 0u;
     }
 }
 
@@ -3723,6 +3817,13 @@ __global__ void k_gather_dom(const PairDev *__restrict__ pairs, const uint64_t *
         D_out[i] = D;
         j0_out[i] = j0;
     }
+}
+
+// The root's place in each listed item's neighbour list.
+__global__ void k_gather_split(const PairDev *__restrict__ pairs, const uint64_t *__restrict__ items, uint32_t nl,
+                               uint32_t *out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x)
+        out[i] = pairs[item_pair(items[i])].v.split[item_root(items[i])];
 }
 
 // Adjacency bytes of the searched roots: row pointers and split of the root
@@ -3760,7 +3861,7 @@ __global__ void k_alg_bytes(const PairDev *__restrict__ pairs, const uint64_t *_
             b += 4ull * (grp[w + 1] - grp[w]);
         }
         // (pairs without items count with the small tier, as their time does)
-        const int slot = tc == 1 || pairs[p].sup ? 0 : (tc == 4 ? 2 : 1);
+        const int slot = tc == 1 || (pairs[p].sup && pairs[p].sup < kSupForms) ? 0 : (tc == 4 ? 2 : 1);
         acc[slot] += a;
         alg[slot] += b;
     }
@@ -3892,7 +3993,7 @@ template <bool ENUM> beep_status large_dfs_blocks_per_sm(int dend, int *out) {
 // Plan and execution of a multi-pair call.
 //
 // plan_pairs does everything that needs the host: views, root classification
-// (one read-back of the tier sizes), sorted item lists and the batching of
+// (one read-back of the tier sizes), bucketed item lists and the batching of
 // large roots into arena-sized groups. It leaves a list of launches whose
 // buffers it owns. execute_plan replays that list as a stream-ordered
 // sequence of memsets and kernels with no host synchronisation, so it can be
@@ -3903,6 +4004,7 @@ struct LaunchRec {
                 kLargeNbhd, kSupTri, kSupEdge, kSupVertex } kind;
     const SupView *sup = nullptr; // degree and triangle-count forms: views and 32-entry chunks
     uint32_t nsup = 0;
+    int form = 0; // kLargeNbhd: the statistics form
     uint64_t nchunks = 0;
     const uint32_t *tstart = nullptr; // list walker: task prefix of the items
     int dend = 0, grid = 0, block = 0;
@@ -4053,9 +4155,21 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         const bool whole = ps.nshards <= 1 && !ps.en && !(options & (BEEP_OPT_REFERENCE_ROOT_CAP | BEEP_OPT_NO_NBHD));
         return whole ? ps.plan.dev.support : (int32_t)kSupNone;
     };
+    // Pairs counted from a root's rows share their items too, on that view when
+    // they count every root.
+    auto row_form = [&](const PairSpec &ps) -> int {
+        if (ps.en)
+            return -1;
+        return ps.plan.dev.wheel4 ? kFormWheel
+                                  : (ps.plan.dev.nbhd && !(options & BEEP_OPT_NO_NBHD) ? (int)ps.plan.dev.nbhd : -1);
+    };
+    auto shares_view = [&](const PairSpec &ps) {
+        return sup_form(ps) ||
+               (row_form(ps) >= 0 && ps.nshards <= 1 && !(options & BEEP_OPT_REFERENCE_ROOT_CAP));
+    };
     std::map<Graph *, int32_t> sup_qdeg; // per graph, the least peel threshold of those pairs
     for (auto &ps : specs)
-        if (ps.g->n != 0 && ps.plan.dev.dend >= 3 && sup_form(ps)) {
+        if (ps.g->n != 0 && ps.plan.dev.dend >= 3 && shares_view(ps)) {
             auto r = sup_qdeg.emplace(ps.g, ps.plan.info.min_qdeg);
             r.first->second = std::min(r.first->second, ps.plan.info.min_qdeg);
         }
@@ -4064,6 +4178,12 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         std::vector<int32_t> pair; // first pair of every form, or -1
     };
     std::vector<SupKey> sups;
+    struct RowsKey {
+        View *v;
+        uint32_t shard, nshards, first; // first: the pair that has the items
+        std::vector<int32_t> pair;      // first pair of every form, or -1
+    };
+    std::vector<RowsKey> rows;
     std::vector<uint64_t> sup_m; // entries of each of their views, at most
     for (size_t i = 0; i < specs.size(); ++i) {
         const PairSpec &ps = specs[i];
@@ -4077,7 +4197,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         bool built = false;
         const int32_t form = sup_form(ps);
         int32_t qdeg = ps.plan.info.min_qdeg, asc = ps.plan.dev.asc;
-        if (form) {
+        if (shares_view(ps)) {
             qdeg = sup_qdeg[ps.g];
             asc = 1;
         } else if (asc && !ps.g->views.count({(int)qdeg, 1})) {
@@ -4114,6 +4234,20 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             pd.en.k = ps.en->k;
         }
         uint32_t from = (uint32_t)hp.size();
+        const int rf = form ? -1 : row_form(ps);
+        if (rf >= 0) {
+            pd.pl.asc = asc;
+            size_t k = 0;
+            while (k < rows.size() && !(rows[k].v == v.get() && rows[k].shard == ps.shard && rows[k].nshards == ps.nshards))
+                ++k;
+            if (k == rows.size())
+                rows.push_back(RowsKey{v.get(), ps.shard, ps.nshards, (uint32_t)hp.size(), std::vector<int32_t>(kForms, -1)});
+            else
+                pd.sup = kSupForms; // counted at the first pair's roots
+            if (rows[k].pair[rf] < 0)
+                rows[k].pair[rf] = (int32_t)hp.size();
+            from = (uint32_t)rows[k].pair[rf];
+        }
         if (form) {
             pd.sup = (uint32_t)form;
             pd.pl.asc = 1;
@@ -4155,6 +4289,21 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         }
         if (options & BEEP_OPT_NO_NBHD)
             hp[i].pl.nbhd = kNbNone;
+    }
+    uint32_t any_forms = 0;
+    for (auto &k : rows) {
+        PairDev &pd = hp[k.first];
+        bool every = false; // a form that takes every domain vertex: roots with no later neighbour too
+        for (int f = 0; f < kForms; ++f)
+            if (k.pair[f] >= 0) {
+                pd.fmask |= 1u << f;
+                pd.fcount[f] = hp[k.pair[f]].count;
+                every = every || !(f == kNbPaw || f == kNbDiamond);
+            }
+        if (every)
+            pd.pl.pos1_after_root = 0;
+        pd.pl.rows_needed = 2;
+        any_forms |= pd.fmask;
     }
     BEEP_TRY(lp->alloc(lp->d_pairs, np));
     BEEP_TRY(lp->alloc(lp->d_offs, np + 1));
@@ -4204,8 +4353,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
         std::memcpy(h_misc, ctx->h_pinned, sizeof(h_misc));
     }
-    if (!sups.empty())
-        lp->d_sup_tiers = d_misc + kMiscSup; // read back with the counts
+    for (auto &pd : hp)
+        if (pd.sup)
+            lp->d_sup_tiers = d_misc + kMiscSup; // read back with the counts
     const unsigned *tier_max = h_misc;
     const unsigned *tier_depth = h_misc + kMiscSlots; // [tier * kSlots + slot]
     const unsigned *tiny_depth = h_misc + kMiscTiny;  // [slot]
@@ -4288,8 +4438,16 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
 
     // large tier, one batch planned on the device when every root's bitmap
     // fits the arena at once (the arena words were summed by k_classify)
+    // (what the context's pool holds free is there for the taking; the device's
+    // free memory is a driver call of up to milliseconds, made only beyond it)
     size_t arena_cap = (size_t)256 << 20;
-    if (tier_n[3] > 0 && large_words * 4 > arena_cap) { // the free memory is asked for only when it matters
+    if (tier_n[3] > 0 && large_words * 4 > arena_cap) {
+        uint64_t held = 0, used = 0;
+        if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+            cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
+            arena_cap = std::max<size_t>(arena_cap, std::min<size_t>((size_t)48 << 30, held - used));
+    }
+    if (tier_n[3] > 0 && large_words * 4 > arena_cap) {
         size_t free_b = 0, total_b = 0;
         BEEP_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         arena_cap = std::max<size_t>((size_t)256 << 20, std::min<size_t>((size_t)48 << 30, free_b / 2));
@@ -4300,8 +4458,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     uint32_t wstride = 0;
     {
         // (roots counted in strips need none)
-        if ((tier_depth[3 * kSlots + kWheelSlot] > 0 || tier_depth[3 * kSlots + kNbhdSlot] > 0) &&
-            (tier_max[3] + 31) / 32 > kC4StripMaxW) {
+        if (tier_depth[3 * kSlots + kWheelSlot] > 0 && (tier_max[3] + 31) / 32 > kC4StripMaxW) {
             wstride = (4 * ((tier_max[3] + 31) / 32) + 31) & ~31u;
             const size_t words = (size_t)ctx->num_sms * kLargeDfsBlocksPerSm * 8 * wstride;
             BEEP_TRY(lp->alloc(wsc, words));
@@ -4364,7 +4521,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         lp->recs.push_back(lr);
         if (list_cap((maxD_all + 31) / 32))
             lp->recs.push_back(lists_rec(lr));
-        if (tier_depth[3 * kSlots + kNbhdSlot] > 0)
+        if (any_forms & ~(1u << kFormWheel))
             lp->recs.push_back(nbdeg_rec(lr));
         uint32_t first = 0;
         for (int sl = 0; sl < kSlots; ++sl) {
@@ -4372,9 +4529,37 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             if (!cnt)
                 continue;
             const int d = sl % kDepths;
+            if (d == (int)kWheelSlot) { // a launch per form, over the same rows
+                for (int f = 0; f < kForms; ++f) {
+                    if (!(any_forms >> f & 1u))
+                        continue;
+                    uint32_t *ft = nullptr, *fs = nullptr;
+                    BEEP_TRY(lp->alloc(ft, cnt));
+                    BEEP_TRY(lp->alloc(fs, (size_t)cnt + 1));
+                    k_form_tasks<<<gl, 256, 0, s>>>(lp->d_pairs, list + first, cnt, d_keys + first, f, ft);
+                    BEEP_CUDA_TRY(cudaGetLastError());
+                    st.kernel_launches += 1;
+                    BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, ft, fs + 1, cnt, s));
+                    BEEP_CUDA_TRY(cudaMemsetAsync(fs, 0, 4, s));
+                    LaunchRec ld;
+                    ld.kind = f == kFormWheel ? LaunchRec::kLargeWheel : LaunchRec::kLargeNbhd;
+                    ld.form = f;
+                    ld.dend = d;
+                    ld.grid = ctx->num_sms * kLargeDfsBlocksPerSm;
+                    ld.block = 256;
+                    ld.bt = Batch{list + first, reinterpret_cast<const uint64_t *>(boff) + first, cstart, fs, cnt};
+                    ld.mptr = arena;
+                    BEEP_TRY(cursor(ld.cursor));
+                    ld.sink = &st.large_dfs_ms;
+                    ld.wsc = wsc;
+                    ld.wstride = wstride;
+                    BEEP_TRY(push_walk(ld));
+                }
+                first += cnt;
+                continue;
+            }
             LaunchRec ld;
-            ld.kind = d == (int)kWheelSlot ? LaunchRec::kLargeWheel
-                                           : (d == (int)kNbhdSlot ? LaunchRec::kLargeNbhd : LaunchRec::kLargeDfs);
+            ld.kind = LaunchRec::kLargeDfs;
             ld.dend = d;
             ld.enumerate = sl >= kDepths;
             ld.grid = ctx->num_sms * kLargeDfsBlocksPerSm;
@@ -4395,7 +4580,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         BEEP_TRY(make_list(3, list));
         const uint32_t nl = tier_n[3];
         std::vector<uint64_t> litems(nl);
-        std::vector<uint32_t> lD(nl), lj(nl);
+        std::vector<uint32_t> lD(nl), lj(nl), lsp(nl, 0);
         k_gather_dom<<<std::max(1u, std::min(nl / 256 + 1, 1024u)), 256, 0, s>>>(lp->d_pairs, list, nl, d_keys,
                                                                                d_sel);
         BEEP_CUDA_TRY(cudaGetLastError());
@@ -4403,19 +4588,26 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         BEEP_CUDA_TRY(cudaMemcpyAsync(litems.data(), list, 8ull * nl, cudaMemcpyDeviceToHost, s));
         BEEP_CUDA_TRY(cudaMemcpyAsync(lD.data(), d_keys, 4ull * nl, cudaMemcpyDeviceToHost, s));
         BEEP_CUDA_TRY(cudaMemcpyAsync(lj.data(), d_sel, 4ull * nl, cudaMemcpyDeviceToHost, s));
+        if (any_forms) {
+            k_gather_split<<<std::max(1u, std::min(nl / 256 + 1, 1024u)), 256, 0, s>>>(lp->d_pairs, list, nl, d_sel);
+            BEEP_CUDA_TRY(cudaGetLastError());
+            st.kernel_launches += 1;
+            BEEP_CUDA_TRY(cudaMemcpyAsync(lsp.data(), d_sel, 4ull * nl, cudaMemcpyDeviceToHost, s));
+        }
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
         struct R {
             uint64_t item;
-            uint32_t D, tasks, dend; // dend: the depth slot
+            uint32_t D, j0, dend; // dend: the depth slot
             uint64_t words; // bitmap rows [rlo, D) of D bits and their word lists
+            uint32_t sp;    // later neighbours start here
         };
         std::vector<R> rs(nl);
         for (uint32_t i = 0; i < nl; ++i) {
             const DevPlan &pl = hp[(uint32_t)(litems[i] >> 32)].pl;
             const uint32_t D = lD[i], rlo = pl.rows_needed == 2 ? 0u : (pl.rows_needed == 1 ? lj[i] : D);
-            const uint64_t words = large_root_words(D, rlo, pl.nbhd != kNbNone);
             const PairDev &pdv = hp[(uint32_t)(litems[i] >> 32)];
-            rs[i] = R{litems[i], D, large_tasks(D, lj[i], pl), depth_slot(pl, 4, pdv.en.out != nullptr), words};
+            const uint64_t words = large_root_words(D, rlo, (pdv.fmask & ~(1u << kFormWheel)) != 0);
+            rs[i] = R{litems[i], D, lj[i], depth_slot(pl, 4, pdv.en.out != nullptr), words, lsp[i]};
         }
         std::sort(rs.begin(), rs.end(), [](const R &a, const R &b) { return a.D > b.D; });
         // batch boundaries and the arena size (largest batch)
@@ -4458,12 +4650,22 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 words += rs[i].words;
                 cstart.push_back(cstart.back() + (rs[i].D + kRowsPerChunk - 1) / kRowsPerChunk);
             }
-            std::vector<std::pair<uint32_t, uint32_t>> groups; // (first entry, count) per depth
+            struct Group {
+                uint32_t first, second; // first entry, count
+                int form;               // -1: the plan's walk
+            };
+            std::vector<Group> groups; // per depth, and per form of the roots that take forms
             for (uint32_t a = 0; a < nbt;) {
                 uint32_t b = a;
                 while (b < nbt && rs[i0 + b].dend == rs[i0 + a].dend)
                     ++b;
-                groups.push_back({a, b - a});
+                if (rs[i0 + a].dend == kWheelSlot) {
+                    for (int f = 0; f < kForms; ++f)
+                        if (any_forms >> f & 1u)
+                            groups.push_back({a, b - a, f});
+                } else {
+                    groups.push_back({a, b - a, -1});
+                }
                 a = b;
             }
             std::vector<uint32_t> ts_all, ts_off;
@@ -4473,7 +4675,11 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 ts_all.push_back(0);
                 for (uint32_t e = 0; e < gp.second; ++e) {
                     const R &x = rs[i0 + gp.first + e];
-                    acc += x.tasks;
+                    const PairDev &pdv = hp[(uint32_t)(x.item >> 32)];
+                    if (gp.form < 0)
+                        acc += x.D - x.j0;
+                    else if (pdv.fmask >> gp.form & 1u)
+                        acc += form_tasks(x.D, x.sp, gp.form);
                     ts_all.push_back(acc);
                 }
             }
@@ -4505,19 +4711,16 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             lp->recs.push_back(lr);
             if (list_cap((bmaxD + 31) / 32))
                 lp->recs.push_back(lists_rec(lr));
-            bool any_nbhd = false;
-            for (size_t i = i0; i < i1; ++i)
-                any_nbhd |= rs[i].dend == kNbhdSlot;
-            if (any_nbhd)
+            if (any_forms & ~(1u << kFormWheel))
                 lp->recs.push_back(nbdeg_rec(lr));
             for (size_t gi = 0; gi < groups.size(); ++gi) {
                 LaunchRec ld;
                 const uint32_t slot = rs[i0 + groups[gi].first].dend; // depth slot
                 ld.dend = (int)(slot % kDepths);
                 ld.enumerate = slot >= (uint32_t)kDepths;
-                ld.kind = ld.dend == (int)kWheelSlot
-                              ? LaunchRec::kLargeWheel
-                              : (ld.dend == (int)kNbhdSlot ? LaunchRec::kLargeNbhd : LaunchRec::kLargeDfs);
+                ld.form = groups[gi].form;
+                ld.kind = ld.form < 0 ? LaunchRec::kLargeDfs
+                                      : (ld.form == kFormWheel ? LaunchRec::kLargeWheel : LaunchRec::kLargeNbhd);
                 ld.grid = ctx->num_sms * kLargeDfsBlocksPerSm;
                 ld.block = 256;
                 ld.bt = Batch{d_bitem + groups[gi].first, d_boff + groups[gi].first, d_cs, d_ts + ts_off[gi],
@@ -4809,7 +5012,7 @@ beep_status issue(Ctx *ctx, LaunchPlan *lp, bool timing, bool serial, bool stall
             st.large_encode_launches++;
             break;
         case LaunchRec::kLargeNbhd:
-            k_large_nbhd<<<r.grid, r.block, 0, rs>>>(lp->d_pairs, r.bt, static_cast<const uint32_t *>(r.mptr),
+            k_large_nbhd<<<r.grid, r.block, 0, rs>>>(lp->d_pairs, r.bt, r.form, static_cast<const uint32_t *>(r.mptr),
                                                      r.cursor, r.wsc, r.wstride, ex);
             BEEP_CUDA_TRY(cudaGetLastError());
             st.large_dfs_launches++;
@@ -5543,6 +5746,11 @@ extern "C" beep_status beep_count_noalloc(int device, void *cuda_stream, int64_t
         pd.min_deg = min_deg;
         pd.cap_deg = 0xffffffffu;
         pd.shard_mod = 1;
+        if (pl.wheel4 || pl.nbhd) {
+            const int f = pl.wheel4 ? kFormWheel : pl.nbhd;
+            pd.fmask = 1u << f;
+            pd.fcount[f] = &ctrl->count;
+        }
         pk.offs[1] = (uint64_t)n;
         k_put_pairs<<<8, 256, 0, s>>>(pk, 1, d_pair, d_offs, d_misc);
         BEEP_CUDA_TRY(cudaGetLastError());

@@ -195,8 +195,9 @@ enum {
      * waits for donated work runs out its wait (beep_ctx_set_wait_timeout)
      * and the call returns BEEP_ERR_TIMEOUT. No effect without large roots. */
     BEEP_OPT_WAIT_STALL_TEST = 1u << 6,
-    /* Count the large tier's roots of every query by walking, even where the
-     * plan has a neighbourhood-statistics form (beep_plan_info.nbhd). */
+    /* Count every query by walking, even where the plan has a
+     * neighbourhood-statistics form (beep_plan_info.nbhd) or is counted from
+     * degrees and triangle counts. */
     BEEP_OPT_NO_NBHD = 1u << 7
 };
 
@@ -212,7 +213,8 @@ typedef struct beep_stats {
     int32_t kernel_launches;    /* kernels this call launched */
     double prep_ms;             /* device time: peel + ordering (BEEP_OPT_TIMING) */
     double count_ms;            /* device time: counting kernels */
-    /* per tier (BEEP_OPT_TIMING); large_encode: row builds and word lists,
+    /* per tier (BEEP_OPT_TIMING); small: also the launches of pairs counted from
+     * degrees and triangle counts; large_encode: row builds and word lists,
      * large_dfs: the large tier's walks and 4-wheel kernels */
     double small_ms, medium_ms, large_encode_ms, large_dfs_ms;
     int32_t small_launches, medium_launches, large_encode_launches, large_dfs_launches;
@@ -278,7 +280,9 @@ enum {
 /* Domain-size limits of the kernel tiers a batch plans with (each clamped to
  * its kernel's bound: 16, 64, 256, 1024; defaults 8, 64, 256, 1024), and the
  * large tier's donation threshold. A root whose search domain has D vertices
- * goes to 8-lane groups if D <= tiny_max, warp groups if D <= small_max,
+ * goes to 8-lane groups if D <= tiny_max, warp groups if D <= small_max
+ * (4-cliques at most 48, 5-cliques, the 4-wheel and the statistics 32, larger
+ * cliques 16),
  * thread-walker blocks if D <= med_a_max, warp-walker blocks if D <= med_max,
  * and the global-arena tier above. In the global-arena tier a warp walking a
  * level hands the upper half of its remaining iterations (32 bitmap words
