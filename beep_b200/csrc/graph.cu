@@ -834,13 +834,9 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
     }
     BEEP_CUDA_TRY(cudaGetLastError());
     BEEP_TRY(launch_stats(ctx, d_rp, n));
-    // the graph's own copy, made before the check's result is known
     BEEP_TRY(ctx->grow(g->row_ptr, (size_t)(n + 1) * 4));
-    BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
     if (g->row_ptr.ptr != (const void *)d_rp)
         BEEP_CUDA_TRY(cudaMemcpyAsync(g->row_ptr.ptr, d_rp, (size_t)(n + 1) * 4, cudaMemcpyDeviceToDevice, s));
-    if (m > 0 && g->col.ptr != (const void *)d_col)
-        BEEP_CUDA_TRY(cudaMemcpyAsync(g->col.ptr, d_col, (size_t)m * 4, cudaMemcpyDeviceToDevice, s));
     const unsigned *h32 = reinterpret_cast<const unsigned *>(ctx->h_pinned);
     BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, ctx->counter.ptr, 40, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned + 6, d_rp + n, 4, cudaMemcpyDeviceToHost, s));
@@ -855,6 +851,13 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
     if (!h_bad) {
         const unsigned long long sumsq = ctx->h_pinned[0];
         const uint32_t maxdeg = (uint32_t)ctx->h_pinned[1];
+        // the columns only now: before the check, m may be more entries than
+        // the caller's array holds (or than memory does)
+        BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
+        if (m > 0 && g->col.ptr != (const void *)d_col) {
+            BEEP_CUDA_TRY(cudaMemcpyAsync(g->col.ptr, d_col, (size_t)m * 4, cudaMemcpyDeviceToDevice, s));
+            BEEP_CUDA_TRY(cudaStreamSynchronize(s)); // the caller may free its array on return
+        }
         g->n = n;
         g->m = m;
         set_stats(g, sumsq, maxdeg);
