@@ -1168,12 +1168,12 @@ constexpr int kTinyMaxD = 16;
 // list every root of more than kSplitMinD vertices `parts` times; each part
 // builds the rows again (a small share of its walk) and takes every parts-th
 // chunk of the walk. (6- and 7-cliques there together: 193 -> 31 ms.)
+// walk_parts and the bound of a launch's items it leads to: internal.h
 constexpr uint32_t kSplitMinD = 24;
 // parts of a root of D vertices (of at most `parts`): 8 vertices each
 __device__ __forceinline__ uint32_t root_parts(uint32_t parts, uint32_t D) {
     return parts == 1 || D <= kSplitMinD ? 1u : min(parts, D / 8);
 }
-inline uint32_t walk_parts(int dend, bool enumerate) { return enumerate || dend < 6 ? 1u : (dend == 6 ? 8u : 32u); }
 
 template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigned long long v, unsigned gmask) {
 #pragma unroll
@@ -4760,13 +4760,16 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             r.grid = ctx->num_sms * per_sm;
             r.block = block;
             r.smem = smem;
-            r.items = list + first;
-            r.n = cnt;
             r.maxD = maxD;
-            BEEP_TRY(cursor(r.cursor));
             r.sink = &st.medium_ms;
             r.tail_slot = 1;
-            lp->recs.push_back(r);
+            const uint32_t most = cursor_items(r.parts, (uint32_t)r.grid);
+            for (uint32_t at = 0; at < cnt; at += r.n) { // one launch but for 2^27 roots and more
+                r.items = list + first + at;
+                r.n = std::min(cnt - at, most);
+                BEEP_TRY(cursor(r.cursor));
+                lp->recs.push_back(r);
+            }
             first += cnt;
         }
     }
@@ -5394,6 +5397,8 @@ static_assert(sizeof(NoAllocCtrl) <= kNoAllocCtrlBytes, "control block");
 // rounded up to 64 words) fits the scratch array after the control block.
 constexpr uint64_t noalloc_slice_words(uint64_t D) { return (D * ((D + 31) / 32) + 63) & ~(uint64_t)63; }
 constexpr uint64_t kNoAllocArenaWords = (BEEP_NOALLOC_SCRATCH_BYTES - kNoAllocCtrlBytes) / 4;
+static_assert(kNoAllocArenaWords * 4 / 17 <= cursor_items(walk_parts(kMaxQ, false), 1u << 16),
+              "a medium launch over every vertex of the tiered form");
 static_assert(noalloc_slice_words(BEEP_NOALLOC_MAX_DOMAIN) <= kNoAllocArenaWords &&
                   noalloc_slice_words(BEEP_NOALLOC_MAX_DOMAIN + 1) > kNoAllocArenaWords,
               "BEEP_NOALLOC_MAX_DOMAIN is the largest domain whose bitmap fits the scratch array");

@@ -122,6 +122,13 @@ struct QueryPlan {
 beep_status compile_plan(int32_t qn, const std::vector<int32_t> &qrow_ptr, const std::vector<int32_t> &qcol,
                          beep_mode mode, QueryPlan *out);
 
+// Times a counting launch of the small and medium tiers lists each of its
+// roots (a part of the root's walk each time).
+constexpr uint32_t walk_parts(int dend, bool enumerate) { return enumerate || dend < 6 ? 1u : (dend == 6 ? 8u : 32u); }
+// Items of one medium launch at most: its 32-bit cursor runs over items * parts
+// and every block draws once past the end. Longer lists take several launches.
+constexpr uint32_t cursor_items(uint32_t parts, uint32_t grid) { return (0xffffffffu - grid) / parts; }
+
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------
