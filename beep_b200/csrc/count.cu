@@ -37,6 +37,7 @@
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <set>
 
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -1101,6 +1102,7 @@ struct PairDev {
                                // (kSupForms) at another pair's roots
     uint32_t fmask;            // bit f: form f is counted at this pair's roots; 0: the plan is walked
     unsigned long long *fcount[kForms]; // ... into these pair counters
+    uint32_t c4_up;            // the 4-wheel counts at a cycle's smallest vertex, not its largest
     uint32_t shard_mod;        // > 1: only roots whose input id % shard_mod == shard_rem
     uint32_t shard_rem;
 };
@@ -1185,17 +1187,20 @@ template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigne
 // ---------------------------------------------------------------------------
 // forms counted from shared-memory rows (small and medium tiers)
 // ---------------------------------------------------------------------------
-// Bit-sliced counters. A lane owns one word column (32 domain
-// vertices c) and counts, for one vertex a, the b of row(a) below a whose row
-// holds c -- |row(a) & row(c) below a| for all 32 c at once: slice k of the
-// counters holds bit k of each. Eight row words at a time go through carry-
+// Bit-sliced counters (the carry-save-adder population count, on columns). A
+// lane owns one word column (32 domain vertices c) and counts, for one vertex
+// a, the b of row(a) on one side of a whose row holds c -- |row(a) & row(c)
+// below a| for all 32 c at once: slice k of the counters holds bit k of each. Eight row words at a time go through carry-
 // save adders (two three-input logic instructions each, about 2.5 a word), so
 // the 32 x nb counter increments of a column cost a load and ~2.5 logic
-// instructions per b. The 4-cycles whose largest vertex is a and whose
+// instructions per b. The 4-cycles whose first vertex is a and whose
 // opposite vertex is c number C(count, 2), and every 4-cycle of the
-// neighbourhood graph is counted once, at its largest vertex. Taking the
-// largest vertex keeps the b below a: in the ascending order these are the
-// sparser rows (R-MAT s16 ef28: half the b-c pairs that the smallest gives).
+// neighbourhood graph is counted once, at its largest vertex (b, c below a) or
+// its smallest (up: b, c above a). The side is the one on which the b are few,
+// away from the hubs: below a in a descending view, above it in an ascending
+// one. (CPU count over 60 of the 696 roots above 1,024 vertices of R-MAT s16
+// ef28, ascending: 1.8e6 steps of eight rows, 2.7e8 words and at most 355 b
+// above a, against 3.6e6, 7.6e8 and 4,645 below it.)
 constexpr int kC4MaxSlices = 15; // counts up to 2^15 - 1
 
 __device__ __forceinline__ void c4_csa(uint32_t &carry, uint32_t &sum, uint32_t x, uint32_t y) {
@@ -1246,7 +1251,7 @@ __device__ __forceinline__ unsigned long long c4_pairs(uint32_t (&s)[NS], int L,
 // What the counters of one vertex a are summed into. b runs over row(a), c over
 // the columns; n_c counts the b whose row holds c.
 enum C4Mode : int {
-    kC4Cycles = 0,    // b < a, every c < a: C(n_c, 2), the 4-cycles with largest vertex a
+    kC4Cycles = 0,    // b < a, every c < a (up: > a): C(n_c, 2), the 4-cycles with largest (smallest) vertex a
     kC4Triangles = 1, // b < a, c of row(a) above a: n_c, the triangles whose middle vertex is a
     kC4Paw = 2,       // b < c, both of row(a): n_c, the triangles at a
     kC4Diamond = 3    // every b of row(a), c of row(a) above a: C(n_c, 2) over the edges (a, c)
@@ -1254,16 +1259,20 @@ enum C4Mode : int {
 
 // Masks of one word of row(a) (index k, contents w): the b's in it, the c's.
 template <int MODE>
-__device__ __forceinline__ uint32_t c4_b_bits(uint32_t w, uint32_t k, uint32_t a) {
+__device__ __forceinline__ uint32_t c4_b_bits(uint32_t w, uint32_t k, uint32_t a, bool up) {
     if (MODE == kC4Paw || MODE == kC4Diamond)
         return w;
+    if (MODE == kC4Cycles && up)
+        return k > (a >> 5) ? w : (k == (a >> 5) ? w & ~((2u << (a & 31)) - 1u) : 0u);
     return k < (a >> 5) ? w : (k == (a >> 5) ? w & ((1u << (a & 31)) - 1u) : 0u);
 }
 template <int MODE>
-__device__ __forceinline__ uint32_t c4_c_bits(uint32_t w, uint32_t k, uint32_t a) {
+__device__ __forceinline__ uint32_t c4_c_bits(uint32_t w, uint32_t k, uint32_t a, bool up = false) {
     if (MODE == kC4Paw)
         return w;
     const uint32_t aw = a >> 5;
+    if (MODE == kC4Cycles && up) // (columns beyond the domain are zero in every row)
+        return k > aw ? 0xffffffffu : (k == aw ? ~((2u << (a & 31)) - 1u) : 0u);
     if (MODE == kC4Cycles)
         return k < aw ? 0xffffffffu : (k == aw ? (1u << (a & 31)) - 1u : 0u);
     return k > aw ? w : (k == aw ? w & ~((2u << (a & 31)) - 1u) : 0u);
@@ -1432,11 +1441,11 @@ __device__ __forceinline__ void forms_thread(uint32_t fmask, const uint64_t *row
 // entries of the group's own.
 template <int MODE, int G, int NS>
 __device__ __forceinline__ unsigned long long c4_group(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t a,
-                                                       uint16_t *ib, int glane, unsigned gmask) {
+                                                       uint16_t *ib, int glane, unsigned gmask, bool up = false) {
     const uint32_t k = (uint32_t)glane;
     const uint32_t ra = k < W ? rows[(size_t)a * RS + k] : 0u;
-    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra, k, a) : 0u;
-    const uint32_t nb = c4_indices<G>(c4_b_bits<MODE>(ra, k, a), k, ib, glane, gmask);
+    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra, k, a, up) : 0u;
+    const uint32_t nb = c4_indices<G>(c4_b_bits<MODE>(ra, k, a, up), k, ib, glane, gmask);
     uint32_t s[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i)
@@ -1705,9 +1714,9 @@ __device__ __forceinline__ void nbhd_medium(int form, const uint32_t *rows, uint
     }
 }
 
-// The 4-wheel the same way, the largest (and most connected) vertices first.
+// The 4-wheel the same way, the vertices farthest from the hubs first.
 template <int G, int NS>
-__device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
+__device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D, bool up,
                                              uint32_t *s_misc, uint16_t *ib_all, unsigned long long &cnt) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
@@ -1722,7 +1731,7 @@ __device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, 
         j = __shfl_sync(gm, j, 0, G);
         if (j >= D)
             break;
-        cnt = sat_add(cnt, c4_group<kC4Cycles, G, NS>(rows, RS, W, D - 1 - j, ib, gl, gm));
+        cnt = sat_add(cnt, c4_group<kC4Cycles, G, NS>(rows, RS, W, up ? j : D - 1 - j, ib, gl, gm, up));
     }
 }
 
@@ -2061,7 +2070,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     const int f = __ffs((int)fm) - 1;
                     unsigned long long c = 0, plus = 0, minus = 0;
                     if (f == kFormWheel)
-                        wheel_medium<GG, NS>(rows, RS, RS, D, s_nb, ib, c);
+                        wheel_medium<GG, NS>(rows, RS, RS, D, pairs[cur].c4_up != 0, s_nb, ib, c);
                     else
                         nbhd_medium<GG, NS>(f, rows, RS, RS, D, f == kNbPaw || f == kNbDiamond ? sp : 0u, A, s_nb, ib,
                                             plus, minus);
@@ -2220,7 +2229,7 @@ __host__ __device__ __forceinline__ uint64_t large_root_words(uint32_t D, uint32
 }
 
 // Tasks of a large root for form f: its vertices, or (vertex, strip) pairs.
-__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f);
+__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f, bool up);
 
 __device__ __forceinline__ uint32_t find_batch(const uint32_t *__restrict__ start, uint32_t nb, uint32_t t) {
     // last b with start[b] <= t
@@ -2498,12 +2507,16 @@ __device__ __forceinline__ void wheel4_task(const uint32_t *__restrict__ bm, con
 // Roots whose rows have at most kC4StripMaxW words: the bit-sliced counters of
 // the medium tier (c4_add8) over the arena's rows. A task is (root, a, strip
 // of 32 words): lane k counts column word 32 s + k over every b of row(a)
-// below a. Strips keep the tasks of a hub's neighbourhood short: its largest a
-// have thousands of b and a dozen strips.
-// Task t of a root: strip s holds the a in [1024 s, D), largest first.
-__host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D) {
+// below a. Strips keep the tasks of a hub's neighbourhood short.
+// Task t of a root: strip s holds the a in [1024 s, D), largest first. Counted
+// upwards, the mirror image: strip s is the words [W - 32 (s + 1), W - 32 s)
+// and holds the a below them or in them, smallest first.
+__host__ __device__ __forceinline__ uint32_t c4_strip_rows(uint32_t D, uint32_t s, bool up) {
+    return s == 0 ? D : (up ? (D + 31) & ~31u : D) - 1024 * s;
+}
+__host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D, bool up) {
     const uint32_t S = (D + 1023) / 1024;
-    return S * D - 512 * S * (S - 1);
+    return D + (S - 1) * (up ? (D + 31) & ~31u : D) - 512 * S * (S - 1);
 }
 static_assert((kC4StripMaxW * 32) >> kC4MaxSlices == 0, "a count fits the slices");
 
@@ -2513,9 +2526,9 @@ constexpr uint32_t kPawParts = 4;
 __host__ __device__ __forceinline__ bool nbhd_strips(int nbhd, uint32_t D) {
     return nbhd >= kNbTriIso && (D + 31) / 32 <= kC4StripMaxW;
 }
-__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f) {
+__host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f, bool up) {
     if (f == kFormWheel)
-        return (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D) : D;
+        return (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D, up) : D;
     const uint32_t n = f == kNbPaw || f == kNbDiamond ? D - sp : D;
     return nbhd_strips(f, D) ? n * ((D + 1023) / 1024) * (f == kNbPaw ? kPawParts : 1u) : n;
 }
@@ -2526,12 +2539,13 @@ __host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp,
 template <int MODE>
 __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restrict__ bm, uint32_t W, uint32_t a,
                                                        uint32_t st, uint16_t *ib, int lane, uint32_t part = 0,
-                                                       uint32_t parts = 1) {
+                                                       uint32_t parts = 1, bool up = false) {
     static_assert(MODE >= 0 && MODE <= 3, "a C4Mode");
-    const uint32_t k = 32 * st + (uint32_t)lane;
+    // (the last strip upwards may begin before the row: those k wrap past W)
+    const uint32_t k = (MODE == kC4Cycles && up ? W - 32 * (st + 1) : 32 * st) + (uint32_t)lane;
     const uint32_t kc = min(k, W - 1);
     const uint32_t *ra = bm + (size_t)a * W, *col = bm + kc;
-    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra[k], k, a) : 0u;
+    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra[k], k, a, up) : 0u;
     if (!__ballot_sync(kFull, cm != 0))
         return 0;
     uint32_t s[kC4MaxSlices];
@@ -2539,11 +2553,13 @@ __device__ __forceinline__ unsigned long long c4_strip(const uint32_t *__restric
     for (int i = 0; i < kC4MaxSlices; ++i)
         s[i] = 0;
     uint32_t total = 0;
-    // the b's: all of row(a), below a, or (paw, c > b) up to the strip's last word
-    const uint32_t wend = MODE == kC4Diamond ? W : (MODE == kC4Paw ? min(W, 32 * st + 32) : (a >> 5) + 1);
-    for (uint32_t w0 = 32 * part; w0 < wend; w0 += 32 * parts) {
+    // the b's: all of row(a), below or above a, or (paw, c > b) up to the strip's last word
+    const bool from_a = MODE == kC4Cycles && up;
+    const uint32_t wend =
+        MODE == kC4Diamond || from_a ? W : (MODE == kC4Paw ? min(W, 32 * st + 32) : (a >> 5) + 1);
+    for (uint32_t w0 = (from_a ? a >> 5 : 0u) + 32 * part; w0 < wend; w0 += 32 * parts) {
         const uint32_t wi = w0 + (uint32_t)lane;
-        const uint32_t nb = c4_indices<32>(wi < wend ? c4_b_bits<MODE>(ra[wi], wi, a) : 0u, wi, ib, lane, kFull);
+        const uint32_t nb = c4_indices<32>(wi < wend ? c4_b_bits<MODE>(ra[wi], wi, a, up) : 0u, wi, ib, lane, kFull);
         total += nb;
         c4_add_rows<MODE, kC4MaxSlices>(s, col, W, kc, ib, nb);
         __syncwarp();
@@ -2558,13 +2574,13 @@ constexpr int kStripBlocksPerSm = 4;
 
 // 4-wheel task t of a root.
 __device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, uint32_t W, uint32_t D, uint32_t t,
-                                              uint16_t *ib, int lane, unsigned long long &cnt) {
+                                              bool up, uint16_t *ib, int lane, unsigned long long &cnt) {
     uint32_t st = 0;
-    while (t >= D - 1024 * st) {
-        t -= D - 1024 * st;
+    for (uint32_t n = D; t >= n; n = c4_strip_rows(D, st, up)) {
+        t -= n;
         ++st;
     }
-    cnt = sat_add(cnt, c4_strip<kC4Cycles>(bm, W, D - 1 - t, st, ib, lane));
+    cnt = sat_add(cnt, c4_strip<kC4Cycles>(bm, W, up ? t : D - 1 - t, st, ib, lane, 0, 1, up));
 }
 
 // A donated task of level P resumes the walk at that level over its
@@ -2783,7 +2799,7 @@ __global__ void __launch_bounds__(256, kStripBlocksPerSm) k_large_wheel(const Pa
         const uint32_t W = (D + 31) >> 5;
         const uint32_t *rows = arena + bt.off[b]; // rows of the whole domain: rlo == 0
         if (W <= kC4StripMaxW) {
-            c4_strip_task(rows, W, D, t - bt.tstart[b], s_ib[threadIdx.x >> 5], lane, cnt);
+            c4_strip_task(rows, W, D, t - bt.tstart[b], pairs[p].c4_up != 0, s_ib[threadIdx.x >> 5], lane, cnt);
             continue;
         }
         RowLists rl;
@@ -3802,7 +3818,7 @@ __global__ void k_form_tasks(const PairDev *__restrict__ pairs, const uint64_t *
                              const uint32_t *__restrict__ D_in, int f, uint32_t *tasks) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
         const PairDev &pd = pairs[item_pair(items[i])];
-        tasks[i] = pd.fmask >> f & 1u ? form_tasks(D_in[i], pd.v.split[item_root(items[i])], f) : 0u;
+        tasks[i] = pd.fmask >> f & 1u ? form_tasks(D_in[i], pd.v.split[item_root(items[i])], f, pd.c4_up != 0) : 0u;
     }
 }
 
@@ -4156,16 +4172,30 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         return whole ? ps.plan.dev.support : (int32_t)kSupNone;
     };
     // Pairs counted from a root's rows share their items too, on that view when
-    // they count every root.
+    // they count every root. The 4-wheel joins the statistics forms of its
+    // graph there, counting upwards; alone it keeps its plan's view, and so it
+    // does where a root may be wider than the strips take: the list kernel
+    // works over the neighbours after a cycle's first vertex, which are the
+    // short side only in its plan's descending view (18 times the row entries
+    // on the ascending one, CPU count of a hub of 31,080 on a power-law graph).
+    // (Alone on R-MAT s16 ef28: 8.9 ms at the largest vertex of the ascending
+    // view, 7.5 on its own. 12 power-law graphs x 15 patterns: 10.8 at the
+    // largest vertex, 10.6 upwards, 11.6 on a view and rows of its own.)
     auto row_form = [&](const PairSpec &ps) -> int {
         if (ps.en)
             return -1;
         return ps.plan.dev.wheel4 ? kFormWheel
                                   : (ps.plan.dev.nbhd && !(options & BEEP_OPT_NO_NBHD) ? (int)ps.plan.dev.nbhd : -1);
     };
+    const bool cap = (options & BEEP_OPT_REFERENCE_ROOT_CAP) != 0;
+    std::set<Graph *> statistics; // graphs with a pair that takes a statistics form at every root
+    for (auto &ps : specs)
+        if (row_form(ps) > kFormWheel && !sup_form(ps) && ps.nshards <= 1 && !cap)
+            statistics.insert(ps.g);
     auto shares_view = [&](const PairSpec &ps) {
-        return sup_form(ps) ||
-               (row_form(ps) >= 0 && ps.nshards <= 1 && !(options & BEEP_OPT_REFERENCE_ROOT_CAP));
+        if (row_form(ps) == kFormWheel && !(ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW && statistics.count(ps.g)))
+            return false;
+        return sup_form(ps) || (row_form(ps) >= 0 && ps.nshards <= 1 && !cap);
     };
     std::map<Graph *, int32_t> sup_qdeg; // per graph, the least peel threshold of those pairs
     for (auto &ps : specs)
@@ -4237,6 +4267,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         const int rf = form ? -1 : row_form(ps);
         if (rf >= 0) {
             pd.pl.asc = asc;
+            pd.c4_up = asc;
             size_t k = 0;
             while (k < rows.size() && !(rows[k].v == v.get() && rows[k].shard == ps.shard && rows[k].nshards == ps.nshards))
                 ++k;
@@ -4679,7 +4710,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                     if (gp.form < 0)
                         acc += x.D - x.j0;
                     else if (pdv.fmask >> gp.form & 1u)
-                        acc += form_tasks(x.D, x.sp, gp.form);
+                        acc += form_tasks(x.D, x.sp, gp.form, pdv.c4_up != 0);
                     ts_all.push_back(acc);
                 }
             }

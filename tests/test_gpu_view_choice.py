@@ -1,0 +1,44 @@
+"""Which peeled and ordered view of a graph each pair of a call is counted on: a view that a call has built is cached,
+so asking for it afterwards launches nothing."""
+import pytest
+
+import beep_b200 as B
+from beep_b200 import patterns as P
+from oracle import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def built(ctx, g, min_qdeg, asc):
+    before = ctx.kernel_launches()
+    g.view(min_qdeg, asc)
+    return ctx.kernel_launches() == before
+
+
+@pytest.fixture()
+def graph(ctx):
+    rp, col = synth.chung_lu(3000, 12.0, 2.1, 8)
+    g = B.Graph.from_csr(ctx, rp, col)
+    yield g
+    g.close()
+
+
+def run(ctx, g, queries):
+    b = B.Batch(ctx)
+    for q in queries:
+        b.add(g, q)
+    counts = b.run(B.OPT_NO_GRAPH)
+    b.close()
+    return counts
+
+
+def test_wheel_alone(ctx, graph):
+    """The 4-wheel's plan is a descending one of threshold 3."""
+    B.count(graph, P.W5)
+    assert built(ctx, graph, 3, False)
+
+
+def test_wheel_beside_triangle_forms(ctx, graph):
+    counts = run(ctx, graph, [P.TAILED_TRIANGLE, P.W5])
+    assert built(ctx, graph, 3, False)
+    assert counts == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in (P.TAILED_TRIANGLE, P.W5)]

@@ -37,3 +37,23 @@ def test_hub_neighbourhoods(ctx, n, p, twins):
     g = B.Graph.from_csr(ctx, rp, col)
     assert B.count(g, P.W5) == exp
     g.close()
+
+
+@pytest.mark.parametrize("n,p,twins", [
+    (64, 0.3, True), (96, 0.5, False), (255, 0.1, True), (257, 0.1, True), (1023, 0.01, True), (1025, 0.01, True),
+    (2048, 0.004, True), (2049, 0.004, True), (2079, 0.004, True), (2081, 0.004, True), (16384, 0.0003, True),
+    (16385, 0.0003, True)])
+def test_hub_neighbourhoods_beside_statistics(ctx, n, p, twins):
+    """Beside a statistics form (4-path cone) the 4-wheel is counted from the same rows, at each cycle's smallest
+    vertex, the strips laid out from the row's end; above 16,384 neighbours on its own view."""
+    rp, col = hub_over(n, p, twins, n)
+    g = B.Graph.from_csr(ctx, rp, col)
+    b = B.Batch(ctx)
+    path = P.central_patterns(5)[6]
+    assert B.Query.from_edges(path).plan()["nbhd"] == 4
+    for q in (path, P.W5):
+        b.add(g, q)
+    assert b.run() == [B.count(g, path, B.SGM, B.OPT_NO_NBHD) if n < 2000 else B.count(g, path),
+                       O.count(rp, col, P.W5, apply_root_cap=False)["count"]]
+    b.close()
+    g.close()
