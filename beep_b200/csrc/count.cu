@@ -4171,8 +4171,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         const bool whole = ps.nshards <= 1 && !ps.en && !(options & (BEEP_OPT_REFERENCE_ROOT_CAP | BEEP_OPT_NO_NBHD));
         return whole ? ps.plan.dev.support : (int32_t)kSupNone;
     };
-    // Pairs counted from a root's rows share their items too, on that view when
-    // they count every root. The 4-wheel joins the statistics forms of its
+    // Pairs counted from a root's rows share their items, on an ascending view
+    // too, when they count every root. The 4-wheel joins the statistics forms of its
     // graph there, counting upwards; alone it keeps its plan's view, and so it
     // does where a root may be wider than the strips take: the list kernel
     // works over the neighbours after a cycle's first vertex, which are the
@@ -4192,15 +4192,19 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     for (auto &ps : specs)
         if (row_form(ps) > kFormWheel && !sup_form(ps) && ps.nshards <= 1 && !cap)
             statistics.insert(ps.g);
-    auto shares_view = [&](const PairSpec &ps) {
-        if (row_form(ps) == kFormWheel && !(ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW && statistics.count(ps.g)))
+    auto shares_rows = [&](const PairSpec &ps) {
+        if (row_form(ps) < 0 || sup_form(ps) || ps.nshards > 1 || cap)
             return false;
-        return sup_form(ps) || (row_form(ps) >= 0 && ps.nshards <= 1 && !cap);
+        return row_form(ps) > kFormWheel ||
+               (ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW && statistics.count(ps.g));
     };
-    std::map<Graph *, int32_t> sup_qdeg; // per graph, the least peel threshold of those pairs
+    // Per graph, the least peel threshold of either kind's pairs. Each kind has
+    // its own: a tailed triangle's threshold of 1 in the same call would leave
+    // every hub of the statistics' rows its neighbours of degree 1 and 2.
+    std::map<Graph *, int32_t> sup_qdeg, row_qdeg;
     for (auto &ps : specs)
-        if (ps.g->n != 0 && ps.plan.dev.dend >= 3 && shares_view(ps)) {
-            auto r = sup_qdeg.emplace(ps.g, ps.plan.info.min_qdeg);
+        if (ps.g->n != 0 && ps.plan.dev.dend >= 3 && (sup_form(ps) || shares_rows(ps))) {
+            auto r = (sup_form(ps) ? sup_qdeg : row_qdeg).emplace(ps.g, ps.plan.info.min_qdeg);
             r.first->second = std::min(r.first->second, ps.plan.info.min_qdeg);
         }
     struct SupKey {
@@ -4227,17 +4231,21 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         bool built = false;
         const int32_t form = sup_form(ps);
         int32_t qdeg = ps.plan.info.min_qdeg, asc = ps.plan.dev.asc;
-        if (shares_view(ps)) {
-            qdeg = sup_qdeg[ps.g];
+        if (form || shares_rows(ps)) {
+            qdeg = (form ? sup_qdeg : row_qdeg)[ps.g];
             asc = 1;
         } else if (asc && !ps.g->views.count({(int)qdeg, 1})) {
             // the call's other view of the graph will do when this pair's own
             // would have to be built for it: the vertices that the stronger
             // peel drops are in no match, and whole matches (not prefixes)
             // are counted once in any order
-            auto it = sup_qdeg.find(ps.g);
-            if (it != sup_qdeg.end() && it->second <= qdeg && ps.plan.dev.dend == ps.plan.dev.K)
-                qdeg = it->second;
+            for (auto *m : {&row_qdeg, &sup_qdeg}) {
+                auto it = m->find(ps.g);
+                if (it != m->end() && it->second <= qdeg && ps.plan.dev.dend == ps.plan.dev.K) {
+                    qdeg = it->second;
+                    break;
+                }
+            }
         }
         BEEP_TRY(get_view(ctx, ps.g, qdeg, asc, false, &v, &built));
         built_any = built_any || built;

@@ -42,3 +42,12 @@ def test_wheel_beside_triangle_forms(ctx, graph):
     counts = run(ctx, graph, [P.TAILED_TRIANGLE, P.W5])
     assert built(ctx, graph, 3, False)
     assert counts == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in (P.TAILED_TRIANGLE, P.W5)]
+
+
+def test_statistics_beside_triangle_forms(ctx, graph):
+    """The statistics forms' view is peeled for them alone (thresholds 2 and 3), whatever the triangle forms need."""
+    five = P.central_patterns(5)
+    queries = [P.TAILED_TRIANGLE, five[9], five[7], P.W5]
+    counts = run(ctx, graph, queries)
+    assert built(ctx, graph, 2, True)
+    assert counts == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in queries]
