@@ -4207,6 +4207,10 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             auto r = (sup_form(ps) ? sup_qdeg : row_qdeg).emplace(ps.g, ps.plan.info.min_qdeg);
             r.first->second = std::min(r.first->second, ps.plan.info.min_qdeg);
         }
+    std::set<Graph *> fresh; // graphs without a view yet
+    for (auto &ps : specs)
+        if (ps.g->views.empty() || (options & BEEP_OPT_NO_VIEW_CACHE))
+            fresh.insert(ps.g);
     struct SupKey {
         View *v;
         std::vector<int32_t> pair; // first pair of every form, or -1
@@ -4234,18 +4238,20 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         if (form || shares_rows(ps)) {
             qdeg = (form ? sup_qdeg : row_qdeg)[ps.g];
             asc = 1;
-        } else if (asc && !ps.g->views.count({(int)qdeg, 1})) {
-            // the call's other view of the graph will do when this pair's own
-            // would have to be built for it: the vertices that the stronger
-            // peel drops are in no match, and whole matches (not prefixes)
-            // are counted once in any order
+        } else if (asc && fresh.count(ps.g) && ps.nshards <= 1 && ps.plan.dev.dend == ps.plan.dev.K) {
+            // The call's other view will do on a graph that is counted for the
+            // first time (and perhaps the last: building this pair's own costs
+            // more than the stronger peel saves). The vertices that it drops
+            // are in no match, and whole matches (not prefixes or shards) are
+            // counted once in any order. A graph that comes back gets the
+            // pair's own view, and keeps it.
+            int32_t other = 0;
             for (auto *m : {&row_qdeg, &sup_qdeg}) {
                 auto it = m->find(ps.g);
-                if (it != m->end() && it->second <= qdeg && ps.plan.dev.dend == ps.plan.dev.K) {
-                    qdeg = it->second;
-                    break;
-                }
+                if (it != m->end() && it->second <= qdeg)
+                    other = std::max(other, it->second);
             }
+            qdeg = other ? other : qdeg;
         }
         BEEP_TRY(get_view(ctx, ps.g, qdeg, asc, false, &v, &built));
         built_any = built_any || built;

@@ -51,3 +51,13 @@ def test_statistics_beside_triangle_forms(ctx, graph):
     counts = run(ctx, graph, queries)
     assert built(ctx, graph, 2, True)
     assert counts == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in queries]
+
+
+@pytest.mark.parametrize("shared", [P.TAILED_TRIANGLE, P.central_patterns(5)[6]], ids=["triangle_form", "statistics_form"])
+def test_clique_views_of_a_graph_that_comes_back(ctx, graph, shared):
+    """A first call builds one view for all its patterns; a graph that is counted again gets the cliques' own."""
+    queries = [shared, P.K4, P.K5]
+    first = run(ctx, graph, queries)
+    assert run(ctx, graph, queries) == first
+    assert built(ctx, graph, 3, True) and built(ctx, graph, 4, True)
+    assert first == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in queries]
