@@ -537,7 +537,7 @@ beep_status beep_enumerate(beep_ctx *ctx, beep_graph *g, const beep_query *q, ui
     BEEP_TRY(compile_plan(q->impl.qn, q->impl.row_ptr, q->impl.col, BEEP_MODE_SGM, &p));
     const size_t K = (size_t)p.info.K;
     DevBuf dout;
-    BEEP_TRY(ctx->impl.grow(dout, std::max<uint64_t>(k, 1) * K * 4));
+    BEEP_TRY(ctx->impl.grow_for_call(dout, std::max<uint64_t>(k, 1) * K * 4));
     EnumRequest er;
     er.k = k;
     er.d_out = dout.as<int32_t>();
@@ -552,7 +552,11 @@ beep_status beep_enumerate(beep_ctx *ctx, beep_graph *g, const beep_query *q, ui
         specs[1].en = &er;
     uint64_t counts[2] = {0, 0};
     beep_stats st;
-    BEEP_TRY(run_pairs(&ctx->impl, specs, 0, &st, counts));
+    const beep_status rc = run_pairs(&ctx->impl, specs, 0, &st, counts);
+    if (rc != BEEP_OK) {
+        cudaDeviceSynchronize(); // walks that were launched may still write tuples: dout goes back to the pool
+        return rc;
+    }
     ctx->impl.launches += (uint64_t)st.kernel_launches;
     st.count = counts[0];
     if (st.count == BEEP_COUNT_OVERFLOW) {

@@ -4484,18 +4484,21 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     // large tier, one batch planned on the device when every root's bitmap
     // fits the arena at once (the arena words were summed by k_classify)
     // (what the context's pool holds free is there for the taking; the device's
-    // free memory is a driver call of up to milliseconds, made only beyond it)
-    size_t arena_cap = (size_t)256 << 20;
+    // free memory is a driver call of up to milliseconds, made only beyond it:
+    // half of that comes on top)
+    size_t arena_cap = Ctx::kArenaMin, pool_free = 0;
+    auto raise_cap = [&](size_t b) { arena_cap = std::max(arena_cap, std::min(ctx->arena_limit, b)); };
     if (tier_n[3] > 0 && large_words * 4 > arena_cap) {
         uint64_t held = 0, used = 0;
         if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
             cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
-            arena_cap = std::max<size_t>(arena_cap, std::min<size_t>((size_t)48 << 30, held - used));
+            pool_free = (size_t)(held - used);
+        raise_cap(pool_free);
     }
     if (tier_n[3] > 0 && large_words * 4 > arena_cap) {
         size_t free_b = 0, total_b = 0;
         BEEP_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        arena_cap = std::max<size_t>((size_t)256 << 20, std::min<size_t>((size_t)48 << 30, free_b / 2));
+        raise_cap(pool_free + free_b / 2);
     }
     // scratch of the large tier's 4-wheel tasks: U, its word list, x1's words
     // and U2 (W words each) for every warp of the DFS grid, zero on entry

@@ -702,22 +702,28 @@ struct Carve {
     }
 };
 
-// Scratch of one build from the context's pool, freed in the stream's order.
+// Scratch of one build, from the context's pool and freed in the stream's
+// order, or (above Ctx::kPoolCallBytes) allocated and freed with the build.
 struct PoolBuf {
     Ctx *ctx;
     void *ptr = nullptr;
+    bool pooled = true;
     explicit PoolBuf(Ctx *c) : ctx(c) {}
     PoolBuf(const PoolBuf &) = delete;
     PoolBuf &operator=(const PoolBuf &) = delete;
     ~PoolBuf() {
-        if (ptr)
+        if (ptr && pooled)
             cudaFreeAsync(ptr, ctx->stream);
+        else if (ptr)
+            cudaFree(ptr); // waits for the device
     }
     beep_status reserve(size_t bytes) {
-        cudaError_t e = cudaMallocFromPoolAsync(&ptr, std::max<size_t>(bytes, 16), ctx->pool, ctx->stream);
+        pooled = bytes <= Ctx::kPoolCallBytes;
+        cudaError_t e = pooled ? cudaMallocFromPoolAsync(&ptr, std::max<size_t>(bytes, 16), ctx->pool, ctx->stream)
+                               : cudaMalloc(&ptr, bytes);
         if (e != cudaSuccess) {
             ptr = nullptr;
-            return fail(BEEP_ERR_OUT_OF_MEMORY, "device pool allocation of " + std::to_string(bytes) +
+            return fail(BEEP_ERR_OUT_OF_MEMORY, "device allocation of " + std::to_string(bytes) +
                                                     " bytes: " + cudaGetErrorString(e));
         }
         return BEEP_OK;

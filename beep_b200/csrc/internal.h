@@ -256,6 +256,17 @@ struct Ctx {
     cudaMemPool_t pool = nullptr; // stream-ordered pool for per-call buffers
     // grow b (a buffer of this context or of an object it builds) from the pool on the context's stream
     beep_status grow(DevBuf &b, size_t bytes) { return b.reserve(bytes, pool, stream); }
+    // The pool keeps what it once held. A buffer of one call whose size the
+    // caller's input sets (edge keys, tuples) comes from it up to this size;
+    // larger ones go back to the device with the call, which an allocation of
+    // about a millisecond does not slow down much.
+    static constexpr size_t kPoolCallBytes = (size_t)64 << 20;
+    beep_status grow_for_call(DevBuf &b, size_t bytes) {
+        return bytes <= kPoolCallBytes ? grow(b, bytes) : b.reserve(bytes);
+    }
+    // most that the large tier's bitmap arena may take (plan_pairs)
+    static constexpr size_t kArenaMin = (size_t)256 << 20, kArenaMax = (size_t)48 << 30;
+    size_t arena_limit = kArenaMax;
     // side streams and events that let the kernel tiers of one call overlap
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};

@@ -124,11 +124,11 @@ struct Server {
     // Device bytes a request can take while its batch runs: its tuple buffer,
     // the planning arrays over its graph's vertices and entries, and the
     // large tier's bitmap arena -- at most the dense bitmaps of all the
-    // graph's roots of degree above 1024, and never more than the arena cap
-    // that planning applies (min(48 GiB, half the free memory)).
+    // graph's roots of degree above 1024, and never more than the limit that
+    // the server sets for its planning (half the budget, at most 48 GiB).
     uint64_t estimate(const Request &r) const {
         const Graph *g = graphs[r.graph];
-        const uint64_t arena = std::min<uint64_t>(graph_large_bytes[r.graph], std::min<uint64_t>(48ull << 30, budget / 2));
+        const uint64_t arena = std::min<uint64_t>(graph_large_bytes[r.graph], ctx.arena_limit);
         return (uint64_t)r.k * (uint64_t)r.plan.info.K * 4ull + (uint64_t)g->n * 64ull + (uint64_t)g->m * 4ull +
                arena;
     }
@@ -414,6 +414,7 @@ beep_status beep_serve_create(beep_ctx *ctx, const beep_serve_options *opt, beep
             return fail(BEEP_ERR_CUDA, std::string("server setup: ") + cudaGetErrorString(e));
         }
         S.budget = free_b > S.reserve ? free_b - S.reserve : 0;
+        S.ctx.arena_limit = std::max<size_t>(Ctx::kArenaMin, std::min<size_t>(Ctx::kArenaMax, S.budget / 2));
     }
     S.thr = std::thread([&S] { S.loop(); });
     *out = s;
