@@ -3610,8 +3610,8 @@ constexpr uint32_t kMiscSlots = 8, kMiscTiny = 120, kMiscLarge = 144, kMiscSup =
 static_assert(kMiscSlots + kTiers * kSlots <= kMiscTiny && kMiscTiny + kSlots <= kMiscLarge, "planning block");
 constexpr uint32_t kMiscWords = kMiscBuckets + kBuckets;
 
-// Largest domain of a plan's roots that the small tier takes (at most; the
-// call's limits may be lower). A warp builds such a root's rows with dependent
+// Largest domain of a plan's roots that the small tier takes where the call
+// leaves it at the tier's bound (a lower limit is taken as it is). A warp builds such a root's rows with dependent
 // loads: near 64 vertices that takes as long as a launch's whole small tier,
 // and a block of the medium tier does it sooner. Counting calls, ms with the
 // limit at 64 / 48 / 32: 4-cliques on a power-law graph of 100,003 vertices
@@ -3665,7 +3665,8 @@ __global__ void __launch_bounds__(256) k_classify(const PairDev *__restrict__ pa
                 D -= j0; // level-1 tasks of the list walker
             }
         } else if (root_ok && D + 1 >= (uint32_t)pd.pl.dend) {
-            const uint32_t smax = min(cfg.small_max, small_limit(pd.pl, pd.en.out != nullptr));
+            const uint32_t smax =
+                cfg.small_max < kSmallMaxD ? cfg.small_max : small_limit(pd.pl, pd.en.out != nullptr);
             tc = D <= smax ? 1 : (D <= cfg.med_a_max ? 2 : (D <= cfg.med_max ? 3 : 4));
         }
         tier[t] = (uint8_t)tc;

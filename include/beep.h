@@ -280,9 +280,9 @@ enum {
 /* Domain-size limits of the kernel tiers a batch plans with (each clamped to
  * its kernel's bound: 16, 64, 256, 1024; defaults 8, 64, 256, 1024), and the
  * large tier's donation threshold. A root whose search domain has D vertices
- * goes to 8-lane groups if D <= tiny_max, warp groups if D <= small_max
- * (4-cliques at most 48, 5-cliques, the 4-wheel and the statistics 32, larger
- * cliques 16),
+ * goes to 8-lane groups if D <= tiny_max, warp groups if D <= small_max (left
+ * at 64, counts take less by their plan: 4-cliques 48, 5-cliques, the 4-wheel
+ * and the statistics 32, larger cliques 16; a lower limit is taken as it is),
  * thread-walker blocks if D <= med_a_max, warp-walker blocks if D <= med_max,
  * and the global-arena tier above. In the global-arena tier a warp walking a
  * level hands the upper half of its remaining iterations (32 bitmap words

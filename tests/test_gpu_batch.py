@@ -129,3 +129,21 @@ def test_batch_with_hub_roots_equals_plain_loop(ctx):
     batch.close()
     for g in graphs:
         g.close()
+
+
+def test_small_limit_of_the_caller(ctx):
+    """A limit below the tier's bound decides alone which roots the small tier takes; at the bound the plan's does."""
+    rp, col = B.gen_erdos_renyi(600, 0.15, 4)  # 90 neighbours a vertex, 0 to 90 of them later ones
+    g = B.Graph.from_csr(ctx, rp, col)
+    exp = O.count(rp, col, P.K5, apply_root_cap=False)["count"]
+    roots = {}
+    for small_max in (16, 32, 48, 60, 64):
+        b = B.Batch(ctx)
+        b.add(g, P.K5)
+        b.set_tiers(dict(tiny_max=8, small_max=small_max, med_a_max=256, med_max=1024))
+        counts, st = b.run(B.OPT_NO_GRAPH, stats=True)
+        roots[small_max] = st["roots_small"]
+        assert counts == [exp]
+        b.close()
+    assert roots[16] < roots[32] == roots[64] < roots[48] < roots[60]
+    g.close()
