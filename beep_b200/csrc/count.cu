@@ -923,7 +923,7 @@ __device__ __forceinline__ void build_rows_flat(const ViewDev &v, int asc, const
 // ---------------------------------------------------------------------------
 constexpr uint32_t kHashEmpty = 0xffffffffu;
 
-__host__ __device__ __forceinline__ uint32_t hash_slots(uint32_t maxD) {
+__host__ __device__ constexpr uint32_t hash_slots(uint32_t maxD) {
     uint32_t s = 64;
     while (s < 8 * maxD)
         s <<= 1;
@@ -1285,7 +1285,7 @@ template <int MODE> __device__ __forceinline__ uint32_t c4_input(uint32_t w, uin
     return k > bw ? w : (k == bw ? w & ~((2u << (b & 31)) - 1u) : 0u);
 }
 // 16-bit entries of a group's index list: D, in 16-byte steps.
-__host__ __device__ __forceinline__ uint32_t c4_list(uint32_t D) { return (D + 7) & ~7u; }
+__host__ __device__ constexpr uint32_t c4_list(uint32_t D) { return (D + 7) & ~7u; }
 
 // Appends the set bits of this lane's word w (word index k) to ib in order,
 // group-wide (G lanes, mask gmask); returns the group's total.
@@ -1941,6 +1941,20 @@ __device__ __forceinline__ void clique_root(const uint32_t *rows, uint32_t RS, u
     }
 }
 
+// The forms counted from rows put their groups' index lists (32 groups a block
+// in either sub-tier, c4_list(D) 16-bit entries each) where the row builder had
+// its three arrays of `pad` words and the domain hash: just large enough.
+constexpr uint32_t kMediumGroups = 32;
+constexpr bool medium_lists_fit() {
+    for (uint32_t D = 4; D <= (uint32_t)kMediumMaxD; ++D) { // five-vertex forms: four neighbours and more
+        const uint32_t pad = (D + 4) & ~3u, nslots = hash_slots(D);
+        if (kMediumGroups * c4_list(D) / 2 > 3 * pad + nslots + nslots / 2 + nslots / 4)
+            return false;
+    }
+    return true;
+}
+static_assert(medium_lists_fit(), "the index lists would run into the rows");
+
 // ---------------------------------------------------------------------------
 // medium tier: block per root, bitmap in shared memory
 // ---------------------------------------------------------------------------
@@ -2060,10 +2074,10 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                 // groups of 8 lanes (rows of 8 words) or a warp take the
                 // vertices of one form after the other. The domain list's
                 // place takes the degrees, the row builder's arrays (free
-                // again) the groups' index lists: (3 pad + 1.75 nslots) words
-                // hold 64 bytes a vertex, D rounded up to 8
+                // again) the groups' index lists (medium_lists_fit)
                 constexpr int GG = G == 0 ? 8 : 32, NS = G == 0 ? 9 : 11;
                 static_assert(2 * kThreadNW == 8, "8 words a row");
+                static_assert((G == 0 ? 256 : 1024) / GG == kMediumGroups, "index lists");
                 const uint32_t RS = G == 0 ? 8u : W, sp = pr.v.split[r];
                 uint16_t *ib = reinterpret_cast<uint16_t *>(s_hb);
                 for (uint32_t fm = fmask; fm; fm &= fm - 1) {
