@@ -1632,8 +1632,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, DEND <= 4 ? 5 : 1) k_small(c
 // Block-wide (block-uniform call); s_deg: D words, s_misc: 2 words.
 // ---------------------------------------------------------------------------
 // Degrees of rows[0, D) into s_deg and their sum into s_misc[0]; a warp per
-// row (rw words of 32 bits, at most 32), or a thread per row (rw > 32 words
-// never occur here: the thread sub-tier's rows are 8 words).
+// row (rw words of 32 bits, at most 32).
 __device__ __forceinline__ void nbhd_degrees(const uint32_t *rows, uint32_t rw, uint32_t D, uint32_t *s_deg,
                                              uint32_t *s_misc) {
     const int lane = threadIdx.x & 31;
@@ -4064,23 +4063,23 @@ static int large_rows_grid(const Ctx *ctx, size_t smemA) {
 }
 
 // The degree pass of the neighbourhood-statistics roots a kLargeRows record builds.
-static LaunchRec nbdeg_rec(const LaunchRec &rows) {
+static LaunchRec nbdeg_rec(const Ctx *ctx, const LaunchRec &rows) {
     LaunchRec r = rows;
     r.kind = LaunchRec::kLargeNbDeg;
     r.block = 256;
     r.smem = 0;
-    r.grid = std::max(rows.grid, 592); // whole SMs' worth of 256-thread blocks
+    r.grid = std::max(rows.grid, 4 * ctx->num_sms); // of 256 threads
     r.cursor = nullptr;
     return r;
 }
 
 // The list pass over the rows a kLargeRows record builds.
-static LaunchRec lists_rec(const LaunchRec &rows) {
+static LaunchRec lists_rec(const Ctx *ctx, const LaunchRec &rows) {
     LaunchRec r = rows;
     r.kind = LaunchRec::kLargeLists;
     r.block = 256;
     r.smem = 0;
-    r.grid = std::max(rows.grid, 592); // whole SMs' worth of 256-thread blocks
+    r.grid = std::max(rows.grid, 4 * ctx->num_sms); // of 256 threads
     r.cursor = nullptr;
     return r;
 }
@@ -4583,9 +4582,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         lr.sink = &st.large_encode_ms;
         lp->recs.push_back(lr);
         if (list_cap((maxD_all + 31) / 32))
-            lp->recs.push_back(lists_rec(lr));
+            lp->recs.push_back(lists_rec(ctx, lr));
         if (any_forms & ~(1u << kFormWheel))
-            lp->recs.push_back(nbdeg_rec(lr));
+            lp->recs.push_back(nbdeg_rec(ctx, lr));
         uint32_t first = 0;
         for (int sl = 0; sl < kSlots; ++sl) {
             const uint32_t cnt = tier_depth[3 * kSlots + sl];
@@ -4773,9 +4772,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             lr.sink = &st.large_encode_ms;
             lp->recs.push_back(lr);
             if (list_cap((bmaxD + 31) / 32))
-                lp->recs.push_back(lists_rec(lr));
+                lp->recs.push_back(lists_rec(ctx, lr));
             if (any_forms & ~(1u << kFormWheel))
-                lp->recs.push_back(nbdeg_rec(lr));
+                lp->recs.push_back(nbdeg_rec(ctx, lr));
             for (size_t gi = 0; gi < groups.size(); ++gi) {
                 LaunchRec ld;
                 const uint32_t slot = rs[i0 + groups[gi].first].dend; // depth slot

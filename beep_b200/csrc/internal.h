@@ -74,7 +74,7 @@ struct DevPlan {
     uint32_t adj0;           // bit p: position p is adjacent to position 0
     uint32_t sym0;           // bit p: position p must follow position 0
     int32_t wheel4;          // the 4-wheel's plan: counted per (x1, x3) pair in closed form
-    int32_t nbhd;            // NbhdForm: in the large tier, counted from neighbourhood statistics
+    int32_t nbhd;            // NbhdForm: counted from statistics of the root's neighbourhood graph
     int32_t support;         // SupForm: counted from degrees and triangle counts
     int32_t clique;          // a complete query, every position ordered after the ones before it
 };

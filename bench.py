@@ -536,7 +536,8 @@ def serial_phases(B, step, timed, steps) -> dict:
     # dominant kernel of the counting phase: its algorithmic bytes (4 * (deg r
     # + sum of the neighbours' degrees) per searched root, on the input CSR)
     # and the adjacency bytes it actually has to read (its own model)
-    tiers = {"small": ("small_ms", "alg_small_bytes", "small_bytes", "small_launches", "k_small"),
+    tiers = {"small": ("small_ms", "alg_small_bytes", "small_bytes", "small_launches",
+                       "k_small and k_sup_*"),  # pairs counted from triangle counts report in the small tier
              "medium": ("medium_ms", "alg_medium_bytes", "medium_bytes", "medium_launches", "k_medium"),
              "large_dfs": ("large_dfs_ms", "alg_large_bytes", "large_bytes", "large_dfs_launches", "k_large_dfs"),
              "large_rows": ("large_encode_ms", "alg_large_bytes", "large_bytes", "large_encode_launches",
@@ -571,7 +572,8 @@ def serial_phases(B, step, timed, steps) -> dict:
                      "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured"
                      else "fallback 6650 GB/s",
                      "bytes_per_launch": dom_bytes / max(dom_launches, 1),
-                     "bytes_def": "algorithmic: 4*(deg r + sum of deg v over N(r)) per searched root, input CSR",
+                     "bytes_def": "algorithmic: 4*(deg r + sum of deg v over N(r)) per searched root (of every pair, those "
+                                  "counted from triangle counts included), input CSR",
                      "read_model_bytes_per_launch": dom_read / max(dom_launches, 1),
                      "ms_per_launch": dom_ms / max(dom_launches, 1),
                      "timing": "per-launch CUDA events in steps with the kernel tiers serialised"},

@@ -166,8 +166,8 @@ typedef struct beep_plan_info {
                               last position) */
     int32_t wheel4;        /* 1: the 4-wheel's plan (positions 1-4 a 4-cycle around the
                               root); counts are summed once per (x1, x3) pair in closed form */
-    int32_t nbhd;          /* > 0: a five-vertex query counted at the large tier's roots from
-                              statistics of the root's neighbourhood graph (degrees, edges,
+    int32_t nbhd;          /* > 0: a five-vertex query counted from statistics of each root's
+                              neighbourhood graph (degrees, edges,
                               common neighbours per edge); 1 wedge + isolated vertex, 2 two
                               disjoint edges, 3 triangle + isolated vertex, 4 path, 5 paw,
                               6 diamond (the query minus its root) */
@@ -195,9 +195,9 @@ enum {
      * waits for donated work runs out its wait (beep_ctx_set_wait_timeout)
      * and the call returns BEEP_ERR_TIMEOUT. No effect without large roots. */
     BEEP_OPT_WAIT_STALL_TEST = 1u << 6,
-    /* Count every query by walking, even where the plan has a
-     * neighbourhood-statistics form (beep_plan_info.nbhd) or is counted from
-     * degrees and triangle counts. */
+    /* Count by walking where the plan has a neighbourhood-statistics form
+     * (beep_plan_info.nbhd) or is counted from degrees and triangle counts.
+     * (The 4-wheel and cliques keep their own counting.) */
     BEEP_OPT_NO_NBHD = 1u << 7
 };
 
