@@ -117,6 +117,15 @@ __global__ void k_check_chunks(const uint32_t *__restrict__ rp, const uint32_t *
         atomicOr(bad, flag);
 }
 
+// The caller's columns: m entries, but none beyond the last row pointer (an m
+// that says more is refused only after this ran).
+__global__ void k_copy_columns(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ col, int64_t n, int64_t m,
+                               uint32_t *__restrict__ out) {
+    const int64_t e = min(m, (int64_t)rp[n]), step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < e; i += step)
+        out[i] = col[i];
+}
+
 // Edge keys (src << bits | dst), ids below 2^bits; self loops become the
 // largest value of 2 bits bits (itself a loop, so no edge has it), which sorts
 // last. flags[0] |= 1: a loop, 2: an id that does not fit.
@@ -843,6 +852,18 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
     BEEP_TRY(ctx->grow(g->row_ptr, (size_t)(n + 1) * 4));
     if (g->row_ptr.ptr != (const void *)d_rp)
         BEEP_CUDA_TRY(cudaMemcpyAsync(g->row_ptr.ptr, d_rp, (size_t)(n + 1) * 4, cudaMemcpyDeviceToDevice, s));
+    // Up to Ctx::kPoolCallBytes of columns are copied before the check's result
+    // is known, so that its wait is the build's only one (step on a graph of
+    // 4,096 vertices: 242 us with a second one, 236 without); more wait for it,
+    // since m may say more than there is room for.
+    const bool own_col = m == 0 || g->col.ptr == (const void *)d_col;
+    const bool early = !own_col && (size_t)m * 4 <= Ctx::kPoolCallBytes;
+    if (early) {
+        BEEP_TRY(ctx->grow(g->col, (size_t)m * 4));
+        k_copy_columns<<<grid_for(m, 256, ctx->num_sms), 256, 0, s>>>(d_rp, d_col, n, m, g->col.as<uint32_t>());
+        ++ctx->launches;
+        BEEP_CUDA_TRY(cudaGetLastError());
+    }
     const unsigned *h32 = reinterpret_cast<const unsigned *>(ctx->h_pinned);
     BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, ctx->counter.ptr, 40, cudaMemcpyDeviceToHost, s));
     BEEP_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned + 6, d_rp + n, 4, cudaMemcpyDeviceToHost, s));
@@ -857,10 +878,8 @@ beep_status graph_build_from_device_csr(Ctx *ctx, Graph *g, int64_t n, int64_t m
     if (!h_bad) {
         const unsigned long long sumsq = ctx->h_pinned[0];
         const uint32_t maxdeg = (uint32_t)ctx->h_pinned[1];
-        // the columns only now: before the check, m may be more entries than
-        // the caller's array holds (or than memory does)
         BEEP_TRY(ctx->grow(g->col, (size_t)(m > 0 ? m : 1) * 4));
-        if (m > 0 && g->col.ptr != (const void *)d_col) {
+        if (!own_col && !early) {
             BEEP_CUDA_TRY(cudaMemcpyAsync(g->col.ptr, d_col, (size_t)m * 4, cudaMemcpyDeviceToDevice, s));
             BEEP_CUDA_TRY(cudaStreamSynchronize(s)); // the caller may free its array on return
         }
