@@ -1102,7 +1102,7 @@ struct PairDev {
                                // (kSupForms) at another pair's roots
     uint32_t fmask;            // bit f: form f is counted at this pair's roots; 0: the plan is walked
     unsigned long long *fcount[kForms]; // ... into these pair counters
-    uint32_t c4_up;            // the 4-wheel counts at a cycle's smallest vertex, not its largest
+    uint32_t c4_up;            // the 4-wheel's strips count at a cycle's smallest vertex, not its largest
     uint32_t shard_mod;        // > 1: only roots whose input id % shard_mod == shard_rem
     uint32_t shard_rem;
 };
@@ -1196,11 +1196,11 @@ template <int G> __device__ __forceinline__ unsigned long long group_sum(unsigne
 // instructions per b. The 4-cycles whose first vertex is a and whose
 // opposite vertex is c number C(count, 2), and every 4-cycle of the
 // neighbourhood graph is counted once, at its largest vertex (b, c below a) or
-// its smallest (up: b, c above a). The side is the one on which the b are few,
-// away from the hubs: below a in a descending view, above it in an ascending
-// one. (CPU count over 60 of the 696 roots above 1,024 vertices of R-MAT s16
-// ef28, ascending: 1.8e6 steps of eight rows, 2.7e8 words and at most 355 b
-// above a, against 3.6e6, 7.6e8 and 4,645 below it.)
+// its smallest (up: b, c above a). The large tier's strips take the side on
+// which the b are few, away from the hubs: below a in a descending view, above
+// it in an ascending one. (CPU count over 60 of the 696 roots above 1,024
+// vertices of R-MAT s16 ef28, ascending: 1.8e6 steps of eight rows, 2.7e8 words
+// and at most 355 b above a, against 3.6e6, 7.6e8 and 4,645 below it.)
 constexpr int kC4MaxSlices = 15; // counts up to 2^15 - 1
 
 __device__ __forceinline__ void c4_csa(uint32_t &carry, uint32_t &sum, uint32_t x, uint32_t y) {
@@ -1259,7 +1259,7 @@ enum C4Mode : int {
 
 // Masks of one word of row(a) (index k, contents w): the b's in it, the c's.
 template <int MODE>
-__device__ __forceinline__ uint32_t c4_b_bits(uint32_t w, uint32_t k, uint32_t a, bool up) {
+__device__ __forceinline__ uint32_t c4_b_bits(uint32_t w, uint32_t k, uint32_t a, bool up = false) {
     if (MODE == kC4Paw || MODE == kC4Diamond)
         return w;
     if (MODE == kC4Cycles && up)
@@ -1441,11 +1441,11 @@ __device__ __forceinline__ void forms_thread(uint32_t fmask, const uint64_t *row
 // entries of the group's own.
 template <int MODE, int G, int NS>
 __device__ __forceinline__ unsigned long long c4_group(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t a,
-                                                       uint16_t *ib, int glane, unsigned gmask, bool up = false) {
+                                                       uint16_t *ib, int glane, unsigned gmask) {
     const uint32_t k = (uint32_t)glane;
     const uint32_t ra = k < W ? rows[(size_t)a * RS + k] : 0u;
-    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra, k, a, up) : 0u;
-    const uint32_t nb = c4_indices<G>(c4_b_bits<MODE>(ra, k, a, up), k, ib, glane, gmask);
+    const uint32_t cm = k < W ? c4_c_bits<MODE>(ra, k, a) : 0u;
+    const uint32_t nb = c4_indices<G>(c4_b_bits<MODE>(ra, k, a), k, ib, glane, gmask);
     uint32_t s[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i)
@@ -1713,9 +1713,13 @@ __device__ __forceinline__ void nbhd_medium(int form, const uint32_t *rows, uint
     }
 }
 
-// The 4-wheel the same way, the vertices farthest from the hubs first.
+// The 4-wheel the same way. A group holds every column, so both sides cost the
+// same row reads, one for every edge: the largest vertex counts, in an
+// ascending view the hubs' side, where the reads come from few vertices with
+// many b, in whole steps of eight (upwards: 214 us a launch against 193 on
+// R-MAT s11 ef28), and the hubs come first.
 template <int G, int NS>
-__device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D, bool up,
+__device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, uint32_t W, uint32_t D,
                                              uint32_t *s_misc, uint16_t *ib_all, unsigned long long &cnt) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned gm = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
@@ -1730,7 +1734,7 @@ __device__ __forceinline__ void wheel_medium(const uint32_t *rows, uint32_t RS, 
         j = __shfl_sync(gm, j, 0, G);
         if (j >= D)
             break;
-        cnt = sat_add(cnt, c4_group<kC4Cycles, G, NS>(rows, RS, W, up ? j : D - 1 - j, ib, gl, gm, up));
+        cnt = sat_add(cnt, c4_group<kC4Cycles, G, NS>(rows, RS, W, D - 1 - j, ib, gl, gm));
     }
 }
 
@@ -2083,7 +2087,7 @@ __global__ void __launch_bounds__(G == 0 ? 256 : 1024, G == 0 ? (DEND <= 5 ? 4 :
                     const int f = __ffs((int)fm) - 1;
                     unsigned long long c = 0, plus = 0, minus = 0;
                     if (f == kFormWheel)
-                        wheel_medium<GG, NS>(rows, RS, RS, D, pairs[cur].c4_up != 0, s_nb, ib, c);
+                        wheel_medium<GG, NS>(rows, RS, RS, D, s_nb, ib, c);
                     else
                         nbhd_medium<GG, NS>(f, rows, RS, RS, D, f == kNbPaw || f == kNbDiamond ? sp : 0u, A, s_nb, ib,
                                             plus, minus);
@@ -2521,9 +2525,10 @@ __device__ __forceinline__ void wheel4_task(const uint32_t *__restrict__ bm, con
 // the medium tier (c4_add8) over the arena's rows. A task is (root, a, strip
 // of 32 words): lane k counts column word 32 s + k over every b of row(a)
 // below a. Strips keep the tasks of a hub's neighbourhood short.
-// Task t of a root: strip s holds the a in [1024 s, D), largest first. Counted
+// Task t of a root: strip s holds the a in [1024 s, D), smallest first. Counted
 // upwards, the mirror image: strip s is the words [W - 32 (s + 1), W - 32 s)
-// and holds the a below them or in them, smallest first.
+// and holds the a below them or in them, largest first (the hubs' end: as in
+// wheel_medium).
 __host__ __device__ __forceinline__ uint32_t c4_strip_rows(uint32_t D, uint32_t s, bool up) {
     return s == 0 ? D : (up ? (D + 31) & ~31u : D) - 1024 * s;
 }
@@ -2589,11 +2594,12 @@ constexpr int kStripBlocksPerSm = 4;
 __device__ __forceinline__ void c4_strip_task(const uint32_t *__restrict__ bm, uint32_t W, uint32_t D, uint32_t t,
                                               bool up, uint16_t *ib, int lane, unsigned long long &cnt) {
     uint32_t st = 0;
-    for (uint32_t n = D; t >= n; n = c4_strip_rows(D, st, up)) {
+    uint32_t n = D;
+    for (; t >= n; n = c4_strip_rows(D, st, up)) {
         t -= n;
         ++st;
     }
-    cnt = sat_add(cnt, c4_strip<kC4Cycles>(bm, W, up ? t : D - 1 - t, st, ib, lane, 0, 1, up));
+    cnt = sat_add(cnt, c4_strip<kC4Cycles>(bm, W, up ? n - 1 - t : D - n + t, st, ib, lane, 0, 1, up));
 }
 
 // A donated task of level P resumes the walk at that level over its
@@ -4186,15 +4192,17 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         return whole ? ps.plan.dev.support : (int32_t)kSupNone;
     };
     // Pairs counted from a root's rows share their items, on an ascending view
-    // too, when they count every root. The 4-wheel joins the statistics forms of its
-    // graph there, counting upwards; alone it keeps its plan's view, and so it
-    // does where a root may be wider than the strips take: the list kernel
-    // works over the neighbours after a cycle's first vertex, which are the
-    // short side only in its plan's descending view (18 times the row entries
-    // on the ascending one, CPU count of a hub of 31,080 on a power-law graph).
-    // (Alone on R-MAT s16 ef28: 8.9 ms at the largest vertex of the ascending
-    // view, 7.5 on its own. 12 power-law graphs x 15 patterns: 10.8 at the
-    // largest vertex, 10.6 upwards, 11.6 on a view and rows of its own.)
+    // too, when they count every root: the later lists that rows are built from
+    // are short there. Where a root may be wider than the strips take, the
+    // 4-wheel keeps its plan's descending view: the list kernel works over the
+    // neighbours after a cycle's first vertex, which are the short side only
+    // there (18 times the row entries on the ascending one, CPU count of a hub
+    // of 31,080 on a power-law graph; served workload of 32 graphs of up to
+    // 10^7 edges: 90.6 s on it, 50.2 s on its own).
+    // (4-wheels of R-MAT s16 ef28: strips downwards 8.9 ms, on the descending
+    // view 7.4, upwards 7.35; s11 ef28: 268, 275 and 266 us. 12 power-law graphs
+    // x 15 patterns: 10.8 ms downwards, 10.6 upwards, 11.6 on a view and rows
+    // of its own.)
     auto row_form = [&](const PairSpec &ps) -> int {
         if (ps.en)
             return -1;
@@ -4202,15 +4210,10 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                                   : (ps.plan.dev.nbhd && !(options & BEEP_OPT_NO_NBHD) ? (int)ps.plan.dev.nbhd : -1);
     };
     const bool cap = (options & BEEP_OPT_REFERENCE_ROOT_CAP) != 0;
-    std::set<Graph *> statistics; // graphs with a pair that takes a statistics form at every root
-    for (auto &ps : specs)
-        if (row_form(ps) > kFormWheel && !sup_form(ps) && ps.nshards <= 1 && !cap)
-            statistics.insert(ps.g);
     auto shares_rows = [&](const PairSpec &ps) {
         if (row_form(ps) < 0 || sup_form(ps) || ps.nshards > 1 || cap)
             return false;
-        return row_form(ps) > kFormWheel ||
-               (ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW && statistics.count(ps.g));
+        return row_form(ps) > kFormWheel || ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW;
     };
     // Per graph, the least peel threshold of either kind's pairs. Each kind has
     // its own: a tailed triangle's threshold of 1 in the same call would leave

@@ -1,5 +1,6 @@
 """Which peeled and ordered view of a graph each pair of a call is counted on: a view that a call has built is cached,
 so asking for it afterwards launches nothing."""
+import numpy as np
 import pytest
 
 import beep_b200 as B
@@ -33,15 +34,29 @@ def run(ctx, g, queries):
 
 
 def test_wheel_alone(ctx, graph):
-    """The 4-wheel's plan is a descending one of threshold 3."""
     B.count(graph, P.W5)
-    assert built(ctx, graph, 3, False)
+    assert built(ctx, graph, 3, True)
 
 
 def test_wheel_beside_triangle_forms(ctx, graph):
+    """The 4-wheel's view is peeled for it (threshold 3), whatever the triangle forms need."""
     counts = run(ctx, graph, [P.TAILED_TRIANGLE, P.W5])
-    assert built(ctx, graph, 3, False)
+    assert built(ctx, graph, 3, True)
     assert counts == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in (P.TAILED_TRIANGLE, P.W5)]
+
+
+@pytest.mark.parametrize("degree,asc", [(16384, True), (16385, False)])
+def test_wheel_on_wide_roots(ctx, degree, asc):
+    """Above 16,384 neighbours the list kernel takes over, and with it the plan's descending order."""
+    rng = np.random.default_rng(3)
+    u, v = rng.integers(1, degree + 1, (2, 3 * degree))
+    rp, col = synth.to_csr(degree + 1, np.concatenate([np.zeros(degree, np.int64), u]),
+                           np.concatenate([np.arange(1, degree + 1), v]))
+    for queries in ([P.W5], [P.W5, P.central_patterns(5)[7]]):
+        g = B.Graph.from_csr(ctx, rp, col)
+        run(ctx, g, queries)
+        assert built(ctx, g, 3 if asc is False or len(queries) == 1 else 2, asc)
+        g.close()
 
 
 def test_statistics_beside_triangle_forms(ctx, graph):

@@ -35,7 +35,8 @@ def test_hub_neighbourhoods(ctx, n, p, twins):
     exp = O.count(rp, col, P.W5, apply_root_cap=False)["count"]
     assert exp > 0
     g = B.Graph.from_csr(ctx, rp, col)
-    assert B.count(g, P.W5) == exp
+    assert B.count(g, P.W5) == exp  # ascending view: strips at the smallest vertex
+    assert sum(B.count_shard(g, P.W5, r, 2) for r in range(2)) == exp  # descending: at the largest
     g.close()
 
 
@@ -44,8 +45,8 @@ def test_hub_neighbourhoods(ctx, n, p, twins):
     (2048, 0.004, True), (2049, 0.004, True), (2079, 0.004, True), (2081, 0.004, True), (16384, 0.0003, True),
     (16385, 0.0003, True)])
 def test_hub_neighbourhoods_beside_statistics(ctx, n, p, twins):
-    """Beside a statistics form (4-path cone) the 4-wheel is counted from the same rows, at each cycle's smallest
-    vertex, the strips laid out from the row's end; above 16,384 neighbours on its own view."""
+    """Beside a statistics form (4-path cone) the 4-wheel is counted from the same rows; above 16,384 neighbours on its
+    own view."""
     rp, col = hub_over(n, p, twins, n)
     g = B.Graph.from_csr(ctx, rp, col)
     b = B.Batch(ctx)
