@@ -681,7 +681,17 @@ __device__ __forceinline__ void dfs_warp(const Lp &lp, const uint32_t *bm, uint3
             unsigned bal = __ballot_sync(gmask, w != 0) >> gbase;
             if constexpr (G < 32)
                 bal &= (1u << G) - 1u;
+            uint32_t taken = 0;
             while (bal) {
+                // (a step holds up to 1,024 candidates: once k tuples are
+                // reserved their leaves alone kept a launch for a millisecond)
+                if constexpr (ENUM) {
+                    if ((++taken & 7u) == 0) {
+                        unsigned full = glane == 0 ? (unsigned)enum_full(ec) : 0u;
+                        if (__shfl_sync(gmask, full, 0, G))
+                            return;
+                    }
+                }
                 const int L = __ffs(bal) - 1;
                 const uint32_t ww = __shfl_sync(gmask, w, L, G);
                 const int b = __ffs(ww) - 1;
