@@ -37,7 +37,6 @@
 #include <cmath>
 #include <map>
 #include <mutex>
-#include <set>
 
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -4176,6 +4175,8 @@ static uint64_t pair_result(const LaunchPlan *lp, uint32_t i) {
     return (v < c[0] || v >= BEEP_COUNT_LIMIT) ? BEEP_COUNT_OVERFLOW : v;
 }
 
+constexpr int kLendCalls = 16;
+
 beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t options, LaunchPlanPtr *out,
                        const TierCfg &tiers) {
     cudaStream_t s = ctx->stream;
@@ -4234,10 +4235,20 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             auto r = (sup_form(ps) ? sup_qdeg : row_qdeg).emplace(ps.g, ps.plan.info.min_qdeg);
             r.first->second = std::min(r.first->second, ps.plan.info.min_qdeg);
         }
-    std::set<Graph *> fresh; // graphs without a view yet
-    for (auto &ps : specs)
-        if (ps.g->views.empty() || (options & BEEP_OPT_NO_VIEW_CACHE))
-            fresh.insert(ps.g);
+    // Whether a walked pair of a graph may take another pair's view while its
+    // own (threshold qdeg) is not cached. Building one costs as much as its
+    // stronger peel saves in a few dozen calls (4- and 5-cliques of a served
+    // mix on graphs of up to 2^15 vertices: 1.5 ms for 6 graphs against 0.1 ms
+    // a pass), so only a graph that has come back that often gets it, and
+    // keeps it.
+    std::map<std::pair<Graph *, int32_t>, bool> lends; // one decision a call
+    auto lent = [&](Graph *g, int32_t qdeg) {
+        auto r = lends.emplace(std::make_pair(g, qdeg), false);
+        if (r.second)
+            r.first->second = !g->views.count({(int)qdeg, 1}) &&
+                              ((options & BEEP_OPT_NO_VIEW_CACHE) || ++g->lent[qdeg] <= kLendCalls);
+        return r.first->second;
+    };
     struct SupKey {
         View *v;
         std::vector<int32_t> pair; // first pair of every form, or -1
@@ -4265,13 +4276,10 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
         if (form || shares_rows(ps)) {
             qdeg = (form ? sup_qdeg : row_qdeg)[ps.g];
             asc = 1;
-        } else if (asc && fresh.count(ps.g) && ps.nshards <= 1 && ps.plan.dev.dend == ps.plan.dev.K) {
-            // The call's other view will do on a graph that is counted for the
-            // first time (and perhaps the last: building this pair's own costs
-            // more than the stronger peel saves). The vertices that it drops
-            // are in no match, and whole matches (not prefixes or shards) are
-            // counted once in any order. A graph that comes back gets the
-            // pair's own view, and keeps it.
+        } else if (asc && ps.nshards <= 1 && ps.plan.dev.dend == ps.plan.dev.K && lent(ps.g, qdeg)) {
+            // The call's other view will do: the vertices that this pair's
+            // stronger peel drops are in no match, and whole matches (not
+            // prefixes or shards) are counted once in any order.
             int32_t other = 0;
             for (auto *m : {&row_qdeg, &sup_qdeg}) {
                 auto it = m->find(ps.g);

@@ -225,6 +225,7 @@ struct Graph {
     DevBuf row_ptr; // u32[n+1]
     DevBuf col;     // u32[m]
     std::map<std::pair<int, int>, std::shared_ptr<View>> views;
+    std::map<int, int> lent; // ascending views not built yet: calls that took another one instead (plan_pairs)
 };
 
 struct Query {

@@ -70,9 +70,21 @@ def test_statistics_beside_triangle_forms(ctx, graph):
 
 @pytest.mark.parametrize("shared", [P.TAILED_TRIANGLE, P.central_patterns(5)[6]], ids=["triangle_form", "statistics_form"])
 def test_clique_views_of_a_graph_that_comes_back(ctx, graph, shared):
-    """A first call builds one view for all its patterns; a graph that is counted again gets the cliques' own."""
+    """A first call builds one view for all its patterns; a graph that keeps being counted gets the cliques' own."""
     queries = [shared, P.K4, P.K5]
+    before = ctx.kernel_launches()
     first = run(ctx, graph, queries)
+    after = ctx.kernel_launches()
     assert run(ctx, graph, queries) == first
+    again = ctx.kernel_launches()
+    assert after - before > again - after  # a view is built in the first call ...
+    for _ in range(15):
+        assert run(ctx, graph, queries) == first
     assert built(ctx, graph, 3, True) and built(ctx, graph, 4, True)
     assert first == [B.count(graph, q, B.SGM, B.OPT_NO_NBHD) for q in queries]
+
+
+def test_clique_views_stay_unbuilt_at_first(ctx, graph):
+    for _ in range(3):
+        run(ctx, graph, [P.TAILED_TRIANGLE, P.K4])
+    assert built(ctx, graph, 1, True) and not built(ctx, graph, 3, True)
