@@ -4193,7 +4193,19 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     std::vector<PairDev> hp;
     std::vector<uint64_t> offs{0};
     std::vector<Graph *> dropped;
-    bool built_any = false;
+    // A view built here is cached on its graph, and its build used the
+    // context's scratch: other streams (another slot of a server, another
+    // context) may use both once this call returns, with or without success.
+    // Otherwise nothing waits: the host arrays copied below are pageable,
+    // consumed by the copies.
+    struct ViewWait {
+        cudaStream_t s;
+        bool built = false;
+        ~ViewWait() {
+            if (built)
+                cudaStreamSynchronize(s);
+        }
+    } views_ready{s};
     // Pairs counted from degrees and triangle counts: whole counts only (the
     // sums are not per root). Their view is an ascending one whose peel
     // removes no more than theirs would: peeled vertices are in no match, and
@@ -4289,7 +4301,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
             qdeg = other ? other : qdeg;
         }
         BEEP_TRY(get_view(ctx, ps.g, qdeg, asc, false, &v, &built));
-        built_any = built_any || built;
+        views_ready.built = views_ready.built || built;
         lp->views.push_back(v);
         st.peel_rounds = v->peel_rounds; // view-build launches are counted where they happen
         if (v->n == 0)
@@ -5012,12 +5024,10 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     lp->nexit = (uint32_t)lp->recs.size();
     BEEP_TRY(lp->alloc(lp->d_exit, 2 * (size_t)lp->nexit));
     BEEP_TRY(ctx->host_results(lp->host_words(), &lp->h_counts));
-    // A view built here is cached on its graph, and its build used the
-    // context's scratch: other streams (another slot of a server, another
-    // context) may use both once this call returns. Otherwise nothing waits:
-    // the host arrays copied above were pageable, consumed by the copies.
-    if (built_any)
+    if (views_ready.built) {
+        views_ready.built = false;
         BEEP_CUDA_TRY(cudaStreamSynchronize(s));
+    }
     tr.mark("lists");
     *out = std::move(lp);
     return BEEP_OK;
