@@ -1098,6 +1098,7 @@ constexpr uint32_t kPairWords = 6;
 // once for all its forms.
 constexpr int kFormWheel = 0; // 1 .. 6: NbhdForm
 constexpr int kForms = 7;
+constexpr int kFormWide = kForms; // the 4-wheel's launch for roots of wide rows
 
 struct PairDev {
     ViewDev v;
@@ -2235,6 +2236,7 @@ constexpr uint32_t kLargeSmemA = 48 * 1024; // domain entries staged in shared m
 // W / 8 entries (rounded down to 32): 1 + W / 8 more words a row, under 13%.
 constexpr uint32_t kListMinW = 256;
 constexpr uint32_t kC4StripMaxW = 512; // widest rows counted in strips (4-wheel, statistics)
+constexpr uint32_t kC4WideMaxW = 8192; // widest rows counted in groups of strips (4-wheel, upwards)
 __host__ __device__ __forceinline__ uint32_t list_cap(uint32_t W) { return W >= kListMinW ? (W / 8) & ~31u : 0u; }
 
 // Arena words of one large root: rows [rlo, D) of W = ceil(D / 32) words,
@@ -2547,6 +2549,21 @@ __host__ __device__ __forceinline__ uint32_t c4_tasks(uint32_t D, bool up) {
 }
 static_assert((kC4StripMaxW * 32) >> kC4MaxSlices == 0, "a count fits the slices");
 
+// Wider rows, counted upwards: a task is (root, a, group of 16 strips), so that
+// the b of a are gathered once for all of the group's strips. Group q is the
+// words [W - 512 (q + 1), W - 512 q) and holds the a below them or in them,
+// largest first.
+constexpr uint32_t kWideGroup = 512; // words of a group
+constexpr int kC4WideSlices = 18;
+static_assert((kC4WideMaxW * 32 - 1) >> kC4WideSlices == 0, "a count fits the slices");
+__host__ __device__ __forceinline__ uint32_t c4_wide_rows(uint32_t D, uint32_t q) {
+    return q == 0 ? D : ((D + 31) & ~31u) - 32 * kWideGroup * q;
+}
+__host__ __device__ __forceinline__ uint32_t c4_wide_tasks(uint32_t D) {
+    const uint32_t Q = ((D + 31) / 32 + kWideGroup - 1) / kWideGroup;
+    return D + (Q - 1) * ((D + 31) & ~31u) - 16 * kWideGroup * Q * (Q - 1);
+}
+
 // A hub's paw strips run over all its neighbours b (its 4-wheel strips do too,
 // but start first and are not the longest launch): 0.5 ms for one of 12,000.
 constexpr uint32_t kPawParts = 4;
@@ -2554,8 +2571,12 @@ __host__ __device__ __forceinline__ bool nbhd_strips(int nbhd, uint32_t D) {
     return nbhd >= kNbTriIso && (D + 31) / 32 <= kC4StripMaxW;
 }
 __host__ __device__ __forceinline__ uint32_t form_tasks(uint32_t D, uint32_t sp, int f, bool up) {
+    const uint32_t W = (D + 31) / 32;
+    const bool wide = up && W > kC4StripMaxW && W <= kC4WideMaxW;
+    if (f == kFormWide)
+        return wide ? c4_wide_tasks(D) : 0u;
     if (f == kFormWheel)
-        return (D + 31) / 32 <= kC4StripMaxW ? c4_tasks(D, up) : D;
+        return W <= kC4StripMaxW ? c4_tasks(D, up) : (wide ? 0u : D);
     const uint32_t n = f == kNbPaw || f == kNbDiamond ? D - sp : D;
     return nbhd_strips(f, D) ? n * ((D + 1023) / 1024) * (f == kNbPaw ? kPawParts : 1u) : n;
 }
@@ -2836,6 +2857,155 @@ __global__ void __launch_bounds__(256, kStripBlocksPerSm) k_large_wheel(const Pa
         rl.nzl = rl.nzc + D;
         wheel4_task(rows, rl, W, t - bt.tstart[b], ws, ws + 3 * (size_t)Wm, ws + Wm, ws + 2 * (size_t)Wm, lane,
                     cnt);
+    }
+    cnt = warp_sum(cnt);
+    if (lane == 0 && cur != 0xffffffffu)
+        flush_count(pairs[cur].fcount[kFormWheel], cnt);
+    if (lane == 0)
+        record_exit(exit_t);
+}
+
+constexpr uint32_t kWideList = 1024; // entries of a warp's index list
+
+// Adds rows ib[0, nb) of one column to the counters (c4_add_rows with 32-bit indices).
+template <int NS>
+__device__ __forceinline__ void c4_add_rows_wide(uint32_t (&s)[NS], const uint32_t *col, uint32_t RS,
+                                                 const uint32_t *ib, uint32_t nb) {
+    uint32_t i = 0;
+    for (; i + 8 <= nb; i += 8) {
+        const uint4 p = *reinterpret_cast<const uint4 *>(ib + i), q = *reinterpret_cast<const uint4 *>(ib + i + 4);
+        const uint32_t at[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+        uint32_t d[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            d[j] = col[(size_t)at[j] * RS];
+        c4_add8<NS>(s, d);
+    }
+    if (i < nb) {
+        uint32_t d[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            d[j] = i + j < nb ? col[(size_t)ib[i + j] * RS] : 0u;
+        c4_add8<NS>(s, d);
+    }
+}
+
+// Vertex a's part of the 4-cycles in the columns of group q, upwards. The b
+// above a come from the row's list of non-zero words where it has one; more of
+// them than the list holds are gathered again for every strip.
+__device__ __forceinline__ unsigned long long c4_wide_task(const uint32_t *__restrict__ bm, const RowLists &rl,
+                                                           uint32_t W, uint32_t a, uint32_t q, uint32_t *ib,
+                                                           int lane) {
+    const uint32_t aw = a >> 5, above = ~((2u << (a & 31)) - 1u), hi = W - kWideGroup * q;
+    const uint32_t *ra = bm + (size_t)a * W, *la = rl.nzl + (size_t)a * rl.cap;
+    const uint32_t nl = rl.nzc[a];
+    const bool listed = nl <= rl.cap;
+    const uint32_t steps = listed ? (nl + 31) / 32 : (W - aw + 31) / 32;
+    // appends the b of steps i, i + 1, .. to ib while they fit; their number
+    auto gather = [&](uint32_t &i) {
+        uint32_t have = 0;
+        for (; i < steps; ++i) {
+            const uint32_t e = 32 * i + (uint32_t)lane;
+            const uint32_t k = listed ? (e < nl ? la[e] : W) : aw + e;
+            uint32_t w = k < W && k >= aw ? ra[k] : 0u;
+            if (k == aw)
+                w &= above;
+            const uint32_t n = (uint32_t)__popc(w);
+            uint32_t inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, inc, o);
+                if (lane >= o)
+                    inc += y;
+            }
+            const uint32_t total = __shfl_sync(kFull, inc, 31); // at most 1,024
+            if (have + total > kWideList)
+                break;
+            for (uint32_t at = have + inc - n; w; w &= w - 1)
+                ib[at++] = (k << 5) + (uint32_t)(__ffs(w) - 1);
+            have += total;
+        }
+        __syncwarp();
+        return have;
+    };
+    uint32_t i = 0, have = gather(i);
+    const bool whole = i == steps;
+    unsigned long long tot = 0;
+    if (!whole || have >= 2) // (a cycle has two b)
+        for (uint32_t w0 = max(aw, hi > kWideGroup ? hi - kWideGroup : 0u); w0 < hi; w0 += 32) {
+            const uint32_t k = w0 + (uint32_t)lane, kc = min(k, W - 1);
+            const uint32_t cm = k < hi ? (k > aw ? 0xffffffffu : above) : 0u;
+            uint32_t s[kC4WideSlices];
+#pragma unroll
+            for (int j = 0; j < kC4WideSlices; ++j)
+                s[j] = 0;
+            uint32_t total = have;
+            if (whole) {
+                c4_add_rows_wide<kC4WideSlices>(s, bm + kc, W, ib, have);
+            } else {
+                total = 0;
+                for (i = 0; i < steps;) {
+                    __syncwarp(); // the list is read no more
+                    have = gather(i);
+                    total += have;
+                    c4_add_rows_wide<kC4WideSlices>(s, bm + kc, W, ib, have);
+                }
+            }
+            if (total >= 2)
+                tot += c4_pairs<kC4WideSlices>(s, 32 - __clz((int)total), cm);
+        }
+    __syncwarp(); // ib is rewritten by the warp's next task
+    return tot;
+}
+
+// The 4-wheel at roots of more than kC4StripMaxW words a row (ascending views).
+// Whichever end of the order the list kernel starts from, one kind of graph has
+// hubs on the side that it walks: R-MAT s17 ef28 took 28 ms on the ascending
+// view and 88 on the descending one, a power-law graph of 2^18 vertices 1,375
+// and 644. Counters cost a row read per (b, strip) instead, however full the
+// rows, and their b are few above a.
+__global__ void __launch_bounds__(256, 3) k_large_wheel_wide(const PairDev *__restrict__ pairs, Batch bt,
+                                                             const uint32_t *arena, unsigned *cursor,
+                                                             unsigned long long *exit_t) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t base0 = bt.tstart[0];
+    const uint32_t total = bt.tstart[bt.nb] - base0;
+    __shared__ __align__(16) uint32_t s_ib[8][kWideList];
+    uint32_t cur = 0xffffffffu;
+    unsigned long long cnt = 0;
+    for (;;) {
+        uint32_t t = 0;
+        if (lane == 0)
+            t = atomicAdd(cursor, 1u);
+        t = __shfl_sync(kFull, t, 0);
+        if (t >= total)
+            break;
+        t += base0;
+        const uint32_t b = find_batch(bt.tstart, bt.nb, t);
+        const uint64_t it = bt.item[b];
+        const uint32_t p = item_pair(it), r = item_root(it);
+        if (p != cur) {
+            cnt = warp_sum(cnt);
+            if (lane == 0 && cur != 0xffffffffu)
+                flush_count(pairs[cur].fcount[kFormWheel], cnt);
+            cnt = 0;
+            cur = p;
+        }
+        const uint32_t *rp = pairs[p].v.rp;
+        const uint32_t D = rp[r + 1] - rp[r]; // every neighbour
+        const uint32_t W = (D + 31) >> 5;
+        const uint32_t *rows = arena + bt.off[b]; // rows of the whole domain: rlo == 0
+        RowLists rl;
+        rl.cap = list_cap(W);
+        rl.nzc = rows + (size_t)D * W;
+        rl.nzl = rl.nzc + D;
+        uint32_t q = 0, n = D;
+        t -= bt.tstart[b];
+        for (; t >= n; n = c4_wide_rows(D, q)) {
+            t -= n;
+            ++q;
+        }
+        cnt = sat_add(cnt, c4_wide_task(rows, rl, W, n - 1 - t, q, s_ib[threadIdx.x >> 5], lane));
     }
     cnt = warp_sum(cnt);
     if (lane == 0 && cur != 0xffffffffu)
@@ -3847,7 +4017,7 @@ __global__ void k_form_tasks(const PairDev *__restrict__ pairs, const uint64_t *
                              const uint32_t *__restrict__ D_in, int f, uint32_t *tasks) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
         const PairDev &pd = pairs[item_pair(items[i])];
-        tasks[i] = pd.fmask >> f & 1u ? form_tasks(D_in[i], pd.v.split[item_root(items[i])], f, pd.c4_up != 0) : 0u;
+        tasks[i] = pd.fmask >> (f == kFormWide ? kFormWheel : f) & 1u ? form_tasks(D_in[i], pd.v.split[item_root(items[i])], f, pd.c4_up != 0) : 0u;
     }
 }
 
@@ -4046,7 +4216,7 @@ template <bool ENUM> beep_status large_dfs_blocks_per_sm(int dend, int *out) {
 // ---------------------------------------------------------------------------
 struct LaunchRec {
     enum Kind { kSmall, kMedium, kLargeRows, kLargeLists, kLargeDfs, kLargeWheel, kGeneral, kMemset, kLargeNbDeg,
-                kLargeNbhd, kSupTri, kSupEdge, kSupVertex } kind;
+                kLargeNbhd, kLargeWide, kSupTri, kSupEdge, kSupVertex } kind;
     const SupView *sup = nullptr; // degree and triangle-count forms: views and 32-entry chunks
     uint32_t nsup = 0;
     int form = 0; // kLargeNbhd: the statistics form
@@ -4236,7 +4406,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     auto shares_rows = [&](const PairSpec &ps) {
         if (row_form(ps) < 0 || sup_form(ps) || ps.nshards > 1 || cap)
             return false;
-        return row_form(ps) > kFormWheel || ps.g->max_degree <= 32 * (int64_t)kC4StripMaxW;
+        return row_form(ps) > kFormWheel || ps.g->max_degree <= 32 * (int64_t)kC4WideMaxW;
     };
     // Per graph, the least peel threshold of either kind's pairs. Each kind has
     // its own: a tailed triangle's threshold of 1 in the same call would leave
@@ -4480,6 +4650,15 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     // a walk launch of the large tier: a persistent grid of resident blocks,
     // and (for k_large_dfs) the donation queue, whose ready flags are cleared
     // before the launch
+    // the large tier's launches of the forms counted from rows
+    auto takes_form = [&](int f, uint32_t most) {
+        return f == kFormWide ? (any_forms >> kFormWheel & 1u) && (most + 31) / 32 > kC4StripMaxW
+                              : (any_forms >> f & 1u) != 0;
+    };
+    auto form_kind = [](int f) {
+        return f == kFormWide ? LaunchRec::kLargeWide
+                              : (f == kFormWheel ? LaunchRec::kLargeWheel : LaunchRec::kLargeNbhd);
+    };
     auto push_walk = [&](LaunchRec ld) -> beep_status {
         ld.tail_slot = 2;
         if (ld.kind == LaunchRec::kLargeDfs) {
@@ -4625,8 +4804,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 continue;
             const int d = sl % kDepths;
             if (d == (int)kWheelSlot) { // a launch per form, over the same rows
-                for (int f = 0; f < kForms; ++f) {
-                    if (!(any_forms >> f & 1u))
+                for (int f = kFormWide; f >= 0; --f) { // (the longest first)
+                    if (!takes_form(f, tier_max[3]))
                         continue;
                     uint32_t *ft = nullptr, *fs = nullptr;
                     BEEP_TRY(lp->alloc(ft, cnt));
@@ -4637,7 +4816,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                     BEEP_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp, tb, ft, fs + 1, cnt, s));
                     BEEP_CUDA_TRY(cudaMemsetAsync(fs, 0, 4, s));
                     LaunchRec ld;
-                    ld.kind = f == kFormWheel ? LaunchRec::kLargeWheel : LaunchRec::kLargeNbhd;
+                    ld.kind = form_kind(f);
                     ld.form = f;
                     ld.dend = d;
                     ld.grid = ctx->num_sms * kLargeDfsBlocksPerSm;
@@ -4755,8 +4934,8 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 while (b < nbt && rs[i0 + b].dend == rs[i0 + a].dend)
                     ++b;
                 if (rs[i0 + a].dend == kWheelSlot) {
-                    for (int f = 0; f < kForms; ++f)
-                        if (any_forms >> f & 1u)
+                    for (int f = kFormWide; f >= 0; --f)
+                        if (takes_form(f, bmaxD))
                             groups.push_back({a, b - a, f});
                 } else {
                     groups.push_back({a, b - a, -1});
@@ -4773,7 +4952,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                     const PairDev &pdv = hp[(uint32_t)(x.item >> 32)];
                     if (gp.form < 0)
                         acc += x.D - x.j0;
-                    else if (pdv.fmask >> gp.form & 1u)
+                    else if (pdv.fmask >> (gp.form == kFormWide ? kFormWheel : gp.form) & 1u)
                         acc += form_tasks(x.D, x.sp, gp.form, pdv.c4_up != 0);
                     ts_all.push_back(acc);
                 }
@@ -4815,7 +4994,7 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
                 ld.enumerate = slot >= (uint32_t)kDepths;
                 ld.form = groups[gi].form;
                 ld.kind = ld.form < 0 ? LaunchRec::kLargeDfs
-                                      : (ld.form == kFormWheel ? LaunchRec::kLargeWheel : LaunchRec::kLargeNbhd);
+                                      : form_kind(ld.form);
                 ld.grid = ctx->num_sms * kLargeDfsBlocksPerSm;
                 ld.block = 256;
                 ld.bt = Batch{d_bitem + groups[gi].first, d_boff + groups[gi].first, d_cs, d_ts + ts_off[gi],
@@ -5116,6 +5295,12 @@ beep_status issue(Ctx *ctx, LaunchPlan *lp, bool timing, bool serial, bool stall
         case LaunchRec::kLargeWheel:
             k_large_wheel<<<r.grid, r.block, 0, rs>>>(lp->d_pairs, r.bt, static_cast<const uint32_t *>(r.mptr),
                                                       r.cursor, r.wsc, r.wstride, ex);
+            BEEP_CUDA_TRY(cudaGetLastError());
+            st.large_dfs_launches++;
+            break;
+        case LaunchRec::kLargeWide:
+            k_large_wheel_wide<<<r.grid, r.block, 0, rs>>>(lp->d_pairs, r.bt, static_cast<const uint32_t *>(r.mptr),
+                                                           r.cursor, ex);
             BEEP_CUDA_TRY(cudaGetLastError());
             st.large_dfs_launches++;
             break;
