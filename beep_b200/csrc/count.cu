@@ -2963,7 +2963,8 @@ __device__ __forceinline__ unsigned long long c4_wide_task(const uint32_t *__res
 // hubs on the side that it walks: R-MAT s17 ef28 took 28 ms on the ascending
 // view and 88 on the descending one, a power-law graph of 2^18 vertices 1,375
 // and 644. Counters cost a row read per (b, strip) instead, however full the
-// rows, and their b are few above a.
+// rows, and their b are few above a: 9 and 28 ms (s20 ef28: 6,111 and 8,672
+// against 208). Bound by those reads, from L2 or, for rows that exceed it, HBM.
 __global__ void __launch_bounds__(256, 3) k_large_wheel_wide(const PairDev *__restrict__ pairs, Batch bt,
                                                              const uint32_t *arena, unsigned *cursor,
                                                              unsigned long long *exit_t) {
@@ -4386,12 +4387,9 @@ beep_status plan_pairs(Ctx *ctx, const std::vector<PairSpec> &specs, uint32_t op
     };
     // Pairs counted from a root's rows share their items, on an ascending view
     // too, when they count every root: the later lists that rows are built from
-    // are short there. Where a root may be wider than the strips take, the
-    // 4-wheel keeps its plan's descending view: the list kernel works over the
-    // neighbours after a cycle's first vertex, which are the short side only
-    // there (18 times the row entries on the ascending one, CPU count of a hub
-    // of 31,080 on a power-law graph; served workload of 32 graphs of up to
-    // 10^7 edges: 90.6 s on it, 50.2 s on its own).
+    // are short there. Where a root may be wider than the groups of strips
+    // take, the 4-wheel keeps its plan's descending view, as shards and the
+    // root cap do, for the list kernel.
     // (4-wheels of R-MAT s16 ef28: strips downwards 8.9 ms, on the descending
     // view 7.4, upwards 7.35; s11 ef28: 268, 275 and 266 us. 12 power-law graphs
     // x 15 patterns: 10.8 ms downwards, 10.6 upwards, 11.6 on a view and rows
