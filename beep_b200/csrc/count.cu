@@ -2964,7 +2964,8 @@ __device__ __forceinline__ unsigned long long c4_wide_task(const uint32_t *__res
 // view and 88 on the descending one, a power-law graph of 2^18 vertices 1,375
 // and 644. Counters cost a row read per (b, strip) instead, however full the
 // rows, and their b are few above a: 9 and 28 ms (s20 ef28: 6,111 and 8,672
-// against 208). Bound by those reads, from L2 or, for rows that exceed it, HBM.
+// against 208). The row reads' latency bounds it (s17 ef28: 55% of what the SMs
+// can issue, at the three blocks an SM that 74 registers leave; 95% L2 hits).
 __global__ void __launch_bounds__(256, 3) k_large_wheel_wide(const PairDev *__restrict__ pairs, Batch bt,
                                                              const uint32_t *arena, unsigned *cursor,
                                                              unsigned long long *exit_t) {
